@@ -179,8 +179,9 @@ def tolerance(case):
     """Relative 2-norm errors from the rounding of the results, measured against the same path in 64 bits and then
     about four times that: a bf16 output alone is off by 1.7e-3 of its norm (the fp32 sums before it by some 1e-6, by
     7e-5 where activations are held as 15-bit integers); a MoE layer rounds to bf16 after every linear (3.9e-3; 5.8e-3
-    in the standard flavour, which rounds every sum); the int8 linear quantises its activations, which every implementation does alike. Table rows are exact (products with
-    trits, one rounding); the int8 grouped GEMM returns float32 sums."""
+    in the standard flavour, which rounds every sum, but alike everywhere); the int8 linear quantises its activations,
+    which every implementation does alike. Table rows are exact (products with trits, one rounding); the int8 grouped
+    GEMM returns float32 sums."""
     if case["kind"] == "table":
         return "exact"
     if case["kind"] == "grouped":
