@@ -87,14 +87,28 @@ def _trits(gen, rows, K):
     return (r >= 4).to(torch.int8) - (r >= 7).to(torch.int8) * 2
 
 
+def _trit_blocks(gen, rows, K):
+    """(first row, fresh trits) of consecutive rows, some 64 M weights at a time."""
+    step = max(1, (1 << 26) // K)
+    for i in range(0, rows, step):
+        yield i, _trits(gen, min(step, rows - i), K)
+
+
 def _packed(gen, E, N, K, fmt):
-    """[E, N, packed_cols] of fresh trits, some 64 M weights at a time."""
+    """[E, N, packed_cols] of fresh trits."""
     out = torch.empty(E, N, packed_cols(fmt, K), dtype=torch.uint8, device=DEV)
-    flat, step = out.view(E * N, -1), max(1, (1 << 26) // K)
-    for i in range(0, E * N, step):
-        n = min(step, E * N - i)
-        flat[i:i + n] = pack(_trits(gen, n, K), fmt)
+    flat = out.view(E * N, -1)
+    for i, t in _trit_blocks(gen, E * N, K):
+        flat[i:i + t.size(0)] = pack(t, fmt)
     return out
+
+
+def _plain(gen, E, N, K):
+    """[E, N, K] int8: the trits that _packed draws from the same generator state."""
+    out = torch.empty(E * N, K, dtype=torch.int8, device=DEV)
+    for i, t in _trit_blocks(gen, E * N, K):
+        out[i:i + t.size(0)] = t
+    return out.view(E, N, K)
 
 
 def _scales(gen, term, *shape, dtype=torch.float16):
@@ -149,6 +163,69 @@ def run(state):
     if s["kind"] == "table":
         return s["table"].rows(s["ids"])
     return grouped_ternary_gemm(s["x"], s["x_scale"], s["offsets"], s["packed"], s["scale"], s["K"], GROUP, s["fmt"])
+
+
+# ------------------------------------------------------------------------------------------------- the same in 64 bits
+def _weight(terms, e, K):
+    """[N, K] float64 of matrix e: sum over the stacked terms of trit * group scale."""
+    return sum(t[e].double() * s[e].double().repeat_interleave(GROUP, -1)[:, :K] for t, s in terms)
+
+
+def _plain_experts(gen, E, hidden, inter, terms):
+    """(w13, w2) as lists of (trits, scales), drawn in the order of _experts."""
+    w13, w2 = [], []
+    for t in range(terms):
+        w13.append((_plain(gen, E, 2 * inter, hidden), _scales(gen, t, E, 2 * inter, hidden // GROUP)))
+        w2.append((_plain(gen, E, hidden, inter), _scales(gen, t, E, hidden, inter // GROUP)))
+    return w13, w2
+
+
+def _expert64(experts, e, x, hidden, inter, row_weight=None):
+    gate, up = (x @ _weight(experts[0], e, hidden).T).split(inter, -1)
+    h = gate * torch.sigmoid(gate) * up
+    return (h if row_weight is None else h * row_weight[:, None]) @ _weight(experts[1], e, inter).T
+
+
+def exact(case, seed):
+    """What run() returns, from the same draws, without any rounding in between (the int8 modes' own quantisation of the
+    activations included: it is part of what they compute)."""
+    c, gen = case, torch.Generator(device=DEV).manual_seed(seed)
+    if c["kind"] == "linear":
+        terms = [(_plain(gen, 1, c["N"], c["K"]), _scales(gen, t, c["N"], c["K"] // GROUP)[None]) for t in range(c["terms"])]
+        x = torch.randn(c["rows"], c["K"], generator=gen, device=DEV).bfloat16().double()
+        if c["act"] == "int8":
+            s = x.abs().amax(-1, keepdim=True) / 127
+            x = (x / s).round() * s
+        return x @ _weight(terms, 0, c["K"]).T
+    if c["kind"] == "moe":
+        H, I = c["hidden"], c["inter"]
+        experts = _plain_experts(gen, c["experts"], H, I, c["terms"])
+        shared = _plain_experts(gen, 1, H, I, c["terms"]) if c["flavour"] == "v4" and c["shared"] else None
+        x = torch.randn(c["tokens"], H, generator=gen, device=DEV).bfloat16().double()
+        logits = torch.randn(c["tokens"], c["experts"], generator=gen, device=DEV).double()
+        score = {"softmax": lambda v: v.softmax(-1), "sigmoid": torch.sigmoid,
+                 "sqrtsoftplus": lambda v: torch.nn.functional.softplus(v).sqrt()}[c["score"]](logits)
+        w, ids = score.topk(c["top_k"], -1)
+        w = w / w.sum(-1, keepdim=True)
+        y = torch.zeros_like(x)
+        for e in range(c["experts"]):
+            tok, slot = (ids == e).nonzero(as_tuple=True)
+            if tok.numel():
+                y.index_add_(0, tok, _expert64(experts, e, x[tok], H, I, w[tok, slot]))
+        return y if shared is None else y + _expert64(shared, 0, x, H, I)
+    if c["kind"] == "table":
+        terms = [(_plain(gen, 1, c["table_rows"], c["K"])[0], _scales(gen, t, c["table_rows"], c["K"] // GROUP)) for t in range(c["terms"])]
+        ids = torch.randint(0, c["table_rows"], (c["ids"],), generator=gen, device=DEV)
+        return sum(t[ids].double() * s[ids].double().repeat_interleave(GROUP, -1) for t, s in terms)
+    E, T, K, N = c["experts"], c["rows"], c["K"], c["N"]
+    of = torch.randint(0, E, (T,), generator=gen, device=DEV).sort().values
+    terms = [(_plain(gen, E, N, K), _scales(gen, 0, E, N, -(-K // GROUP), dtype=torch.float32))]
+    x = torch.randint(-127, 128, (T, K), generator=gen, device=DEV, dtype=torch.int8).double()
+    x = x * (torch.rand(T, generator=gen, device=DEV) * 0.02 + 0.01).double()[:, None]
+    y = x.new_empty(T, N)
+    for e in of.unique().tolist():
+        y[of == e] = x[of == e] @ _weight(terms, e, K).T
+    return y
 
 
 # ------------------------------------------------------------------------------------------------- work and tolerance
