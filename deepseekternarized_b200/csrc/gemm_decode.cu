@@ -2,7 +2,7 @@
 //
 //     out[m, n] = row_scale[m] * sum_i sum_g scale_i[e, n, g] * sum_{k in g} x[m, k] * trit_i[e, n, k]
 //
-// Every packed byte crosses HBM once: one thread per CTA streams the item's rows of the tiled layout's 8 KB slabs
+// Every packed byte crosses HBM once: one thread per CTA streams the unit's rows of the tiled layout's 8 KB slabs
 // (layout_kernels.cu), two superblocks at a time, into a shared-memory ring with cp.async.bulk + mbarrier; the consumer
 // warps read them from there with 128-bit loads. The multiply-adds are exact integer arithmetic on mma.sync.m16n8k32 (u8 x s8 -> s32)
 // fed straight from registers:
@@ -26,10 +26,12 @@
 //               boilerplate/kernels/csrc/boilerplate_cpu.cpp:116-124) runs once per four groups, each lane of a
 //               quad doing one of them; the quad's partial results are added with two shuffles at the end of K.
 //
-// Up to four token rows per expert: four consumer warps of 16 weight rows each and several CTAs per SM; a work item
-// is (expert, 64-row half tile) over the whole of K. Five or more: the staged token rows take most of an SM's shared
-// memory, so one CTA per SM of eight consumer warps that own two 16-row tiles each (a 256-row item; see the kernel).
-// Items are dealt to CTAs in contiguous, equally sized ranges so an expert's token rows are staged once per CTA and run.
+// Up to four token rows per expert: four consumer warps of 16 weight rows each and several CTAs per SM; a work unit
+// is (expert, pass, 64-row half tile) over the whole of K. Where the row counts are on the device only, a pass takes up to
+// four rows and each pass picks its column sharing by the rows it has. Five or more: the staged token rows take most of an
+// SM's shared memory, so one CTA per SM of eight consumer warps that own two 16-row tiles each (256 rows; see the kernel).
+// Measured with two TQ2 terms, both GEMVs of a layer (384 experts, 4096 x 2048): one token (6 experts, 75 MB) 31 us, 64
+// tokens (245 experts, 3.3 GB) 674 us = 4.8 TB/s; 563 and 2853 us when all experts shared the grid and a pass had one row.
 // Every mbarrier wait is bounded by elapsed clock cycles; on expiry the CTA raises its abort flag, all warps leave
 // and the kernel records DST_ERR_TIMEOUT in the status word dst_check_device_status reads.
 //
@@ -40,13 +42,13 @@
 namespace dst {
 namespace {
 
-// CW consumer warps of RW 16-row MMA tiles each (+ the producer warp) make a CTA; a work item is CW * RW * 16 rows of one
+// CW consumer warps of RW 16-row MMA tiles each (+ the producer warp) make a CTA; a work unit is CW * RW * 16 rows of one
 // expert over the whole of K. Few token rows: CW = 4, RW = 1 and several CTAs per SM. Five or more: the staged token rows
 // take most of an SM's shared memory, so ONE CTA of 8 consumer warps with two tiles each shares them (cw below counts
 // 16-row tiles: CW * RW).
 constexpr int DC_QWARPS = 4;                      // warps per block of decode_quant_kernel
-__host__ __device__ constexpr int dc_part(int cw) { return cw * 16 * 64; }           // bytes of one item's share of a superblock: 64 B per row
-__host__ __device__ constexpr int dc_slot_data(int cw) { return 2 * dc_part(cw); }   // a ring slot holds the item's share of TWO superblocks (four scale groups)
+__host__ __device__ constexpr int dc_part(int cw) { return cw * 16 * 64; }           // bytes of one unit's share of a superblock: 64 B per row
+__host__ __device__ constexpr int dc_slot_data(int cw) { return 2 * dc_part(cw); }   // a ring slot holds the unit's share of TWO superblocks (four scale groups)
 __host__ __device__ constexpr int dc_slot(int cw) { return dc_slot_data(cw) + 16; }  // ... followed by its own "full" and "empty" mbarriers (one address register serves all)
 #ifndef DC_RING_SLOTS
 #define DC_RING_SLOTS 4
@@ -141,22 +143,109 @@ __device__ __forceinline__ void mma_u8s8(int* d, uint32_t a0, uint32_t a1, uint3
                  : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// ------------------------------------------------------------------------------------------ work items
-// Item -> (expert, block of RI = 64, 128 or 256 weight rows starting at row n0). Token rows [ra, rb) of the expert.
-struct Item {
-  int e, n0;
-  int64_t ra, rb;
+// ------------------------------------------------------------------------------------------ work units
+// A work unit is (expert, pass, block of RI = 64, 128 or 256 weight rows): pass i covers the expert's token rows
+// ra + i MT .. (MT at most). Only experts with rows have units; they are numbered expert by expert, pass by pass, row
+// block by row block, and every CTA takes an equal, contiguous run of them, so a pass's token rows are staged once per CTA.
+// Experts without rows get no share of the grid: a decode step that reaches 6 of 384 experts ran on ten of the 592 CTAs
+// when the runs were cut over all experts' row blocks (one token, two stacked terms: 563 us for both GEMVs).
+template <int RI>
+__host__ __device__ __forceinline__ int blocks_per_expert(int NT) { return (NT * 128 + RI - 1) / RI; }
+
+struct Unit {
+  int e, n0;           // expert and first weight row
+  int64_t ra, rb, m0;  // the expert's token rows [ra, rb) and the pass's first one
 };
-template <int RI>
-__host__ __device__ __forceinline__ int items_per_expert(int NT) { return (NT * 128 + RI - 1) / RI; }
-template <int RI>
-__device__ __forceinline__ Item item_of(const DecodeParams& p, long long item) {
-  Item it;
-  const int ipe = items_per_expert<RI>(p.NT);
-  it.e = (int)(item / ipe);
-  it.n0 = (int)(item - (long long)it.e * ipe) * RI;
-  row_range(p.offsets, it.e, p.T, it.ra, it.rb);
-  return it;
+
+// A warp's position in the unit sequence (the same in all its lanes; every call is made by the whole warp).
+template <int MT, int RI>
+struct UnitWalk {
+  int block, blocks;  // row block inside the pass
+  Unit u;
+  // local = the unit's index among the units of expert e (which has rows)
+  __device__ __forceinline__ void start(const DecodeParams& p, int e, long long local) {
+    blocks = blocks_per_expert<RI>(p.NT);
+    u.e = e;
+    row_range(p.offsets, e, p.T, u.ra, u.rb);
+    const long long pass = local / blocks;
+    block = (int)(local - pass * blocks);
+    u.m0 = u.ra + pass * MT;
+    u.n0 = block * RI;
+  }
+  __device__ __forceinline__ void next(const DecodeParams& p) {
+    if (++block == blocks) {
+      block = 0;
+      u.m0 += MT;
+      if (u.m0 >= u.rb) {
+        // the next expert with rows, 32 at a time (an empty or inverted range has none)
+        const int lane = threadIdx.x & 31;
+        for (int e0 = u.e + 1; e0 < p.E; e0 += 32) {
+          int64_t a = 0, b = 0;
+          if (e0 + lane < p.E) row_range(p.offsets, e0 + lane, p.T, a, b);
+          const uint32_t some = __ballot_sync(0xffffffffu, b > a);
+          if (some) {
+            const int src = __ffs(some) - 1;
+            u.e = e0 + src;
+            u.ra = __shfl_sync(0xffffffffu, a, src);
+            u.rb = __shfl_sync(0xffffffffu, b, src);
+            break;
+          }
+        }
+        u.m0 = u.ra;
+      }
+    }
+    u.n0 = block * RI;
+  }
+};
+
+// The CTA's run of units, found by all its threads together: every thread counts the units of a contiguous run of experts,
+// a block-wide scan gives their number and the expert that holds the CTA's first unit. scratch: one long long per warp.
+struct UnitRun {
+  long long count;    // units of this CTA
+  long long local;    // the first one's index among the units of expert e
+  int e;
+};
+template <int MT, int RI, int THREADS>
+__device__ __forceinline__ void find_run(const DecodeParams& p, long long* scratch, UnitRun* run) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (p.E + THREADS - 1) / THREADS;
+  const int e0 = threadIdx.x * per, e1 = e0 + per < p.E ? e0 + per : p.E;
+  const int blocks = blocks_per_expert<RI>(p.NT);
+  auto units_of = [&](int e) -> long long {
+    int64_t a, b;
+    row_range(p.offsets, e, p.T, a, b);
+    return (b - a + MT - 1) / MT * blocks;
+  };
+  long long sum = 0;
+  for (int e = e0; e < e1; ++e) sum += units_of(e);
+  long long incl = sum;
+  for (int d = 1; d < 32; d <<= 1) {
+    const long long up = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += up;
+  }
+  if (lane == 31) scratch[warp] = incl;
+  if (threadIdx.x == 0) run->count = 0;
+  __syncthreads();
+  long long before = incl - sum, total = 0;
+  for (int w = 0; w < THREADS / 32; ++w) {
+    if (w < warp) before += scratch[w];
+    total += scratch[w];
+  }
+  const long long u0 = total * blockIdx.x / gridDim.x, u1 = total * (blockIdx.x + 1) / gridDim.x;
+  if (u0 < u1 && u0 >= before && u0 < before + sum) {
+    long long left = u0 - before;
+    for (int e = e0; e < e1; ++e) {
+      const long long n = units_of(e);
+      if (left < n) {
+        run->e = e;
+        run->local = left;
+        run->count = u1 - u0;
+        break;
+      }
+      left -= n;
+    }
+  }
+  __syncthreads();
 }
 
 // ------------------------------------------------------------------------------------------ staging
@@ -326,18 +415,286 @@ decode_quant_kernel(const DecodeParams p, uint8_t* __restrict__ q_rows, int* __r
 #endif
 __host__ __device__ constexpr int dc_min_blocks(int nb, int cw) { return cw > 4 ? 1 : (nb == 1 ? DC_MINB : (nb == 2 ? DC_MINB2 : DC_MINB4)); }
 
+// What a consumer lane keeps while it walks the ring.
+struct RingPos {
+  uint32_t base, end;  // first byte of the ring and the one after it
+  uint32_t slot;       // the current slot
+  uint32_t ph;         // parity of its "full" phase
+};
+
+// One pass over one row block: mc staged token rows against the warp's RW 16-row tiles, the whole of K, all terms.
+template <int GS, int NB, int CW, int RW>
+__device__ __forceinline__ bool run_pass(const DecodeParams& p, const Unit& it, int mc, RingPos& ring, uint32_t xs_a, uint32_t zero_a,
+                                         const int* xsum4, const float* xexp, volatile int* abort_flag) {
+  constexpr int TPB = 4 / GS;      // token rows per column block
+  constexpr int PART = dc_part(CW * RW), SLOT_DATA = dc_slot_data(CW * RW), SLOT = dc_slot(CW * RW);
+  constexpr bool ONEACC = RW > 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g8 = lane >> 2, c = lane & 3;
+  const int swz = (g8 >> 1) & 3;
+  // this lane's unit of row g8 of the warp's first 16-row tile; row g8 + 8: + 512; the second tile: + 1024
+  const uint32_t a_off = (uint32_t)((warp * 16 * RW + g8) * 64 + ((c ^ swz) << 4));
+  // B column of this lane: pair g8 / 2, part g8 & 1; C columns of this lane: pair c
+  const int col_pair = g8 >> 1, col_part = g8 & 1;
+  const int tok_c = c / GS, slot_c = c % GS;  // (+ b * TPB) the token and the group slot of this lane's C columns
+  const int n_first = it.n0 + warp * 16 * RW + g8;  // this lane's output rows: n_first + 8 i, i < 2 RW
+  const int64_t m0 = it.m0;
+  uint32_t sbase = ring.slot, ph = ring.ph;
+  // B pointers. Shared columns (GS > 1): for phase s (= group % GS) the lane reads its column's staged row when
+  // the column's pair belongs to that phase and its token exists, else the zeros. One group per MMA (GS == 1):
+  // column pair j of block b is token 4 b + j; the columns of tokens that do not exist read whatever the staged
+  // rows hold there (integers: an MMA column only reaches its own outputs, which are not stored).
+  constexpr int NPTR = GS > 1 ? GS : 1;
+  uint32_t bbase[NPTR], bstep[NPTR];
+  uint32_t bblock = 0;  // GS == 1: bytes between the staged rows of consecutive column blocks
+  if (GS > 1) {
+#pragma unroll
+    for (int s = 0; s < NPTR; ++s) {
+      const int tok = col_pair / GS;
+      const bool act = (col_pair % GS) == s && tok < mc;
+      bbase[s] = act ? xs_a + (uint32_t)(2 * tok + col_part) * (uint32_t)p.xstride + (uint32_t)c * 16u : zero_a;
+      bstep[s] = act ? 256u : 0u;
+    }
+  } else {
+    bbase[0] = xs_a + (uint32_t)(2 * col_pair + col_part) * (uint32_t)p.xstride + (uint32_t)c * 16u;
+    bstep[0] = 256u;
+    bblock = 8u * (uint32_t)p.xstride;
+  }
+  float y[RW][NB][2];
+#pragma unroll
+  for (int t = 0; t < RW; ++t)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) y[t][b][0] = y[t][b][1] = 0.f;
+
+  for (int term = 0; term < p.n_terms; ++term) {
+    // scale rows of this lane's outputs (rows beyond N read row 0 and are not stored)
+    const __half* srow[2 * RW];
+#pragma unroll
+    for (int i = 0; i < 2 * RW; ++i) {
+      const int n = n_first + 8 * i;
+      srow[i] = p.scale[term] + ((int64_t)it.e * p.N + (n < p.N ? n : 0)) * p.G;
+    }
+    int accA[1][ONEACC ? 1 : NB][4], accB[ONEACC ? 1 : NB][4];  // the x1 and the x4 fields' sums (one tile per warp)
+#pragma unroll
+    for (int b = 0; b < (ONEACC ? 1 : NB); ++b)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) accA[0][b][i] = accB[b][i] = 0;
+    // scales of the lane's group of the next epilogue, requested ahead: a block of GS groups (shared columns), or
+    // two groups at a time, two groups ahead, as one 32-bit load per output row (GS == 1; G is a multiple of 4)
+    auto scale_at = [&](const __half* s, int grp) { return grp < p.G ? __half2float(s[grp]) : 0.f; };
+    auto scale2_at = [&](const __half* s, int grp) { return grp < p.G ? *reinterpret_cast<const uint32_t*>(s + grp) : 0u; };
+    float s_next[2 * RW];
+    uint32_t s2_cur[2 * RW], s2_next[2 * RW];
+#pragma unroll
+    for (int i = 0; i < 2 * RW; ++i) {
+      s_next[i] = GS > 1 ? scale_at(srow[i], slot_c) : 0.f;
+      s2_cur[i] = 0u;
+      s2_next[i] = GS == 1 ? scale2_at(srow[i], 0) : 0u;
+    }
+    // Epilogue of the block of GS groups whose first group is g_first: this lane's group is g_first + slot_c.
+    // First the group's scales (odd: g_first & 1 as a compile-time value) ...
+    float sc[2 * RW];
+    auto take_scales = [&](int g_first, bool odd) {
+      const int g_mine = g_first + slot_c;
+#pragma unroll
+      for (int i = 0; i < 2 * RW; ++i) {
+        if (GS > 1) {
+          sc[i] = s_next[i];
+          s_next[i] = scale_at(srow[i], g_mine + GS);
+        } else {
+          if (!odd) {
+            s2_cur[i] = s2_next[i];
+            s2_next[i] = scale2_at(srow[i], g_first + 2);
+          }
+          const __half2 h2 = *reinterpret_cast<const __half2*>(&s2_cur[i]);
+          sc[i] = odd ? __high2float(h2) : __low2float(h2);
+        }
+      }
+    };
+    // ... then per column block: 4 * sum_k u_k q_k - 4 * sum_k q_k as one integer, converted and multiplied.
+    // x1 / x4 accumulators: 128 * (4 A_hi + B_hi) + (4 A_lo + B_lo)
+    auto epilogue = [&](int g_first) {
+      const int g_mine = g_first + slot_c;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const int xs4 = g_mine < p.G ? xsum4[(b * TPB + tok_c) * p.GP + g_mine] : 0;
+        const int v_lo = ((((accA[0][b][0] << 2) + accB[b][0]) << 7) + ((accA[0][b][1] << 2) + accB[b][1])) - xs4;
+        const int v_hi = ((((accA[0][b][2] << 2) + accB[b][2]) << 7) + ((accA[0][b][3] << 2) + accB[b][3])) - xs4;
+        y[0][b][0] = fmaf(sc[0], (float)v_lo, y[0][b][0]);
+        y[0][b][1] = fmaf(sc[1], (float)v_hi, y[0][b][1]);
+      }
+    };
+    // plain digits, one accumulator set, a pair of column blocks: 4 * (128 * A_hi + A_lo)
+    auto epilogue_pair = [&](int g, int b0, const int (&acc)[RW][2][4]) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int xs4 = xsum4[((b0 + j) * TPB + tok_c) * p.GP + g];
+#pragma unroll
+        for (int t = 0; t < RW; ++t) {
+          const int v_lo = (acc[t][j][0] << 9) + ((acc[t][j][1] << 2) - xs4);
+          const int v_hi = (acc[t][j][2] << 9) + ((acc[t][j][3] << 2) - xs4);
+          y[t][b0 + j][0] = fmaf(sc[2 * t], (float)v_lo, y[t][b0 + j][0]);
+          y[t][b0 + j][1] = fmaf(sc[2 * t + 1], (float)v_hi, y[t][b0 + j][1]);
+        }
+      }
+    };
+
+    // two superblocks (one ring slot, four scale groups) per iteration: the phase of every group (group % GS) is a
+    // compile-time value, and the barrier traffic and slot arithmetic are paid once per 2 KB of a 16-row tile
+    for (int sb0 = 0; sb0 < p.S; sb0 += 2) {
+      if (!__all_sync(0xffffffffu, mbar_wait(sbase + SLOT_DATA, ph, abort_flag))) return false;
+      const uint32_t sa = sbase + a_off;
+      // [superblock][tile]: rows g8 and g8 + 8. One tile per warp: both superblocks' words are read up front and the
+      // slot is handed back at once; two tiles: the second superblock's words are read after the first one's MMAs
+      // (registers), and the slot goes back then
+      uint4 w_lo2[2][RW], w_hi2[2][RW];
+      const uint32_t slot_bar = sbase + SLOT_DATA + 8;
+#pragma unroll
+      for (int u = 0; u < (RW == 1 ? 2 : 1); ++u)
+#pragma unroll
+        for (int t = 0; t < RW; ++t) {
+          w_lo2[u][t] = lds128(sa + u * PART + t * 1024);
+          w_hi2[u][t] = lds128(sa + u * PART + t * 1024 + 512);
+        }
+      if (RW == 1) mbar_arrive(slot_bar);  // every lane arrives for itself: its loads above are done
+      sbase += SLOT;
+      if (sbase == ring.end) { sbase = ring.base; ph ^= 1u; }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int sb = sb0 + u;
+        if (RW > 1 && u == 1) {
+#pragma unroll
+          for (int t = 0; t < RW; ++t) {
+            w_lo2[1][t] = lds128(sa + PART + t * 1024);
+            w_hi2[1][t] = lds128(sa + PART + t * 1024 + 512);
+          }
+          mbar_arrive(slot_bar);
+        }
+#pragma unroll
+        for (int gi = 0; gi < 2; ++gi) {
+          constexpr uint32_t M1 = 0x03030303u, M4 = 0x0c0c0c0cu;
+          const int phase = (u * 2 + gi) % GS;   // group % GS
+          const bool fresh = phase == 0;         // first group of an epilogue block: the accumulators restart
+          const uint32_t bgrp = bbase[phase] + (uint32_t)sb * bstep[phase] + (uint32_t)gi * 128u;
+          if (ONEACC) {
+            // operands of both tiles: [tile][field][a0..a3]
+            uint32_t op[RW][4][4];
+#pragma unroll
+            for (int t = 0; t < RW; ++t) {
+              const uint4 w_lo = w_lo2[u][t], w_hi = w_hi2[u][t];
+              const uint32_t wd[4] = {gi ? w_lo.z : w_lo.x, gi ? w_hi.z : w_hi.x, gi ? w_lo.w : w_lo.y, gi ? w_hi.w : w_hi.y};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                op[t][0][i] = wd[i] & M1;
+                op[t][1][i] = (wd[i] >> 2) & M1;
+                op[t][2][i] = (wd[i] >> 4) & M1;
+                op[t][3][i] = (wd[i] >> 6) & M1;
+              }
+            }
+            // two column blocks at a time, field by field: consecutive MMAs go to different accumulators (four
+            // independent chains), so none waits for the one before it; a pair's epilogue follows its MMAs, so
+            // it can run under the next pair's
+            take_scales(sb * 2 + gi, gi == 1);
+#pragma unroll
+            for (int b0 = 0; b0 < NB; b0 += 2) {
+              if (b0 > 0 && b0 * TPB >= mc) continue;  // a short last pass: no token rows in this pair of blocks
+              uint32_t bq[2][4][2];  // [block][field][b0, b1]
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const uint32_t ba = bgrp + (uint32_t)(b0 + j) * bblock;
+                const uint4 q0 = lds128(ba), q1 = lds128(ba + 64);
+                bq[j][0][0] = q0.x; bq[j][0][1] = q0.y; bq[j][1][0] = q0.z; bq[j][1][1] = q0.w;
+                bq[j][2][0] = q1.x; bq[j][2][1] = q1.y; bq[j][3][0] = q1.z; bq[j][3][1] = q1.w;
+              }
+              int acc[RW][2][4];
+#pragma unroll
+              for (int f = 0; f < 4; ++f)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                  for (int t = 0; t < RW; ++t) {
+                    if (f == 0) mma_u8s8<true>(acc[t][j], op[t][f][0], op[t][f][1], op[t][f][2], op[t][f][3], bq[j][f][0], bq[j][f][1]);
+                    else mma_u8s8<false>(acc[t][j], op[t][f][0], op[t][f][1], op[t][f][2], op[t][f][3], bq[j][f][0], bq[j][f][1]);
+                  }
+              epilogue_pair(sb * 2 + gi, b0, acc);
+            }
+          } else {
+            const uint4 w_lo = w_lo2[u][0], w_hi = w_hi2[u][0];
+            const uint32_t l0 = gi ? w_lo.z : w_lo.x, l1 = gi ? w_lo.w : w_lo.y, h0 = gi ? w_hi.z : w_hi.x, h1 = gi ? w_hi.w : w_hi.y;
+            const uint32_t l0s = l0 >> 4, l1s = l1 >> 4, h0s = h0 >> 4, h1s = h1 >> 4;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+              const uint32_t ba = bgrp + (uint32_t)b * bblock;
+              const uint4 q0 = lds128(ba), q1 = lds128(ba + 64);
+              if (fresh) {
+                mma_u8s8<true>(accA[0][b], l0 & M1, h0 & M1, l1 & M1, h1 & M1, q0.x, q0.y);
+                mma_u8s8<true>(accB[b], l0 & M4, h0 & M4, l1 & M4, h1 & M4, q0.z, q0.w);
+              } else {
+                mma_u8s8<false>(accA[0][b], l0 & M1, h0 & M1, l1 & M1, h1 & M1, q0.x, q0.y);
+                mma_u8s8<false>(accB[b], l0 & M4, h0 & M4, l1 & M4, h1 & M4, q0.z, q0.w);
+              }
+              mma_u8s8<false>(accA[0][b], l0s & M1, h0s & M1, l1s & M1, h1s & M1, q1.x, q1.y);
+              mma_u8s8<false>(accB[b], l0s & M4, h0s & M4, l1s & M4, h1s & M4, q1.z, q1.w);
+            }
+          }
+          if (!ONEACC && phase == GS - 1) {
+            take_scales(sb * 2 + gi - (GS - 1), gi == 1);
+            epilogue(sb * 2 + gi - (GS - 1));
+          }
+        }
+      }
+    }
+  }
+  // the quad's lanes hold the partial sums of their group slots
+#pragma unroll
+  for (int t = 0; t < RW; ++t)
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (GS >= 2) y[t][b][i] += __shfl_xor_sync(0xffffffffu, y[t][b][i], 1);
+        if (GS == 4) y[t][b][i] += __shfl_xor_sync(0xffffffffu, y[t][b][i], 2);
+      }
+  if (slot_c == 0) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int tok = b * TPB + tok_c;
+      if (tok < mc) {
+        const float f = xexp[tok];
+#pragma unroll
+        for (int i = 0; i < 2 * RW; ++i) {
+          const int n = n_first + 8 * i;
+          if (n < p.N) {
+            const float v = y[i >> 1][b][i & 1] * f;
+            const int64_t o = (m0 + tok) * p.N + n;
+            if (p.out_dtype == DST_OUT_F32) {
+              float* out = static_cast<float*>(p.out);
+              out[o] = p.accumulate ? out[o] + v : v;
+            } else if (p.out_dtype == DST_OUT_BF16) {
+              static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
+            } else {
+              static_cast<__half*>(p.out)[o] = __float2half_rn(v);
+            }
+          }
+        }
+      }
+    }
+  }
+  ring.slot = sbase;
+  ring.ph = ph;
+  return true;
+}
+
 template <int GS, int NB, int CW, int RW, typename XT>
 __global__ void __launch_bounds__((CW + 1) * 32, dc_min_blocks(NB, CW))
 decode_kernel(const DecodeParams p) {
-  constexpr int MT = 4 * NB / GS;  // token rows per pass
-  constexpr int TPB = 4 / GS;      // token rows per column block
+  constexpr int MT = GS == 0 ? 4 : 4 * NB / GS;  // token rows per pass
   constexpr int THREADS = (CW + 1) * 32;
-  constexpr int RI = CW * RW * 16;  // weight rows of an item
+  constexpr int RI = CW * RW * 16;  // weight rows of a unit
   constexpr int PART = dc_part(CW * RW), SLOT_DATA = dc_slot_data(CW * RW), SLOT = dc_slot(CW * RW);
-  constexpr bool ONEACC = RW > 1;
   static_assert(GS == 1 || NB == 1, "column blocks only with one scale group per MMA");
   static_assert(RW == 1 || NB % 2 == 0, "two-tile warps take the column blocks in pairs");
-  static_assert(RI == 64 || RI == 128 || RI == 256, "an item is half a tile, a tile or two tiles");
+  static_assert(RI == 64 || RI == 128 || RI == 256, "a unit is half a tile, a tile or two tiles");
   extern __shared__ __align__(128) uint8_t dsm[];
   uint8_t* ring = dsm;                                           // p.ring x SLOT: [two parts][full barrier][empty barrier]
   uint8_t* zero = ring + p.ring * SLOT;                          // DC_ZERO
@@ -363,60 +720,60 @@ decode_kernel(const DecodeParams p) {
   for (int i = threadIdx.x; i < DC_ZERO / 4; i += THREADS) reinterpret_cast<uint32_t*>(zero)[i] = 0u;
   __syncthreads();
 
-  // contiguous, equally sized (+-1) range of items for this CTA
-  const long long items = (long long)p.E * items_per_expert<RI>(p.NT);
-  const long long i0 = items * blockIdx.x / gridDim.x, i1 = items * (blockIdx.x + 1) / gridDim.x;
+  __shared__ long long scan_s[CW + 1];
+  __shared__ UnitRun run_s;
+  find_run<MT, RI, THREADS>(p, scan_s, &run_s);
+  const long long n_units = run_s.count;
 
   if (warp == CW) {
     // ------------------------------------------------------------------ producer: packed slabs -> ring
-    if (lane == 0) {
-      const uint32_t ring_a = smem_u32(ring), ring_end = ring_a + p.ring * SLOT;
-      uint32_t sbase = ring_a, ph = 0;
-      bool ok = true;
-      for (long long item = i0; ok && item < i1; ++item) {
-        const Item it = item_of<RI>(p, item);
-        const int passes = (int)((it.rb - it.ra + MT - 1) / MT);
-        // the item's rows inside the slab of their tile; 256 rows: two whole tiles (the second may not exist)
+    // the whole warp walks the units (the walk uses warp votes); lane 0 waits and copies
+    const uint32_t ring_a = smem_u32(ring), ring_end = ring_a + p.ring * SLOT;
+    uint32_t sbase = ring_a, ph = 0;
+    bool ok = true;
+    UnitWalk<MT, RI> walk;
+    if (n_units > 0) walk.start(p, run_s.e, run_s.local);
+    for (long long i = 0; i < n_units; ++i) {
+      if (lane == 0 && ok) {
+        const Unit& it = walk.u;
+        // the unit's rows inside the slab of their tile; 256 rows: two whole tiles (the second may not exist)
         const int tile = it.n0 >> 7;
         const int64_t off0 = (((int64_t)it.e * p.NT + tile) * p.S) * 8192 + (it.n0 & 127) * 64;
         const bool two = RI == 256 && tile + 1 < p.NT;
         const int64_t tile_step = (int64_t)p.S * 8192;
-        for (int ps = 0; ok && ps < passes; ++ps)
-          for (int term = 0; ok && term < p.n_terms; ++term)
-            for (int sb = 0; sb < p.S; sb += 2) {
-              if (!mbar_wait<DC_PRODUCER_SLEEP>(sbase + SLOT_DATA + 8, ph ^ 1u, abort_flag)) { ok = false; break; }
-              const uint32_t full = sbase + SLOT_DATA;
-              const uint8_t* src = p.tiled[term] + off0 + (int64_t)sb * 8192;
-              if (RI == 256) {
-                mbar_arrive_expect_tx(full, two ? SLOT_DATA : SLOT_DATA / 2);
-                bulk_load(sbase, src, 8192, full);
-                bulk_load(sbase + PART, src + 8192, 8192, full);
-                if (two) {
-                  bulk_load(sbase + 8192, src + tile_step, 8192, full);
-                  bulk_load(sbase + PART + 8192, src + tile_step + 8192, 8192, full);
-                }
-              } else {
-                mbar_arrive_expect_tx(full, SLOT_DATA);
-                bulk_load(sbase, src, PART, full);
-                bulk_load(sbase + PART, src + 8192, PART, full);
+        for (int term = 0; ok && term < p.n_terms; ++term)
+          for (int sb = 0; sb < p.S; sb += 2) {
+            if (!mbar_wait<DC_PRODUCER_SLEEP>(sbase + SLOT_DATA + 8, ph ^ 1u, abort_flag)) { ok = false; break; }
+            const uint32_t full = sbase + SLOT_DATA;
+            const uint8_t* src = p.tiled[term] + off0 + (int64_t)sb * 8192;
+            if (RI == 256) {
+              mbar_arrive_expect_tx(full, two ? SLOT_DATA : SLOT_DATA / 2);
+              bulk_load(sbase, src, 8192, full);
+              bulk_load(sbase + PART, src + 8192, 8192, full);
+              if (two) {
+                bulk_load(sbase + 8192, src + tile_step, 8192, full);
+                bulk_load(sbase + PART + 8192, src + tile_step + 8192, 8192, full);
               }
-              sbase += SLOT;
-              if (sbase == ring_end) { sbase = ring_a; ph ^= 1u; }
+            } else {
+              mbar_arrive_expect_tx(full, SLOT_DATA);
+              bulk_load(sbase, src, PART, full);
+              bulk_load(sbase + PART, src + 8192, PART, full);
             }
+            sbase += SLOT;
+            if (sbase == ring_end) { sbase = ring_a; ph ^= 1u; }
+          }
       }
+      if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
+      if (i + 1 < n_units) walk.next(p);
     }
   } else {
     // ------------------------------------------------------------------ consumers
-    const int g8 = lane >> 2, c = lane & 3;
-    const int swz = (g8 >> 1) & 3;
-    // this lane's unit of row g8 of the warp's first 16-row tile; row g8 + 8: + 512; the second tile: + 1024
-    const uint32_t a_off = (uint32_t)((warp * 16 * RW + g8) * 64 + ((c ^ swz) << 4));
-    const uint32_t ring_a = smem_u32(ring), zero_a = smem_u32(zero), xs_a = smem_u32(xs);
-    // B column of this lane: pair g8 / 2, part g8 & 1; C columns of this lane: pair c
-    const int col_pair = g8 >> 1, col_part = g8 & 1;
-    const int tok_c = c / GS, slot_c = c % GS;  // (+ b * TPB) the token and the group slot of this lane's C columns
-    const uint32_t ring_end = ring_a + p.ring * SLOT;
-    uint32_t sbase = ring_a, ph = 0, stage_ph = 0, rows_ph = 0;  // the current ring slot and the parity of its "full" phase
+    const uint32_t zero_a = smem_u32(zero), xs_a = smem_u32(xs);
+    RingPos pos;
+    pos.base = pos.slot = smem_u32(ring);
+    pos.end = pos.base + p.ring * SLOT;
+    pos.ph = 0;
+    uint32_t stage_ph = 0, rows_ph = 0;
     int staged_e = -1;
     int64_t staged_m0 = -1;
     auto consumer_sync = [&]() -> bool {
@@ -428,275 +785,45 @@ decode_kernel(const DecodeParams p) {
       return r;
     };
 
-    for (long long item = i0; item < i1; ++item) {
-      const Item it = item_of<RI>(p, item);
-      const int n_first = it.n0 + warp * 16 * RW + g8;  // this lane's output rows: n_first + 8 i, i < 2 RW
-      for (int64_t m0 = it.ra; m0 < it.rb; m0 += MT) {
-        const int mc = (int)(it.rb - m0 < MT ? it.rb - m0 : MT);
-        if (staged_e != it.e || staged_m0 != m0) {
-          // every consumer is done with the previous rows; then stage; then everyone sees the new ones
-          if (!consumer_sync()) goto aborted;  // every consumer is done with the previous rows
-          if (p.q_rows != nullptr) {
-            // quantised ahead of this kernel: one thread has the rows copied in (bulk copies onto the staging barrier), the
-            // others fetch the small per-(token, group) sums and the row factors
-            if (warp == 0 && lane == 0) {
-              const uint32_t bar = smem_u32(&bar_rows);
-              mbar_arrive_expect_tx(bar, (uint32_t)mc * 2u * (uint32_t)p.K);
-              for (int m = 0; m < 2 * mc; ++m)
-                bulk_load(xs_a + (uint32_t)m * (uint32_t)p.xstride, p.q_rows + ((size_t)m0 * 2 + m) * p.K, (uint32_t)p.K, bar);
-            }
-            for (int m = warp; m < MT; m += CW)
-              for (int g = lane; g < p.G; g += 32) xsum4[m * p.GP + g] = m < mc ? p.q_xsum4[(m0 + m) * p.G + g] : 0;
-            if (threadIdx.x < MT) xexp[threadIdx.x] = threadIdx.x < mc ? p.q_xexp[m0 + threadIdx.x] : 0.f;
-            if (!mbar_wait(smem_u32(&bar_rows), rows_ph, abort_flag)) goto aborted;
-            rows_ph ^= 1u;
-          } else if (!stage_tokens<MT, CW>(p, static_cast<const XT*>(p.x), m0, mc, xs, (size_t)p.xstride, xsum4, p.GP, xexp, xinv, consumer_sync)) {
-            goto aborted;
+    UnitWalk<MT, RI> walk;
+    if (n_units > 0) walk.start(p, run_s.e, run_s.local);
+    for (long long i = 0; i < n_units; ++i) {
+      if (i > 0) walk.next(p);
+      const Unit& it = walk.u;
+      const int64_t m0 = it.m0;
+      const int mc = (int)(it.rb - m0 < MT ? it.rb - m0 : MT);
+      if (staged_e != it.e || staged_m0 != m0) {
+        // every consumer is done with the previous rows; then stage; then everyone sees the new ones
+        if (!consumer_sync()) goto aborted;  // every consumer is done with the previous rows
+        if (p.q_rows != nullptr) {
+          // quantised ahead of this kernel: one thread has the rows copied in (bulk copies onto the staging barrier), the
+          // others fetch the small per-(token, group) sums and the row factors
+          if (warp == 0 && lane == 0) {
+            const uint32_t bar = smem_u32(&bar_rows);
+            mbar_arrive_expect_tx(bar, (uint32_t)mc * 2u * (uint32_t)p.K);
+            for (int m = 0; m < 2 * mc; ++m)
+              bulk_load(xs_a + (uint32_t)m * (uint32_t)p.xstride, p.q_rows + ((size_t)m0 * 2 + m) * p.K, (uint32_t)p.K, bar);
           }
-          if (!consumer_sync()) goto aborted;
-          staged_e = it.e;
-          staged_m0 = m0;
+          for (int m = warp; m < MT; m += CW)
+            for (int g = lane; g < p.G; g += 32) xsum4[m * p.GP + g] = m < mc ? p.q_xsum4[(m0 + m) * p.G + g] : 0;
+          if (threadIdx.x < MT) xexp[threadIdx.x] = threadIdx.x < mc ? p.q_xexp[m0 + threadIdx.x] : 0.f;
+          if (!mbar_wait(smem_u32(&bar_rows), rows_ph, abort_flag)) goto aborted;
+          rows_ph ^= 1u;
+        } else if (!stage_tokens<MT, CW>(p, static_cast<const XT*>(p.x), m0, mc, xs, (size_t)p.xstride, xsum4, p.GP, xexp, xinv, consumer_sync)) {
+          goto aborted;
         }
-        // B pointers. Shared columns (GS > 1): for phase s (= group % GS) the lane reads its column's staged row when
-        // the column's pair belongs to that phase and its token exists, else the zeros. One group per MMA (GS == 1):
-        // column pair j of block b is token 4 b + j; the columns of tokens that do not exist read whatever the staged
-        // rows hold there (integers: an MMA column only reaches its own outputs, which are not stored).
-        constexpr int NPTR = GS > 1 ? GS : 1;
-        uint32_t bbase[NPTR], bstep[NPTR];
-        uint32_t bblock = 0;  // GS == 1: bytes between the staged rows of consecutive column blocks
-        if (GS > 1) {
-#pragma unroll
-          for (int s = 0; s < NPTR; ++s) {
-            const int tok = col_pair / GS;
-            const bool act = (col_pair % GS) == s && tok < mc;
-            bbase[s] = act ? xs_a + (uint32_t)(2 * tok + col_part) * (uint32_t)p.xstride + (uint32_t)c * 16u : zero_a;
-            bstep[s] = act ? 256u : 0u;
-          }
-        } else {
-          bbase[0] = xs_a + (uint32_t)(2 * col_pair + col_part) * (uint32_t)p.xstride + (uint32_t)c * 16u;
-          bstep[0] = 256u;
-          bblock = 8u * (uint32_t)p.xstride;
-        }
-        float y[RW][NB][2];
-#pragma unroll
-        for (int t = 0; t < RW; ++t)
-#pragma unroll
-          for (int b = 0; b < NB; ++b) y[t][b][0] = y[t][b][1] = 0.f;
-
-        for (int term = 0; term < p.n_terms; ++term) {
-          // scale rows of this lane's outputs (rows beyond N read row 0 and are not stored)
-          const __half* srow[2 * RW];
-#pragma unroll
-          for (int i = 0; i < 2 * RW; ++i) {
-            const int n = n_first + 8 * i;
-            srow[i] = p.scale[term] + ((int64_t)it.e * p.N + (n < p.N ? n : 0)) * p.G;
-          }
-          int accA[1][ONEACC ? 1 : NB][4], accB[ONEACC ? 1 : NB][4];  // the x1 and the x4 fields' sums (one tile per warp)
-#pragma unroll
-          for (int b = 0; b < (ONEACC ? 1 : NB); ++b)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) accA[0][b][i] = accB[b][i] = 0;
-          // scales of the lane's group of the next epilogue, requested ahead: a block of GS groups (shared columns), or
-          // two groups at a time, two groups ahead, as one 32-bit load per output row (GS == 1; G is a multiple of 4)
-          auto scale_at = [&](const __half* s, int grp) { return grp < p.G ? __half2float(s[grp]) : 0.f; };
-          auto scale2_at = [&](const __half* s, int grp) { return grp < p.G ? *reinterpret_cast<const uint32_t*>(s + grp) : 0u; };
-          float s_next[2 * RW];
-          uint32_t s2_cur[2 * RW], s2_next[2 * RW];
-#pragma unroll
-          for (int i = 0; i < 2 * RW; ++i) {
-            s_next[i] = GS > 1 ? scale_at(srow[i], slot_c) : 0.f;
-            s2_cur[i] = 0u;
-            s2_next[i] = GS == 1 ? scale2_at(srow[i], 0) : 0u;
-          }
-          // Epilogue of the block of GS groups whose first group is g_first: this lane's group is g_first + slot_c.
-          // First the group's scales (odd: g_first & 1 as a compile-time value) ...
-          float sc[2 * RW];
-          auto take_scales = [&](int g_first, bool odd) {
-            const int g_mine = g_first + slot_c;
-#pragma unroll
-            for (int i = 0; i < 2 * RW; ++i) {
-              if (GS > 1) {
-                sc[i] = s_next[i];
-                s_next[i] = scale_at(srow[i], g_mine + GS);
-              } else {
-                if (!odd) {
-                  s2_cur[i] = s2_next[i];
-                  s2_next[i] = scale2_at(srow[i], g_first + 2);
-                }
-                const __half2 h2 = *reinterpret_cast<const __half2*>(&s2_cur[i]);
-                sc[i] = odd ? __high2float(h2) : __low2float(h2);
-              }
-            }
-          };
-          // ... then per column block: 4 * sum_k u_k q_k - 4 * sum_k q_k as one integer, converted and multiplied.
-          // x1 / x4 accumulators: 128 * (4 A_hi + B_hi) + (4 A_lo + B_lo)
-          auto epilogue = [&](int g_first) {
-            const int g_mine = g_first + slot_c;
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-              const int xs4 = g_mine < p.G ? xsum4[(b * TPB + tok_c) * p.GP + g_mine] : 0;
-              const int v_lo = ((((accA[0][b][0] << 2) + accB[b][0]) << 7) + ((accA[0][b][1] << 2) + accB[b][1])) - xs4;
-              const int v_hi = ((((accA[0][b][2] << 2) + accB[b][2]) << 7) + ((accA[0][b][3] << 2) + accB[b][3])) - xs4;
-              y[0][b][0] = fmaf(sc[0], (float)v_lo, y[0][b][0]);
-              y[0][b][1] = fmaf(sc[1], (float)v_hi, y[0][b][1]);
-            }
-          };
-          // plain digits, one accumulator set, a pair of column blocks: 4 * (128 * A_hi + A_lo)
-          auto epilogue_pair = [&](int g, int b0, const int (&acc)[RW][2][4]) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const int xs4 = xsum4[((b0 + j) * TPB + tok_c) * p.GP + g];
-#pragma unroll
-              for (int t = 0; t < RW; ++t) {
-                const int v_lo = (acc[t][j][0] << 9) + ((acc[t][j][1] << 2) - xs4);
-                const int v_hi = (acc[t][j][2] << 9) + ((acc[t][j][3] << 2) - xs4);
-                y[t][b0 + j][0] = fmaf(sc[2 * t], (float)v_lo, y[t][b0 + j][0]);
-                y[t][b0 + j][1] = fmaf(sc[2 * t + 1], (float)v_hi, y[t][b0 + j][1]);
-              }
-            }
-          };
-
-          // two superblocks (one ring slot, four scale groups) per iteration: the phase of every group (group % GS) is a
-          // compile-time value, and the barrier traffic and slot arithmetic are paid once per 2 KB of a 16-row tile
-          for (int sb0 = 0; sb0 < p.S; sb0 += 2) {
-            if (!mbar_wait(sbase + SLOT_DATA, ph, abort_flag)) goto aborted;
-            const uint32_t sa = sbase + a_off;
-            // [superblock][tile]: rows g8 and g8 + 8. One tile per warp: both superblocks' words are read up front and the
-            // slot is handed back at once; two tiles: the second superblock's words are read after the first one's MMAs
-            // (registers), and the slot goes back then
-            uint4 w_lo2[2][RW], w_hi2[2][RW];
-            const uint32_t slot_bar = sbase + SLOT_DATA + 8;
-#pragma unroll
-            for (int u = 0; u < (RW == 1 ? 2 : 1); ++u)
-#pragma unroll
-              for (int t = 0; t < RW; ++t) {
-                w_lo2[u][t] = lds128(sa + u * PART + t * 1024);
-                w_hi2[u][t] = lds128(sa + u * PART + t * 1024 + 512);
-              }
-            if (RW == 1) mbar_arrive(slot_bar);  // every lane arrives for itself: its loads above are done
-            sbase += SLOT;
-            if (sbase == ring_end) { sbase = ring_a; ph ^= 1u; }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int sb = sb0 + u;
-              if (RW > 1 && u == 1) {
-#pragma unroll
-                for (int t = 0; t < RW; ++t) {
-                  w_lo2[1][t] = lds128(sa + PART + t * 1024);
-                  w_hi2[1][t] = lds128(sa + PART + t * 1024 + 512);
-                }
-                mbar_arrive(slot_bar);
-              }
-#pragma unroll
-              for (int gi = 0; gi < 2; ++gi) {
-                constexpr uint32_t M1 = 0x03030303u, M4 = 0x0c0c0c0cu;
-                const int phase = (u * 2 + gi) % GS;   // group % GS
-                const bool fresh = phase == 0;         // first group of an epilogue block: the accumulators restart
-                const uint32_t bgrp = bbase[phase] + (uint32_t)sb * bstep[phase] + (uint32_t)gi * 128u;
-                if (ONEACC) {
-                  // operands of both tiles: [tile][field][a0..a3]
-                  uint32_t op[RW][4][4];
-#pragma unroll
-                  for (int t = 0; t < RW; ++t) {
-                    const uint4 w_lo = w_lo2[u][t], w_hi = w_hi2[u][t];
-                    const uint32_t wd[4] = {gi ? w_lo.z : w_lo.x, gi ? w_hi.z : w_hi.x, gi ? w_lo.w : w_lo.y, gi ? w_hi.w : w_hi.y};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                      op[t][0][i] = wd[i] & M1;
-                      op[t][1][i] = (wd[i] >> 2) & M1;
-                      op[t][2][i] = (wd[i] >> 4) & M1;
-                      op[t][3][i] = (wd[i] >> 6) & M1;
-                    }
-                  }
-                  // two column blocks at a time, field by field: consecutive MMAs go to different accumulators (four
-                  // independent chains), so none waits for the one before it; a pair's epilogue follows its MMAs, so
-                  // it can run under the next pair's
-                  take_scales(sb * 2 + gi, gi == 1);
-#pragma unroll
-                  for (int b0 = 0; b0 < NB; b0 += 2) {
-                    if (b0 > 0 && b0 * TPB >= mc) continue;  // a short last pass: no token rows in this pair of blocks
-                    uint32_t bq[2][4][2];  // [block][field][b0, b1]
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                      const uint32_t ba = bgrp + (uint32_t)(b0 + j) * bblock;
-                      const uint4 q0 = lds128(ba), q1 = lds128(ba + 64);
-                      bq[j][0][0] = q0.x; bq[j][0][1] = q0.y; bq[j][1][0] = q0.z; bq[j][1][1] = q0.w;
-                      bq[j][2][0] = q1.x; bq[j][2][1] = q1.y; bq[j][3][0] = q1.z; bq[j][3][1] = q1.w;
-                    }
-                    int acc[RW][2][4];
-#pragma unroll
-                    for (int f = 0; f < 4; ++f)
-#pragma unroll
-                      for (int j = 0; j < 2; ++j)
-#pragma unroll
-                        for (int t = 0; t < RW; ++t) {
-                          if (f == 0) mma_u8s8<true>(acc[t][j], op[t][f][0], op[t][f][1], op[t][f][2], op[t][f][3], bq[j][f][0], bq[j][f][1]);
-                          else mma_u8s8<false>(acc[t][j], op[t][f][0], op[t][f][1], op[t][f][2], op[t][f][3], bq[j][f][0], bq[j][f][1]);
-                        }
-                    epilogue_pair(sb * 2 + gi, b0, acc);
-                  }
-                } else {
-                  const uint4 w_lo = w_lo2[u][0], w_hi = w_hi2[u][0];
-                  const uint32_t l0 = gi ? w_lo.z : w_lo.x, l1 = gi ? w_lo.w : w_lo.y, h0 = gi ? w_hi.z : w_hi.x, h1 = gi ? w_hi.w : w_hi.y;
-                  const uint32_t l0s = l0 >> 4, l1s = l1 >> 4, h0s = h0 >> 4, h1s = h1 >> 4;
-#pragma unroll
-                  for (int b = 0; b < NB; ++b) {
-                    const uint32_t ba = bgrp + (uint32_t)b * bblock;
-                    const uint4 q0 = lds128(ba), q1 = lds128(ba + 64);
-                    if (fresh) {
-                      mma_u8s8<true>(accA[0][b], l0 & M1, h0 & M1, l1 & M1, h1 & M1, q0.x, q0.y);
-                      mma_u8s8<true>(accB[b], l0 & M4, h0 & M4, l1 & M4, h1 & M4, q0.z, q0.w);
-                    } else {
-                      mma_u8s8<false>(accA[0][b], l0 & M1, h0 & M1, l1 & M1, h1 & M1, q0.x, q0.y);
-                      mma_u8s8<false>(accB[b], l0 & M4, h0 & M4, l1 & M4, h1 & M4, q0.z, q0.w);
-                    }
-                    mma_u8s8<false>(accA[0][b], l0s & M1, h0s & M1, l1s & M1, h1s & M1, q1.x, q1.y);
-                    mma_u8s8<false>(accB[b], l0s & M4, h0s & M4, l1s & M4, h1s & M4, q1.z, q1.w);
-                  }
-                }
-                if (!ONEACC && phase == GS - 1) {
-                  take_scales(sb * 2 + gi - (GS - 1), gi == 1);
-                  epilogue(sb * 2 + gi - (GS - 1));
-                }
-              }
-            }
-          }
-        }
-        // the quad's lanes hold the partial sums of their group slots
-#pragma unroll
-        for (int t = 0; t < RW; ++t)
-#pragma unroll
-          for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              if (GS >= 2) y[t][b][i] += __shfl_xor_sync(0xffffffffu, y[t][b][i], 1);
-              if (GS == 4) y[t][b][i] += __shfl_xor_sync(0xffffffffu, y[t][b][i], 2);
-            }
-        if (slot_c == 0) {
-#pragma unroll
-          for (int b = 0; b < NB; ++b) {
-            const int tok = b * TPB + tok_c;
-            if (tok < mc) {
-              const float f = xexp[tok];
-#pragma unroll
-              for (int i = 0; i < 2 * RW; ++i) {
-                const int n = n_first + 8 * i;
-                if (n < p.N) {
-                  const float v = y[i >> 1][b][i & 1] * f;
-                  const int64_t o = (m0 + tok) * p.N + n;
-                  if (p.out_dtype == DST_OUT_F32) {
-                    float* out = static_cast<float*>(p.out);
-                    out[o] = p.accumulate ? out[o] + v : v;
-                  } else if (p.out_dtype == DST_OUT_BF16) {
-                    static_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(v);
-                  } else {
-                    static_cast<__half*>(p.out)[o] = __float2half_rn(v);
-                  }
-                }
-              }
-            }
-          }
-        }
+        if (!consumer_sync()) goto aborted;
+        staged_e = it.e;
+        staged_m0 = m0;
+      }
+      if constexpr (GS == 0) {
+        // one, two, or three and four token rows: as many scale groups share the columns as the rows leave room for
+        const bool done = mc == 1   ? run_pass<4, 1, CW, RW>(p, it, mc, pos, xs_a, zero_a, xsum4, xexp, abort_flag)
+                          : mc == 2 ? run_pass<2, 1, CW, RW>(p, it, mc, pos, xs_a, zero_a, xsum4, xexp, abort_flag)
+                                    : run_pass<1, 1, CW, RW>(p, it, mc, pos, xs_a, zero_a, xsum4, xexp, abort_flag);
+        if (!done) goto aborted;
+      } else {
+        if (!run_pass<GS, NB, CW, RW>(p, it, mc, pos, xs_a, zero_a, xsum4, xexp, abort_flag)) goto aborted;
       }
     }
   aborted:;  // a bounded wait gave up (the abort flag is up): leave without touching anything else
@@ -715,13 +842,13 @@ decode_kernel(const DecodeParams p) {
 // Shared memory of a CTA apart from its ring
 template <int GS, int NB, int CW>
 size_t decode_fixed_smem(const DecodeParams& p) {
-  constexpr int MT = 4 * NB / GS;
+  constexpr int MT = GS == 0 ? 4 : 4 * NB / GS;
   return DC_ZERO + (size_t)2 * MT * p.xstride + (size_t)MT * p.GP * 4 + (size_t)MT * 4 * (1 + CW);
 }
 
 template <int GS, int NB, int CW, int RW, typename XT>
 int launch_one(DecodeParams p, int sms, cudaStream_t stream) {
-  constexpr int THREADS = (CW + 1) * 32, RI = CW * RW * 16, SLOT = dc_slot(CW * RW);
+  constexpr int THREADS = (CW + 1) * 32, RI = CW * RW * 16, SLOT = dc_slot(CW * RW), MT = GS == 0 ? 4 : 4 * NB / GS;
   const size_t budget = 226 * 1024, fixed = decode_fixed_smem<GS, NB, CW>(p);  // 227 KB per CTA less the static barriers
   if (fixed + (size_t)2 * SLOT > budget) return DST_ERR_UNSUPPORTED;
   // small CTAs: the full ring, and as many CTAs per SM as fit; the 256-row CTA: one per SM, the ring takes what is left
@@ -730,12 +857,14 @@ int launch_one(DecodeParams p, int sms, cudaStream_t stream) {
   const size_t smem = (size_t)p.ring * SLOT + fixed;
   auto kernel = decode_kernel<GS, NB, CW, RW, XT>;
   DST_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  DST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem));
-  if (per_sm < 1) return DST_ERR_UNSUPPORTED;
-  const long long items = (long long)p.E * items_per_expert<RI>(p.NT);
+  // resident CTAs per SM: what the launch bounds promise, or fewer by shared memory (1 KB per CTA is the system's)
+  const size_t fit = (size_t)(228 * 1024) / (smem + 1024 + 256);
+  const int per_sm = fit < 1 ? 1 : (fit < (size_t)dc_min_blocks(NB, CW) ? (int)fit : dc_min_blocks(NB, CW));
+  // units at most: every token row a pass of its own, or every expert with rows in them and full passes
+  const long long passes = p.T < p.E ? (long long)p.T : (long long)p.E + p.T / MT;
+  const long long units = passes * blocks_per_expert<RI>(p.NT);
   const long long want = (long long)sms * per_sm;
-  const int grid = (int)(items < want ? items : want);
+  const int grid = (int)(units < want ? units : want);
   kernel<<<grid, THREADS, smem, stream>>>(p);
   DST_CUDA_TRY(cudaGetLastError());
   return DST_OK;
@@ -745,21 +874,22 @@ int launch_one(DecodeParams p, int sms, cudaStream_t stream) {
 #define DC_WIDE_FROM 5
 #endif
 template <typename XT>
-int launch_rows(const DecodeParams& p, int64_t rows_hint, int sms, cudaStream_t stream) {
-  if (rows_hint <= 1) return launch_one<4, 1, 4, 1, XT>(p, sms, stream);
-  if (rows_hint <= 2) return launch_one<2, 1, 4, 1, XT>(p, sms, stream);
-  if (rows_hint < DC_WIDE_FROM && rows_hint <= 4) return launch_one<1, 1, 4, 1, XT>(p, sms, stream);
+int launch_rows(const DecodeParams& p, int64_t rows_hint, bool rows_known, int sms, cudaStream_t stream) {
+  // one row per expert at most, for certain: passes of one row, the least shared memory
+  if (p.T == 1 || (rows_known && rows_hint <= 1)) return launch_one<4, 1, 4, 1, XT>(p, sms, stream);
+  // up to four: passes of up to four rows, each pass shaped by the rows it has
+  if (rows_hint < DC_WIDE_FROM && rows_hint <= 4) return launch_one<0, 1, 4, 1, XT>(p, sms, stream);
   // five or more rows: one CTA per SM whose eight consumer warps own 32 weight rows each and share the staged token
-  // rows (8, then 16 per pass), when there is a 256-row item for every SM; else the small CTAs
-  const long long wide_items = (long long)p.E * items_per_expert<256>(p.NT);
-  if (wide_items >= sms) {
+  // rows (8, then 16 per pass), when there is a 256-row unit for every SM; else the small CTAs
+  const long long wide_units = (long long)p.E * blocks_per_expert<256>(p.NT);
+  if (wide_units >= sms) {
     int rc = rows_hint <= 8 ? DST_ERR_UNSUPPORTED : launch_one<1, 4, 8, 2, XT>(p, sms, stream);
     if (rc == DST_ERR_UNSUPPORTED) rc = launch_one<1, 2, 8, 2, XT>(p, sms, stream);
     if (rc != DST_ERR_UNSUPPORTED) return rc;
   }
-  if (rows_hint <= 4) return launch_one<1, 1, 4, 1, XT>(p, sms, stream);
+  if (rows_hint <= 4) return launch_one<0, 1, 4, 1, XT>(p, sms, stream);
   const int rc = launch_one<1, 2, 4, 1, XT>(p, sms, stream);
-  return rc == DST_ERR_UNSUPPORTED ? launch_one<1, 1, 4, 1, XT>(p, sms, stream) : rc;  // 16 staged rows of a long K may not fit
+  return rc == DST_ERR_UNSUPPORTED ? launch_one<0, 1, 4, 1, XT>(p, sms, stream) : rc;  // 16 staged rows of a long K may not fit
 }
 
 }  // namespace
@@ -772,7 +902,7 @@ size_t decode_workspace_bytes(int64_t T, int64_t K) {
 }
 
 // Up to how many token rows per expert the decode GEMV beats the tcgen05 kernel (measured on 4096 x 4096 experts): 32
-// where the many-row CTAs apply (TQ2 tiles, a 256-row item for every SM; two passes of 16 rows), else 16.
+// where the many-row CTAs apply (TQ2 tiles, a 256-row unit for every SM; two passes of 16 rows), else 16.
 int64_t decode_row_limit(int fmt, int64_t E, int64_t N) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -841,9 +971,9 @@ int launch_decode(const GemmArgs& a, cudaStream_t stream) {
     p.q_xsum4 = q_xsum4;
     p.q_xexp = q_xexp;
   }
-  if (a.act_dtype == DST_ACT_BF16) return launch_rows<__nv_bfloat16>(p, rows_hint, sms, stream);
-  if (a.act_dtype == DST_ACT_F16) return launch_rows<__half>(p, rows_hint, sms, stream);
-  return launch_rows<int8_t>(p, rows_hint, sms, stream);
+  if (a.act_dtype == DST_ACT_BF16) return launch_rows<__nv_bfloat16>(p, rows_hint, a.max_rows >= 0, sms, stream);
+  if (a.act_dtype == DST_ACT_F16) return launch_rows<__half>(p, rows_hint, a.max_rows >= 0, sms, stream);
+  return launch_rows<int8_t>(p, rows_hint, a.max_rows >= 0, sms, stream);
 }
 
 // Reads and clears the decode kernel's status word (DST_OK or DST_ERR_TIMEOUT in *status).

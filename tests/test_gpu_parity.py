@@ -286,6 +286,28 @@ def test_grouped_decode_sizes_with_empty_and_ragged_experts(kb, algo, fmt):
             np.testing.assert_allclose(y[a:b], want, rtol=1e-4, atol=1e-3)
 
 
+@pytest.mark.parametrize("fmt", ["tq2", "tq1"])
+@pytest.mark.parametrize("rows", [{0: 1}, {99: 2}, {0: 2, 1: 1, 40: 4, 41: 3, 98: 9, 99: 1}, {31: 1, 32: 5, 64: 1}, {e: 1 + e % 3 for e in range(100)}])
+def test_grouped_decode_few_of_many_experts(kb, fmt, rows):
+    """A decode step whose tokens reach a few of many experts, the row counts known on the device only: every pass is
+    shaped by its rows (1, 2, 3 or 4) and the CTAs' runs are cut over the experts with rows (first, last, neighbours, 32
+    apart, all)."""
+    E, N, K = 100, 200, 1024
+    rng = np.random.default_rng(len(rows))
+    terms = make_terms(rng, N, K, 128, fmt, 2, lead=(E,))
+    counts = np.zeros(E, np.int64)
+    counts[list(rows)] = list(rows.values())
+    offsets = np.concatenate([[0], counts.cumsum()]).astype(np.int64)
+    x = O.synth_acts(rng, (int(offsets[-1]), K))
+    tiled = [kb.tile_weights(torch.from_numpy(p).to(DEV), fmt, K) for p, _ in terms]
+    y = kb.grouped_ternary_gemm_bf16(bf16_tensor(x, DEV), torch.from_numpy(offsets).to(DEV), tiled, [torch.from_numpy(s).to(DEV) for _, s in terms],
+                                     K, 128, fmt, algo="decode", validate_offsets=False).cpu().numpy()
+    assert kb.ext().dst_check_device_status(None) == 0
+    for e in rows:
+        a, b = int(offsets[e]), int(offsets[e + 1])
+        check_gemm(y[a:b], x[a:b], [(p[e], s[e]) for p, s in terms], K, 128, fmt)
+
+
 @pytest.mark.parametrize("N,K,terms_k", [(1024, 1024, 1), (384, 512, 2)])
 def test_grouped_decode_many_row_ctas(kb, N, K, terms_k):
     """Five or more rows per expert with at least one 256-row item per SM: the decode GEMV runs as one CTA per SM whose
