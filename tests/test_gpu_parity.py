@@ -308,6 +308,30 @@ def test_grouped_decode_few_of_many_experts(kb, fmt, rows):
         check_gemm(y[a:b], x[a:b], [(p[e], s[e]) for p, s in terms], K, 128, fmt)
 
 
+@pytest.mark.parametrize("fmt", ["tq2", "tq1"])
+@pytest.mark.parametrize("K,group", [(4160, 128), (2048, 256), (192, 64), (131, 64), (7, 64), (4096 + 36, 128), (1024, 192)])
+def test_int8_grouped_canonical_weights(kb, fmt, K, group):
+    """int8 activations against canonical weights and float32 scales: rows per expert around the pass sizes (8, 16, 32), an
+    empty expert, N and K off every tile, packed rows and token rows of any alignment (also one tensor off by a byte)."""
+    N = 70
+    for counts in ([1, 0, 8], [9, 2, 16], [17, 33, 70]):
+        E = len(counts)
+        rng = np.random.default_rng(K + sum(counts))
+        packed = np.stack([O.pack(O.synth_trits(rng, (N, K)), fmt) for _ in range(E)])
+        scales = rng.random((E, N, -(-K // group))).astype(np.float32) + np.float32(0.01)
+        offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+        q = rng.integers(-127, 128, (int(offsets[-1]), K)).astype(np.int8)
+        xs = rng.random(q.shape[0]).astype(np.float32) + np.float32(0.1)
+        want = O.grouped_gemm_i8(q, xs, offsets, packed, scales, K, group, fmt)
+        for shift in (0, 1):
+            buf = torch.zeros(packed.size + shift, dtype=torch.uint8, device=DEV)
+            buf[shift:] = torch.from_numpy(packed.reshape(-1)).to(DEV)
+            got = kb.grouped_ternary_gemm(torch.from_numpy(q).to(DEV), torch.from_numpy(xs).to(DEV), offsets, buf[shift:].view(packed.shape),
+                                          torch.from_numpy(scales).to(DEV), K, group, fmt)
+            # exact integer group sums, then one fp32 product and sum per group: G roundings of 2^-24 of the largest partial sum
+            np.testing.assert_allclose(got.cpu().numpy(), want, rtol=1e-5, atol=1e-5 * float(np.abs(want).max()))
+
+
 @pytest.mark.parametrize("N,K,terms_k", [(1024, 1024, 1), (384, 512, 2)])
 def test_grouped_decode_many_row_ctas(kb, N, K, terms_k):
     """Five or more rows per expert with at least one 256-row item per SM: the decode GEMV runs as one CTA per SM whose
