@@ -205,9 +205,8 @@ canonical_i8_kernel(const CanonArgs a) {
   extern __shared__ __align__(16) uint8_t ci_smem[];
   __shared__ uint32_t lut_s[FMT == 1 ? 256 * CI_LUT_REPL : 1];
   const int xstride = a.chunk + 16;                                            // two rows read together hit all banks once
-  const int steps_max = a.chunk / STEP;
   uint8_t* xs = ci_smem;                                                       // [TOK][xstride], lane order
-  int* xsum = reinterpret_cast<int*>(ci_smem + (size_t)TOK * xstride);         // [steps_max][TOK]
+  int* xsum = reinterpret_cast<int*>(ci_smem + (size_t)TOK * xstride);         // [chunk / STEP][TOK]
   float* red = reinterpret_cast<float*>(ci_smem);                              // [warps][NB * 4][32], after the last chunk
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, c = lane & 3;
   if (FMT == 1)

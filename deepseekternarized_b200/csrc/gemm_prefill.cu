@@ -7,16 +7,21 @@
 // Mapping ("swap AB"): the 128 weight rows of a tile are the MMA M dimension (TMEM lanes), the token rows of
 // one expert (up to 320 per tile) are the MMA N dimension (TMEM columns), so tiles stay full when an expert
 // has few rows and an expert with up to 320 rows has its weights dequantised ONCE per 128-row weight tile.
-// Both operands are fp16, 64 K-elements per pipeline stage:
+// Both operands are fp16, 64 K-elements per pipeline stage (128 for token tiles of at most 128 rows, the SMALL form):
 //   A (weights)      packed 8 KB slabs of the tiled layout (layout_kernels.cu) arrive by cp.async.bulk in a
-//                    small ring; 16 dequant warps turn them into scale * trit, exact in fp16, and write them
+//                    small ring; the dequant warps turn them into scale * trit, exact in fp16, and write them
 //                    with tcgen05.st straight into TENSOR MEMORY (lane = weight row, one 32-bit column = two
-//                    consecutive K elements; 32 columns per stage): the MMA takes A from TMEM, so the
+//                    consecutive K elements; 32 columns per 64 K): the MMA takes A from TMEM, so the
 //                    dequantised tile never passes through shared memory
 //   B (activations)  fp16 rows fetched by one thread with cp.async.bulk.tensor (TMA) into K-major,
 //                    128-byte-swizzled shared-memory stages (one box for up to 256 rows, two for more)
-//   D (accumulator)  fp32 in TMEM columns 0..319 (two MMAs per K step, each over half of the token rows, from two
-//                    issuing threads); columns 320..511 hold the A ring (stage s = slot s)
+//   D (accumulator)  fp32 in TMEM columns 0 .. tn_max - 1 (above 256 rows two MMAs per K step, each over half of the
+//                    rows); the columns behind hold the A ring. A and B rings have their own depths (na, nb)
+// What bounds it: up to ~128 token rows the instruction streams of the dequant warps and of the MMA issuer (130 to 500
+// cycles of tensor work per 64 K, ~470 spent), above that the tensor pipe and the drain of the one accumulator. Measured
+// on 96 experts of 4096 x 4096, one launch, this form / the one before (one 64-trit piece per group and step, two issuing
+// warps on one ring of A and B slots, digit-field tables): TQ1 64 rows 326 / 629 us, 256 rows 615 / 736; TQ2 64 rows
+// 338 / 577, 256 rows 607 / 689; two TQ2 terms 64 rows 521 / 869.
 // Shared-memory bandwidth is what bounds this kernel when A goes through shared memory (measured: the MMA
 // issuer stalled ~1100 cycles per 512-cycle stage); with A in TMEM only B is written and read there.
 // bf16 activations are converted once to fp16 with a power-of-two factor per row (exact for every
@@ -25,15 +30,14 @@
 //
 // Warp roles (896 threads, one CTA per SM, persistent over tiles):
 //   warp 0      TMA producer for B (one thread)
-//   warp 1, 3   MMA issuers (one thread each, each over half of a tile's token rows); warp 1 owns the TMEM allocation
+//   warp 1      MMA issuer (all lanes run the loop, the elected one issues); owns the TMEM allocation
 //   warp 2      bulk-copy producer of the packed slabs (one thread)
 //   warps 4-11  epilogue: TMEM -> registers -> global, two warps per TMEM lane quarter (warp id % 4) taking
 //               alternate 32-column chunks
-//   warps 12-27 dequant producers for A, in four groups of four warps: group g owns the stages with global
-//               index = g (mod 4), so four stages are dequantised at once (each warp's instruction stream is a
-//               long dependent chain; one group per stage could not keep up with the MMAs); inside a group
-//               the warp with id % 4 == q owns the 32 weight rows of TMEM lane quarter q, one thread per row
-//               per 64-trit stage
+//   warps 12-27 dequant producers for A, in four groups of four warps: group g owns the 128-trit units with index = g
+//               (mod 4), so four units are dequantised at once (each warp's instruction stream is a long dependent
+//               chain); inside a group the warp with id % 4 == q owns the 32 weight rows of TMEM lane quarter q, one
+//               thread per row. SMALL: the warps 8-11 are a fifth group, four epilogue warps drain
 // The accumulator is drained by warps that do nothing else. A variant in which the 20 dequant warps also drained
 // it (tcgen05.ld in the same, register-starved instruction stream as the dequantisation) raised "unspecified
 // launch failure" on the GPU although the same code with extra progress stores passed; tcgen05.ld writes its
@@ -44,6 +48,7 @@
 // roles leave their loops, the CTA frees TMEM and the kernel records DST_ERR_TIMEOUT in the status word.
 #include <cuda.h>
 
+#include <cmath>
 #include <cstring>
 
 #include "dst_common.cuh"
@@ -60,13 +65,23 @@ constexpr int PF_THREADS = 32 * (PF_DQ_WARP0 + PF_DQ_WARPS);
 constexpr int PF_TN_MAX = 320;               // token rows per tile at most = accumulator columns in TMEM
 constexpr int PF_A_COLS = 32;                // TMEM columns of one A stage: 64 fp16 per weight row
 constexpr int PF_MAX_STAGES = 12;            // stage ring depth at most; tn_max + depth * 32 <= 512 TMEM columns
-constexpr int PF_MAX_SLABS = 3;
-constexpr int PF_LUT_BYTES = 256 * 16 * 4;   // TQ1: 256 byte values x 16 bank replicas x 4 B
+// Barriers of stage g (slab i): entry g % 16 (i % 16) of their ring, phase g / 16, whatever the number of data slots. A parity
+// tells a phase from its neighbour only, and a dequant group jumps over the others' units to a stage up to 7 further on (a
+// slab up to 6, in tiles of few K elements); sixteen entries keep every phase that a role waits for the next one of its entry.
+constexpr uint32_t PF_BARS = 16;
+constexpr int PF_SMALL_TN = 128;             // token tiles up to this many rows: the SMALL form of the kernel
+// TQ1 selector tables (see tq1_stage_select): 64 KB where the token tiles leave room for it, else 32 KB
+enum { PF_TABLE_NONE = 0, PF_TABLE_32K = 1, PF_TABLE_64K = 2 };
+__host__ __device__ constexpr int pf_table(int fmt, int terms, bool small) {
+  return fmt != 1 ? PF_TABLE_NONE : (small && terms <= 2 ? PF_TABLE_64K : PF_TABLE_32K);
+}
 constexpr int PF_SLAB = 8192;                // one (row tile, superblock) slab of packed weights
 constexpr int PF_MAX_E = 1023;               // experts per launch: two int arrays of E + 1 entries live in shared memory
 constexpr int PF_EPI_TILE = 2048;             // bytes of an epilogue warp's transposition tile (32 token rows x 32 columns x 2 bytes)
-constexpr int PF_SMEM_MAX = 232448;          // 227 KB of shared memory per CTA
-constexpr int PF_SMEM_STATIC = 6144;         // allowance for the statically declared barriers, flags and the scatter form's row pointers
+// Shared memory is planned in addresses of the shared window, because the selector tables sit at multiples of their size.
+// The dynamic part starts behind the system's 1 KB and the static part (under 1 KB, the kernel checks it) and may reach up
+// to PF_SMEM_END: 227 KB per CTA less the static part.
+constexpr uint32_t PF_SMEM_FIRST = 1024, PF_SMEM_START = 2048, PF_SMEM_END = 232448;
 constexpr long long PF_WAIT_CYCLES = 4000000000LL;  // ~2 s
 
 __device__ int g_device_status = 0;
@@ -112,11 +127,12 @@ struct PrefillParams {
   // chosen by the host from the shared-memory budget
   int tn_max;       // token rows per tile at most (a multiple of 32, <= PF_TN_MAX): accumulator columns 0 .. tn_max - 1, the A ring after them
   int rows_hint;    // most rows an expert is expected to have (host knowledge or twice the mean), sizes tn_max
-  int nb;           // depth of the stage ring (B stage in shared memory + A slot in TMEM), 2..6
+  int nb;           // B stages in shared memory
+  int na;           // A slots in TMEM = length of the barrier rings (nb <= na): stage g uses A slot g % na and B stage g % nb
   int nslab;        // slots of the packed-slab ring, 2 or 3
+  // places in the shared window (see plan_smem): B stage ring, packed slabs, tables and epilogue tiles, selector table
+  uint32_t a_ring, a_slabs, a_front, a_table;
   int wide_drain;   // 16-bit outputs, N % 8 == 0, 16-byte aligned rows: the accumulator is drained with 128-bit stores (drain_tile_wide)
-  int small;        // token tiles of at most 128 rows: four warps drain the accumulator and the other four of that role join
-                    // the dequantisation as a fifth group (the MMAs of such tiles are short, the dequantisation is the limit)
   // Scatter of the output rows (null: rows go to `out` in place). Row r is stored at row (row_target[r] & (2^48 - 1)) of
   // peer_out[row_target[r] >> 48]: the buffers of the GPUs whose tokens the rows belong to, written from the epilogue
   // with plain stores over NVLink while the tensor pipe works on the next tile. A negative target drops the row.
@@ -149,12 +165,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // Up to PF_SPIN_TRIES try_waits in a loop written in PTX: three to five instructions per poll. The same loop in C++
-// compiles to about nine (convergence bookkeeping around a divergent loop), and with every role of the CTA polling
-// some barrier most of the time the polls were ~40 % of all instructions this kernel issued at 64 rows per expert
-// (per-opcode counters: 147 try_waits, 350 branches, 135 BSSY/BSYNC pairs and 138 YIELDs per 64-K stage).
-#ifndef PF_SPLIT_MIN
-#define PF_SPLIT_MIN 64
-#endif
+// compiles to about nine (convergence bookkeeping around a divergent loop). A suspend-time hint does not reduce the polls
+// (103 per 64 K elements with one of 20 us, 124 without).
 #ifndef PF_SPIN_TRIES
 #define PF_SPIN_TRIES 64
 #endif
@@ -183,20 +195,20 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
-// Bounded wait: false when the abort flag is up or ~2 s of clock cycles have passed (checked between bursts of polls).
-// BACKOFF sleeps between bursts: for roles that wait long, so their polling does not take issue slots from the dequant warps.
+// Bounded wait: false when the abort flag is up or ~2 s of clock cycles have passed.
+// BACKOFF sleeps between polls: for roles that wait long.
 template <bool BACKOFF = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_test(bar, parity)) return true;
   const long long t0 = clock64();
   for (;;) {
-    if (mbar_spin(bar, parity)) return true;
+    if (BACKOFF ? mbar_test(bar, parity) : mbar_spin(bar, parity)) return true;
     if (*abort_flag) return false;
     if (clock64() - t0 > g_wait_cycles) {
       *abort_flag = 1;
       return false;
     }
-    if (BACKOFF) __nanosleep(40);
+    if (BACKOFF) __nanosleep(200);
   }
 }
 
@@ -206,14 +218,23 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
          ((uint64_t)2 << 61);
 }
 
-// tcgen05.mma: A operand from tensor memory (lane = row, 32-bit column = 2 K elements), B from shared memory.
-// Executed by a whole (converged) warp: one elected lane issues. The issuing warps run their loops with
-// all 32 lanes so that addresses and descriptors are warp-uniform values (a single-lane branch keeps them in
-// per-thread registers and every MMA then pays for moving them to the uniform registers the instruction reads).
-__device__ __forceinline__ void umma_f16_ts_elect(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p, e;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|e, 0xffffffff;\n"
-               "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+// The four tcgen05.mma (K = 16 each) of 64 K elements: A from tensor memory (lane = row, 32-bit column = 2 K elements), B from
+// shared memory. Executed by a whole (converged) warp, one elected lane issues. One block with one election: the issuing
+// warp's instruction stream is what bounds tiles of few token rows (see the MMA issuer), and an election, two predicates
+// and a descriptor assembled per instruction made it ~290 cycles per 64 K elements.
+__device__ __forceinline__ void umma_f16_ts_64(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, t, e;\n.reg .b32 a1, a2, a3, l1, l2, l3;\n.reg .b64 d0, d1, d2, d3;\n"
+      "setp.ne.b32 p, %5, 0;\nsetp.eq.b32 t, %5, %5;\n"
+      "add.u32 a1, %1, 8;\nadd.u32 a2, %1, 16;\nadd.u32 a3, %1, 24;\n"
+      "add.u32 l1, %2, 2;\nadd.u32 l2, %2, 4;\nadd.u32 l3, %2, 6;\n"
+      "mov.b64 d0, {%2, %3};\nmov.b64 d1, {l1, %3};\nmov.b64 d2, {l2, %3};\nmov.b64 d3, {l3, %3};\n"
+      "elect.sync _|e, 0xffffffff;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d0, %4, p;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], d1, %4, t;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], d2, %4, t;\n"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], d3, %4, t;\n}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit_elect(uint32_t bar) {
   asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n"
@@ -305,6 +326,11 @@ __device__ __forceinline__ __half2 trit_pair(uint32_t w) {
   constexpr float a = F == 0 ? -1025.f : F == 1 ? -257.f : F == 2 ? -65.f : F == 3 ? -17.f : -5.f;
   return __hfma2(bits_h2((w & (0x00030003u << (2 * F))) | 0x64006400u), __floats2half2_rn(m, m), __floats2half2_rn(a, a));
 }
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
 template <bool FIRST>
 __device__ __forceinline__ void put(__half2& acc, __half2 t, __half2 s2) {
   acc = FIRST ? __hmul2(t, s2) : __hfma2(t, s2, acc);  // the group scale is applied exactly (trit in {-1, 0, 1})
@@ -324,49 +350,121 @@ __device__ __forceinline__ void tq2_word(uint32_t w, __half2 s2, __half2* acc /*
   put<FIRST>(acc[7], trit_pair<2>(w2), s2);
 }
 
-// TQ1, tiled grouping (layout_kernels.cu): the 64 trits of stage s of a row-superblock are the 12 bytes
-// 12 s .. 12 s + 11 (5 trits each) plus digit s of the 4 bytes 60..63. A shared-memory table maps a byte to its
-// five digits as 2-bit fields placed for BOTH positions a byte can have in a pair of bytes (10 trits = 5 fp16
-// pairs): as the first byte its digits 0,2,4 are the even trits of pairs 0,1,2 and digits 1,3 the odd trits of
-// pairs 0,1; as the second byte digit 0 is the odd trit of pair 2, digits 1,3 the even and digits 2,4 the odd
-// trits of pairs 3,4. The two placements use disjoint bits, so one AND-OR merges two table entries into a
-// word of the TQ2 pair format above.
-constexpr uint32_t TQ1_FIRST_MASK = 0x000F003Fu, TQ1_SECOND_MASK = 0x03F003C0u;
-__host__ __device__ inline uint32_t tq1_table_entry(uint32_t byte) {
+// TQ1, tiled grouping (layout_kernels.cu): the 64 trits of piece s of a row-superblock are the 12 bytes 12 s .. 12 s + 11
+// (5 trits each) plus digit s of the 4 bytes 60..63. No arithmetic: an fp16 pair of scale * trit is ONE byte permutation of
+// the four bytes {scale low, scale high, scale high with the sign flipped, 0}, and its selector (two bytes, one per trit: low
+// nibble = source of the low byte, high nibble = source of the high byte) comes from a table in shared memory, 64 bits per
+// byte value. A pair of bytes holds ten trits = five pairs, the third of them split between the two bytes.
+//   64 KB table   an entry for either position in the pair, [byte value][position][16 replicas]: 256 bytes per byte value, so
+//                 ONE byte permutation forms the address (the table sits at a multiple of 64 KB)
+//                   first byte    x = trits 0, 1 | trit 4 in bits 16..23      y = trits 2, 3
+//                   second byte   x = trits 6, 7 | trit 5 in bits 24..31      y = trits 8, 9
+//   32 KB table   one entry for both, [byte value][16 replicas]: a shift and an AND-OR per address, two shifts per byte pair
+//                   x = trits 0, 1, 2, 3      y = trits 3, 4, 1, 2
+// (a permutation reads the low 16 bits of its selector). 16 replicas: the 64-bit reads of a half warp hit all banks once.
+// A table of 2-bit digit fields expanded by fused multiply-adds (16 KB) took ~200 instructions per warp and 64 trits, this
+// takes ~110: 96 experts of 4096 x 4096, 64 rows 457 -> 381 us in the form of the kernel of that time.
+__host__ __device__ inline uint32_t tq1_select_byte(uint32_t digit) { return digit == 2u ? 0x10u : digit == 0u ? 0x20u : 0x33u; }
+template <int TABLE>
+__host__ __device__ inline void tq1_select_entry(uint32_t byte, int second, uint32_t& x, uint32_t& y) {
   const uint32_t f = tq1_fields(byte);
-  const uint32_t d0 = f & 3u, d1 = (f >> 2) & 3u, d2 = (f >> 4) & 3u, d3 = (f >> 6) & 3u, d4 = (f >> 8) & 3u;
-  const uint32_t first = d0 | (d2 << 2) | (d4 << 4) | (d1 << 16) | (d3 << 18);
-  const uint32_t second = (d0 << 20) | (d1 << 6) | (d2 << 22) | (d3 << 8) | (d4 << 24);
-  return first | second;
+  uint32_t t[5];
+#pragma unroll
+  for (int d = 0; d < 5; ++d) t[d] = tq1_select_byte((f >> (2 * d)) & 3u);
+  if (TABLE == PF_TABLE_64K) {
+    x = second ? t[1] | (t[2] << 8) | (t[0] << 24) : t[0] | (t[1] << 8) | (t[4] << 16);
+    y = second ? t[3] | (t[4] << 8) : t[2] | (t[3] << 8);
+  } else {
+    x = t[0] | (t[1] << 8) | (t[2] << 16) | (t[3] << 24);
+    y = t[3] | (t[4] << 8) | (t[1] << 16) | (t[2] << 24);
+  }
 }
-__device__ __forceinline__ uint32_t tq1_lookup(uint32_t lut_addr, uint32_t word, int byte) {
-  const uint32_t idx = byte == 0 ? (word << 6) & 0x3FC0u : (word >> (8 * byte - 6)) & 0x3FC0u;  // byte value * 64
-  uint32_t v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(lut_addr + idx));
+// where digit d of a byte is in its (first) entry
+template <int TABLE>
+__device__ __forceinline__ uint32_t tq1_select_place(int d) { return ((TABLE == PF_TABLE_64K ? 0x25410u : 0x53210u) >> (4 * d)) & 7u; }
+// entry address of byte B of `word` for a lane whose replica of the first entry is at `base`
+template <int TABLE, int B>
+__device__ __forceinline__ uint32_t tq1_select_addr(uint32_t word, uint32_t base) {
+  if (TABLE == PF_TABLE_64K) return __byte_perm(word, base, 0x7604 | (B << 4));  // the byte becomes bits 8..15 of base
+  return ((B == 0 ? word << 7 : word >> (8 * B - 7)) & 0x7F80u) | base;          // ... bits 7..14
+}
+template <int SECOND>
+__device__ __forceinline__ uint2 tq1_select_load(uint32_t addr) {
+  uint2 v;
+  if (SECOND) asm("ld.shared.v2.u32 {%0,%1}, [%2+128];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  else asm("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
 }
-// w[0..2]: the stage's 12 own bytes, w[3]: bytes 60..63 of the row-superblock; sbk: stage inside the superblock
-template <bool FIRST>
-__device__ __forceinline__ void tq1_stage(const uint32_t* w, int sbk, uint32_t lut_addr, __half2 s2, __half2* acc /* 32 */) {
+template <int TABLE, int B>
+__device__ __forceinline__ uint32_t tq1_select_digit(uint32_t word, uint32_t base) {
+  uint32_t v;
+  asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(tq1_select_addr<TABLE, B>(word, base)));
+  return v;
+}
+// prmt itself: __byte_perm masks every selector to three bits per nibble first, an instruction more for run-time selectors
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+__device__ __forceinline__ void put_select(bool first, uint32_t& acc, uint32_t pool, uint32_t sel) {
+  const uint32_t v = prmt(pool, pool, sel);
+  acc = first ? v : h2_bits(__hadd2(bits_h2(acc), bits_h2(v)));
+}
+// The four source bytes of a scale (fp16 bits). A scale that is not finite makes NaN of its zero trits, as a product does.
+__device__ __forceinline__ uint32_t tq1_select_pool(uint32_t h) {
+  const uint32_t hi = h >> 8;
+  return h | ((hi ^ 0x80u) << 16) | ((h & 0x7c00u) == 0x7c00u ? 0x7f000000u : 0u);
+}
+// One 64-trit piece of a row, all stacked terms, into 32 TMEM columns from `taddr` on, eight as soon as they are complete.
+// w[i][0..2]: term i's 12 own bytes, w[i][3]: bytes 60..63 of the row-superblock; base: the lane's replica of the table;
+// base_d: the same plus the place of the piece's digit inside an entry. n_terms <= TERMS.
+template <int TABLE, int TERMS>
+__device__ __forceinline__ void tq1_stage_select(const uint32_t (&w)[TERMS][4], int n_terms, uint32_t base, uint32_t base_d,
+                                                 const uint32_t (&pool)[TERMS], uint32_t taddr) {
+  uint32_t v[32];
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
-    const uint32_t c0 = tq1_lookup(lut_addr, w[(2 * q) >> 2], (2 * q) & 3);
-    const uint32_t c1 = tq1_lookup(lut_addr, w[(2 * q + 1) >> 2], (2 * q + 1) & 3);
-    const uint32_t m = (c0 & TQ1_FIRST_MASK) | (c1 & TQ1_SECOND_MASK);
-    put<FIRST>(acc[5 * q + 0], trit_pair<0>(m), s2);
-    put<FIRST>(acc[5 * q + 1], trit_pair<1>(m), s2);
-    put<FIRST>(acc[5 * q + 2], trit_pair<2>(m), s2);
-    put<FIRST>(acc[5 * q + 3], trit_pair<3>(m), s2);
-    put<FIRST>(acc[5 * q + 4], trit_pair<4>(m), s2);
+#pragma unroll
+    for (int i = 0; i < TERMS; ++i) {
+      if (i < n_terms) {
+        const uint32_t word = w[i][q >> 1];
+        const uint2 a = tq1_select_load<0>((q & 1) ? tq1_select_addr<TABLE, 2>(word, base) : tq1_select_addr<TABLE, 0>(word, base));
+        const uint2 b = tq1_select_load<TABLE == PF_TABLE_64K>((q & 1) ? tq1_select_addr<TABLE, 3>(word, base) : tq1_select_addr<TABLE, 1>(word, base));
+        if (TABLE == PF_TABLE_64K) {
+          put_select(i == 0, v[5 * q + 0], pool[i], a.x);
+          put_select(i == 0, v[5 * q + 1], pool[i], a.y);
+          put_select(i == 0, v[5 * q + 2], pool[i], __byte_perm(a.x, b.x, 0x0072));
+          put_select(i == 0, v[5 * q + 3], pool[i], b.x);
+          put_select(i == 0, v[5 * q + 4], pool[i], b.y);
+        } else {
+          put_select(i == 0, v[5 * q + 0], pool[i], a.x);
+          put_select(i == 0, v[5 * q + 1], pool[i], a.x >> 16);
+          put_select(i == 0, v[5 * q + 2], pool[i], __byte_perm(a.y, b.x, 0x0041));
+          put_select(i == 0, v[5 * q + 3], pool[i], b.y >> 16);
+          put_select(i == 0, v[5 * q + 4], pool[i], b.y);
+        }
+      }
+    }
+    if (q == 1) tmem_st_8(taddr, v);
+    if (q == 3) tmem_st_8(taddr + 8, v + 8);
+    if (q == 4) tmem_st_8(taddr + 16, v + 16);
   }
-  // trits 60..63: digit sbk of bytes 60..63; as a "first byte" entry digit d sits at bit (d >> 1) * 2 + (d & 1) * 16
-  const int sh = (sbk >> 1) * 2 + (sbk & 1) * 16;
-  const uint32_t e0 = (tq1_lookup(lut_addr, w[3], 0) >> sh) & 3u, e1 = (tq1_lookup(lut_addr, w[3], 1) >> sh) & 3u;
-  const uint32_t e2 = (tq1_lookup(lut_addr, w[3], 2) >> sh) & 3u, e3 = (tq1_lookup(lut_addr, w[3], 3) >> sh) & 3u;
-  put<FIRST>(acc[30], trit_pair<0>(e0 | (e1 << 16)), s2);
-  put<FIRST>(acc[31], trit_pair<0>(e2 | (e3 << 16)), s2);
+#pragma unroll
+  for (int i = 0; i < TERMS; ++i) {  // trits 60..63
+    if (i < n_terms) {
+      put_select(i == 0, v[30], pool[i], tq1_select_digit<TABLE, 0>(w[i][3], base_d) | (tq1_select_digit<TABLE, 1>(w[i][3], base_d) << 8));
+      put_select(i == 0, v[31], pool[i], tq1_select_digit<TABLE, 2>(w[i][3], base_d) | (tq1_select_digit<TABLE, 3>(w[i][3], base_d) << 8));
+    }
+  }
+  tmem_st_8(taddr + 24, v + 24);
 }
 
+// Scale of group g (0..7 inside the 8 scales held in `sc`), as fp16 bits.
+__device__ __forceinline__ uint32_t pick_scale_bits(const uint4& sc, int g) {
+  const uint32_t w = (g & 4) ? ((g & 2) ? sc.w : sc.z) : ((g & 2) ? sc.y : sc.x);
+  return (g & 1) ? (w >> 16) : (w & 0xFFFFu);
+}
 // Scale of group g (0..7 inside the 8 scales held in `sc`), as an fp16 pair.
 __device__ __forceinline__ __half2 pick_scale(const uint4& sc, int g) {
   const uint32_t w = (g & 4) ? ((g & 2) ? sc.w : sc.z) : ((g & 2) ? sc.y : sc.x);
@@ -381,7 +479,7 @@ __device__ __forceinline__ bool drain_tile(const PrefillParams& p, uint32_t tmem
                                         uint32_t d_tile, const uint64_t* __restrict__ row_ptr) {
   const int lane = r & 31;
   const uint32_t lane_base = (uint32_t)(r & ~31) << 16;
-  if (!mbar_wait(tfull_bar, d_tile & 1u, abort_flag)) return false;
+  if (!mbar_wait<true>(tfull_bar, d_tile & 1u, abort_flag)) return false;
   // Lanes leave the polling loop (and its per-thread sleeps) one by one; the .sync.aligned tcgen05 instructions
   // below must be executed by the whole warp together.
   __syncwarp();
@@ -464,7 +562,7 @@ __device__ __forceinline__ bool drain_tile(const PrefillParams& p, uint32_t tmem
 __device__ __forceinline__ bool drain_tile_wide(const PrefillParams& p, uint32_t tmem, int col_first, int col_step, int warp_q, int lane,
                                                 uint32_t tfull_bar, uint32_t tempty_bar, volatile int* abort_flag, int d_nt, int d_row0,
                                                 int d_rows, uint32_t d_tile, const uint64_t* __restrict__ row_ptr, uint8_t* tile_smem) {
-  if (!mbar_wait(tfull_bar, d_tile & 1u, abort_flag)) return false;
+  if (!mbar_wait<true>(tfull_bar, d_tile & 1u, abort_flag)) return false;
   __syncwarp();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const int n_eff = tile_neff(d_rows);
@@ -533,51 +631,72 @@ __device__ __forceinline__ bool drain_tile_wide(const PrefillParams& p, uint32_t
 }
 
 // ------------------------------------------------------------------------------------------ the kernel
-// Shared memory map (dynamic, 1024-byte aligned), per CTA:
-//   [0, nb * tn_max * 128)          B stage ring: tn_max token rows x 64 fp16 per stage; stage s pairs with A slot s in TMEM
-//   then nslab * n_terms * 8 KB     packed-weight slabs: slot-major, one 8 KB slab per stacked term
-//   then 16 KB (TQ1 only)           table of digit fields, see tq1_table_entry
-//   then 2 x 4 KB                   offs[E + 1], tpre[E + 1] (see tile_seek)
-template <int FMT, int TERMS>
+// Shared memory of a CTA (plan_smem places the parts):
+//   B stage ring       nb stages of tn_max token rows x 64 (SMALL: 2 x 64) fp16, 1024-byte aligned
+//   packed slabs       nslab x n_terms x 8 KB, slot-major
+//   selector table     TQ1
+//   front              offs[E + 1] and tpre[E + 1] (see tile_seek), the scatter form's row pointers, the epilogue warps' tiles
+// SMALL: token tiles of at most PF_SMALL_TN rows: 128-K stages, four epilogue warps, five dequant groups.
+template <int FMT, int TERMS, bool SMALL>
 __global__ void __launch_bounds__(PF_THREADS, 1)
 prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
-  constexpr int SPB = FMT == 2 ? 4 : 5;  // 64-trit stages per 64-byte row-superblock
+  constexpr int SPB = FMT == 2 ? 4 : 5;  // 64-trit pieces per 64-byte row-superblock
+  constexpr int TABLE = pf_table(FMT, TERMS, SMALL);
+  constexpr int KH = SMALL ? 2 : 1;      // 64-K pieces per stage
+  constexpr int EPI = SMALL ? 4 : PF_EPI_WARPS;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const uint32_t NB = (uint32_t)p.nb;
-  const uint32_t stage_bytes = (uint32_t)p.tn_max * 128u;
-  uint8_t* slabs = smem + NB * stage_bytes;
-  uint8_t* lut = slabs + (size_t)p.nslab * p.n_terms * PF_SLAB;  // TQ1 only
-  int* offs = reinterpret_cast<int*>(lut + (FMT == 1 ? PF_LUT_BYTES : 0));
+  const uint32_t NB = (uint32_t)p.nb, NA = (uint32_t)p.na;
+  const uint32_t half_bytes = (uint32_t)p.tn_max * 128u, stage_bytes = half_bytes * KH;
+  const uint32_t first = smem_u32(smem_raw);
+  if (first < PF_SMEM_FIRST || first > PF_SMEM_START) {  // the plan does not fit this start of the dynamic part
+    if (threadIdx.x == 0) atomicExch(&g_device_status, DST_ERR_UNSUPPORTED);
+    return;
+  }
+  uint8_t* stages = smem_raw + (p.a_ring - first);
+  uint8_t* slabs = smem_raw + (p.a_slabs - first);
+  int* offs = reinterpret_cast<int*>(smem_raw + (p.a_front - first));
   int* tpre = offs + (PF_MAX_E + 1);
-  uint8_t* epi_tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tpre + (PF_MAX_E + 1)) + 127) & ~static_cast<uintptr_t>(127));  // PF_EPI_WARPS x 2 KB
-  __shared__ uint64_t bar_full[PF_MAX_STAGES], bar_empty[PF_MAX_STAGES], bar_tfull[1], bar_tempty[1], bar_pfull[PF_MAX_SLABS],
-      bar_pempty[PF_MAX_SLABS];
+  // scatter form: destination of every token row of a tile, two tiles alternating (absent otherwise)
+  constexpr int ROWS = SMALL ? PF_SMALL_TN : PF_TN_MAX;
+  uint64_t* rowptr_s = reinterpret_cast<uint64_t*>(tpre + (PF_MAX_E + 1));
+  uint8_t* epi_tiles = reinterpret_cast<uint8_t*>(rowptr_s + (p.row_target != nullptr ? 2 * ROWS : 0));  // EPI x 2 KB
+  __shared__ uint64_t bar_full[PF_BARS], bar_empty[PF_BARS], bar_tfull[1], bar_tempty[1], bar_pfull[PF_BARS], bar_pempty[PF_BARS];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
   __shared__ uint64_t bar_epi;                      // scatter form: the epilogue warps' own barrier, once per tile
-  __shared__ uint64_t rowptr_s[2][PF_TN_MAX];       // scatter form: destination of every token row of a tile, two tiles alternating
   volatile int* abort_flag = &abort_s;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the warp index as a broadcast: the compiler then knows it to be the same in all lanes and keeps what follows from it (the
+  // MMA issuer's loop counters and addresses) in uniform registers
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
-    for (int s = 0; s < PF_MAX_STAGES; ++s) {
+    for (int s = 0; s < (int)PF_BARS; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1 + 4);  // the TMA producer's expect_tx arrive + one arrive per warp of the dequant group that owns the stage
-      mbar_init(smem_u32(&bar_empty[s]), 2);     // one tcgen05.commit per MMA issuer: the MMAs that read the stage are done
+      mbar_init(smem_u32(&bar_empty[s]), 1);     // tcgen05.commit: the MMAs that read the stage are done
     }
-    mbar_init(smem_u32(&bar_tfull[0]), 2);             // one tcgen05.commit per MMA issuer after the tile's last MMA
-    mbar_init(smem_u32(&bar_tempty[0]), p.small ? 4 : PF_EPI_WARPS);  // every epilogue warp has drained its share of the accumulator
-    mbar_init(smem_u32(&bar_epi), p.small ? 4 : PF_EPI_WARPS);
-    for (int a = 0; a < PF_MAX_SLABS; ++a) {
+    for (int a = 0; a < (int)PF_BARS; ++a) {
       mbar_init(smem_u32(&bar_pfull[a]), 1);         // bulk-copy producer's expect_tx arrive
-      mbar_init(smem_u32(&bar_pempty[a]), 4 * SPB);  // one arrive per (stage of the superblock, warp of its group)
+      mbar_init(smem_u32(&bar_pempty[a]), 4 * SPB);  // one arrive per (piece of the superblock, warp of its group)
     }
+    mbar_init(smem_u32(&bar_tfull[0]), 1);             // tcgen05.commit after the tile's last MMA
+    mbar_init(smem_u32(&bar_tempty[0]), EPI);  // every epilogue warp has drained its share of the accumulator
+    mbar_init(smem_u32(&bar_epi), EPI);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (FMT == 1) {
-    uint32_t* lut32 = reinterpret_cast<uint32_t*>(lut);  // [byte value][replica]
-    for (int i = tid; i < 256 * 16; i += PF_THREADS) lut32[i] = tq1_table_entry((uint32_t)i >> 4);
+  if (TABLE != PF_TABLE_NONE) {
+    // every entry is computed once (into the B ring, not in use yet), then copied to its 16 replicas
+    constexpr int ENTRIES = TABLE == PF_TABLE_64K ? 512 : 256;
+    uint2* once = reinterpret_cast<uint2*>(stages);
+    for (int i = tid; i < ENTRIES; i += PF_THREADS) {
+      uint2 v;
+      tq1_select_entry<TABLE>(TABLE == PF_TABLE_64K ? (uint32_t)i >> 1 : (uint32_t)i, i & 1, v.x, v.y);
+      once[i] = v;
+    }
+    __syncthreads();
+    uint2* table = reinterpret_cast<uint2*>(smem_raw + (p.a_table - first));
+    for (int i = tid; i < ENTRIES * 16; i += PF_THREADS) table[i] = once[i >> 4];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the ring is written by bulk copies from here on
   }
   for (int i = tid; i <= p.E; i += PF_THREADS) {
     // offsets that were not validated on the host are clamped so no row index leaves [0, T)
@@ -617,22 +736,29 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer for B (activations)
     if (lane == 0) {
-      uint32_t s = 0, ph = 0;
+      uint32_t gst = 0, b = 0;  // stage, counted over all tiles of this CTA, and its place in the B ring
       bool ok = true;
       RT_DECL(w_empty = 0, n_it = 0, t_begin = RT_NOW());
-      const uint32_t full0 = smem_u32(&bar_full[0]), empty0 = smem_u32(&bar_empty[0]), dst0 = smem_u32(smem);
+      const uint32_t full0 = smem_u32(&bar_full[0]), empty0 = smem_u32(&bar_empty[0]), dst0 = smem_u32(stages);
       for (int t = (int)blockIdx.x; ok && t < n_tiles; t += t_step) {
         tile_seek(p, offs, tpre, t, e, nt, row0, rows);
         const int n_eff = tile_neff(rows);
         const int h = n_eff > 256 ? n_eff >> 1 : n_eff;  // token rows per TMA box and per MMA (a multiple of 16)
         const CUtensorMap* map = &xmaps.m[h / 16 - 1];
-        const uint32_t bytes = (uint32_t)n_eff * 128u;
-        for (int ks = 0; ks < p.kstages; ++ks) {
-          if (!RT_WAIT(w_empty, mbar_wait(empty0 + s * 8, ph ^ 1u, abort_flag))) { ok = false; break; }
-          mbar_arrive_expect_tx(full0 + s * 8, bytes);
-          tma_load_2d(dst0 + s * stage_bytes, map, ks * 64, row0, full0 + s * 8);
-          if (h != n_eff) tma_load_2d(dst0 + s * stage_bytes + (uint32_t)h * 128u, map, ks * 64, row0 + h, full0 + s * 8);
-          if (++s == NB) { s = 0; ph ^= 1u; }
+        const uint32_t bytes = (uint32_t)n_eff * 128u * KH;
+        for (int ks = 0; ks < p.kstages; ks += KH) {
+          const uint32_t prev = gst - NB;  // the stage whose place this is
+          if (gst >= NB && !RT_WAIT(w_empty, mbar_wait(empty0 + prev % PF_BARS * 8, prev / PF_BARS & 1u, abort_flag))) { ok = false; break; }
+          const uint32_t full = full0 + gst % PF_BARS * 8;
+          mbar_arrive_expect_tx(full, bytes);
+#pragma unroll
+          for (int x = 0; x < KH; ++x) {
+            const uint32_t dst = dst0 + b * stage_bytes + x * half_bytes;
+            tma_load_2d(dst, map, (ks + x) * 64, row0, full);
+            if (h != n_eff) tma_load_2d(dst + (uint32_t)h * 128u, map, (ks + x) * 64, row0 + h, full);
+          }
+          ++gst;
+          if (++b == NB) b = 0;
 #ifdef DST_ROLE_TIMERS
           ++n_it;
 #endif
@@ -643,36 +769,38 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
   } else if (warp == 2) {
     // ------------------------------------------------------------------ bulk-copy producer for the packed slabs
     if (lane == 0) {
-      uint32_t slot = 0, ph = 0;
+      uint32_t gsl = 0, slot = 0;  // slab, counted over all tiles of this CTA, and its place
       bool ok = true;
       RT_DECL(w_pempty = 0, t_begin = RT_NOW());
       for (int t = (int)blockIdx.x; ok && t < n_tiles; t += t_step) {
         tile_seek(p, offs, tpre, t, e, nt, row0, rows);
         const int64_t off0 = ((int64_t)e * p.NT + nt) * p.S * PF_SLAB;
         for (int sb = 0; sb < nsb; ++sb) {
-          if (!RT_WAIT(w_pempty, mbar_wait<true>(smem_u32(&bar_pempty[slot]), ph ^ 1u, abort_flag))) { ok = false; break; }
-          const uint32_t full = smem_u32(&bar_pfull[slot]);
+          const uint32_t prev = gsl - (uint32_t)p.nslab;  // the slab whose place this is
+          if (gsl >= (uint32_t)p.nslab &&
+              !RT_WAIT(w_pempty, mbar_wait<true>(smem_u32(&bar_pempty[prev % PF_BARS]), prev / PF_BARS & 1u, abort_flag))) { ok = false; break; }
+          const uint32_t full = smem_u32(&bar_pfull[gsl % PF_BARS]);
           mbar_arrive_expect_tx(full, (uint32_t)p.n_terms * PF_SLAB);
           for (int i = 0; i < p.n_terms; ++i)
             bulk_load(smem_u32(slabs + ((size_t)slot * p.n_terms + i) * PF_SLAB), p.tiled[i] + off0 + (int64_t)sb * PF_SLAB, PF_SLAB, full);
-          if (++slot == (uint32_t)p.nslab) { slot = 0; ph ^= 1u; }
+          ++gsl;
+          if (++slot == (uint32_t)p.nslab) slot = 0;
         }
       }
       RT_ADD(5, RT_NOW() - t_begin); RT_ADD(1, w_pempty);
     }
-  } else if (warp == 1 || warp == 3) {
-    // ------------------------------------------------------------------ MMA issuers
-    // Two threads (in two warps, on two scheduler partitions) issue the MMAs of a stage: each owns half of the token
-    // rows (its own accumulator columns and its own half of the B stage), so a stage costs each of them four
-    // instructions instead of eight; a single thread could not issue them as fast as the tensor pipe runs them.
-    // Tiles whose row count (padded to 16) is not a multiple of 32, or below 64, are issued by the first thread
-    // alone; the second then only adds its arrivals to the barriers.
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    // One warp, all of whose lanes run the loop (the elected lane issues). Next to the dequant warps its own instructions per
+    // stage - a barrier wait, a vote, a commit and the MMAs - cost several hundred cycles whatever the number of token rows:
+    // with a 64-K stage and every MMA elected by itself, 16 rows and 64 rows both took ~780 cycles per 64 K elements
+    // (MMAs of 64 rows: 128; alone on the SM the same instructions take 166) and the dequant warps spent half of their
+    // time waiting for a free A slot. Hence the 128-K stages of the small tiles and the one block per 64 K.
     {
-      // all 32 lanes run this loop (see umma_f16_ts_elect); the elected lane issues the MMAs and the commits
-      const uint32_t who = warp == 1 ? 0u : 1u;
-      uint32_t s = 0, ph = 0, tile = 0;
+      uint32_t gst = 0, s = 0, b = 0, tile = 0;  // stage, counted over all tiles of this CTA; its A slot and its place in the B ring
       bool ok = true;
-      const uint64_t b_desc0 = umma_desc(smem_u32(smem));
+      const uint64_t b_desc0 = umma_desc(smem_u32(stages));
+      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
       const uint32_t b_desc_lo = (uint32_t)b_desc0, b_desc_hi = (uint32_t)(b_desc0 >> 32);
       RT_DECL(w_tempty = 0, w_full = 0, n_it = 0, t_begin = RT_NOW());
       for (int t = (int)blockIdx.x; ok && t < n_tiles; t += t_step) {
@@ -680,31 +808,24 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
         // one accumulator: the previous tile must have been drained
         if (!__all_sync(0xffffffffu, RT_WAIT(w_tempty, mbar_wait(smem_u32(&bar_tempty[0]), (tile & 1u) ^ 1u, abort_flag)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t n_eff = (uint32_t)tile_neff(rows);
-        const bool split = n_eff >= (uint32_t)PF_SPLIT_MIN && (n_eff & 31u) == 0u;  // tiles above 256 rows are padded to 32: always split
-        const uint32_t h = split ? n_eff >> 1 : n_eff;           // token rows per MMA (a multiple of 16, at most 256)
-        const bool active = split || who == 0u;
+        const uint32_t n_eff = __shfl_sync(0xffffffffu, (uint32_t)tile_neff(rows), 0);  // (uniform, as above)
+        const bool two = n_eff > 256u;
+        const uint32_t h = two ? n_eff >> 1 : n_eff;             // token rows per MMA (a multiple of 16, at most 256)
         // instruction descriptor: D f32, A f16, B f16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
         const uint32_t idesc = (1u << 4) | ((h >> 3) << 17) | ((128u >> 4) << 24);
-        const uint32_t mine = split ? who * h : 0u;              // first token row (= accumulator column) of this warp's MMAs
-        const uint32_t d_tmem = tmem + mine;
-        const uint32_t b_off = (mine * 128u) >> 4;               // descriptor start-address units
-        for (int ks = 0; ks < p.kstages; ++ks) {
-          if (!__all_sync(0xffffffffu, RT_WAIT(w_full, mbar_wait(smem_u32(&bar_full[s]), ph, abort_flag)))) { ok = false; break; }
+        for (int ks = 0; ks < p.kstages; ks += KH) {
+          if (!__all_sync(0xffffffffu, RT_WAIT(w_full, mbar_wait(smem_u32(&bar_full[gst % PF_BARS]), gst / PF_BARS & 1u, abort_flag)))) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (active) {
-            const uint32_t a_tmem = tmem + (uint32_t)p.tn_max + s * PF_A_COLS;  // this stage's slot of the A ring
-            // only the start-address field of the B descriptor changes with the stage, the K step and the half
-            const uint32_t b_lo = b_desc_lo + s * (stage_bytes >> 4) + b_off;
+          const uint32_t a_tmem = tmem_u + (uint32_t)p.tn_max + s * (PF_A_COLS * KH);  // this stage's slot of the A ring
+          const uint32_t b_lo = b_desc_lo + b * (stage_bytes >> 4);                  // start address of the B descriptor
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              uint64_t db;
-              asm volatile("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + kk * 2), "r"(b_desc_hi));
-              umma_f16_ts_elect(d_tmem, a_tmem + kk * 8, db, idesc, (ks > 0 || kk > 0) ? 1u : 0u);
-            }
-          }
-          umma_commit_elect(smem_u32(&bar_empty[s]));  // this warp's MMAs (if any) have read the stage
-          if (++s == NB) { s = 0; ph ^= 1u; }
+          for (int x = 0; x < KH; ++x)
+            umma_f16_ts_64(tmem_u, a_tmem + x * PF_A_COLS, b_lo + x * (half_bytes >> 4), b_desc_hi, idesc, (ks > 0 || x > 0) ? 1u : 0u);
+          if (!SMALL && two) umma_f16_ts_64(tmem_u + h, a_tmem, b_lo + ((h * 128u) >> 4), b_desc_hi, idesc, ks > 0 ? 1u : 0u);
+          umma_commit_elect(smem_u32(&bar_empty[gst % PF_BARS]));  // the MMAs have read the stage
+          ++gst;
+          if (++s == NA) s = 0;
+          if (++b == NB) b = 0;
 #ifdef DST_ROLE_TIMERS
           ++n_it;
 #endif
@@ -712,15 +833,17 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
         if (ok) umma_commit_elect(smem_u32(&bar_tfull[0]));
         ++tile;
       }
-      if (who == 0u && lane == 0) {
+      if (lane == 0) {
         RT_ADD(8, RT_NOW() - t_begin); RT_ADD(9, w_tempty); RT_ADD(10, w_full); RT_ADD(11, n_it); RT_ADD(12, 1); RT_ADD(13, tile);
       }
     }
-  } else if (warp < PF_CTRL_WARPS + (p.small ? 4 : PF_EPI_WARPS)) {
+  } else if (warp == 3) {
+    // no role
+  } else if (warp < PF_CTRL_WARPS + EPI) {
     // ------------------------------------------------------------------ epilogue: TMEM -> registers -> global
     const int r = (warp & 3) * 32 + lane;  // a warp may only read the TMEM lanes of its own quarter (warp id % 4)
     uint32_t tile = 0;
-    const int epi_threads = 32 * (p.small ? 4 : PF_EPI_WARPS), epi_tid = tid - 32 * PF_CTRL_WARPS;
+    const int epi_threads = 32 * EPI, epi_tid = tid - 32 * PF_CTRL_WARPS;
     for (int t = (int)blockIdx.x; t < n_tiles; t += t_step, ++tile) {
       tile_seek(p, offs, tpre, t, e, nt, row0, rows);
       const uint64_t* row_ptr = nullptr;
@@ -728,7 +851,7 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
         // scatter form: while the tile is computed, look up where its token rows go (a global load and a pointer
         // per row, shared by the role's warps through shared memory; the buffer of the tile before stays intact for
         // warps still draining it, and nobody passes the barrier before all are done with the tile before that)
-        uint64_t* rp = rowptr_s[tile & 1u];
+        uint64_t* rp = rowptr_s + (tile & 1u) * ROWS;
         const size_t ostep = (size_t)p.N * 2;
         for (int j = epi_tid; j < rows; j += epi_threads) {
           const int64_t tg = p.row_target[row0 + j];
@@ -743,7 +866,7 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
         row_ptr = rp;
       }
       // the two warps of a lane quarter take alternate 32-column chunks
-      const int col_first = ((warp - PF_CTRL_WARPS) >> 2) * 32, col_step = p.small ? 32 : 32 * (PF_EPI_WARPS / 4);
+      const int col_first = ((warp - PF_CTRL_WARPS) >> 2) * 32, col_step = 32 * (EPI / 4);
       if (p.wide_drain) {
         if (!drain_tile_wide(p, tmem, col_first, col_step, warp & 3, lane, smem_u32(&bar_tfull[0]), smem_u32(&bar_tempty[0]), abort_flag, nt,
                              row0, rows, tile, row_ptr, epi_tiles + (warp - PF_CTRL_WARPS) * PF_EPI_TILE))
@@ -759,23 +882,30 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
     const int q = warp & 3;
     const int r = q * 32 + lane;
     // groups 0..3: warps 12..27; with small token tiles warps 8..11 (epilogue warps otherwise) are group 4
-    const uint32_t n_groups = p.small ? PF_GROUPS + 1 : PF_GROUPS;
+    constexpr uint32_t n_groups = SMALL ? PF_GROUPS + 1 : PF_GROUPS;
     const uint32_t grp = warp >= PF_DQ_WARP0 ? (uint32_t)(warp - PF_DQ_WARP0) >> 2 : (uint32_t)PF_GROUPS;
-    const int swz = (r >> 1) & 3;  // swizzle of the tiled layout: logical word w sits at physical word (((w & 3) ^ swz) << 2) | (w >> 2)
-    const uint32_t lut_addr = smem_u32(lut) + (uint32_t)(lane & 15) * 4u;
+    // logical word w of a row-superblock sits at physical word (((w & 3) ^ swizzle) << 2) | (w >> 2) of its 64 bytes
+    const uint32_t slabs_a = smem_u32(slabs);
+    uint32_t unit_off[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) unit_off[j] = (uint32_t)(r * 64 + ((j ^ ((r >> 1) & 3)) << 4));
+    const uint32_t table_a = p.a_table + (uint32_t)(lane & 15) * 8u;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     const bool vec_scales = (p.G & 7) == 0;  // rows of 8 k scales are 16-byte aligned
     const int kstages = p.kstages;
-    uint32_t own = grp;  // global index (counted over all tiles of this CTA) of this group's next stage
-    uint32_t s = grp % NB, ph = (grp / NB) & 1u;
-    uint32_t it0 = 0, gs0 = 0;  // first stage / first slab of the current tile
+    // A group takes 128 trits (two pieces: one scale group) at a time: unit `own`, counted over all tiles of this CTA. The
+    // bookkeeping around a piece (barriers, slab slots, scale, loop) costs as much as its arithmetic and is paid once for two.
+    const int units = kstages >> 1;
+    uint32_t own = grp;
+    uint32_t gst = grp * (2 / KH), s = gst % NA;  // the unit's (first) stage and its A slot
+    uint32_t it0 = 0, gs0 = 0;                     // first unit / first slab of the current tile
     bool ok = true;
     RT_DECL(w_pfull = 0, w_dempty = 0, w_drain = 0, w_comp = 0, w_st = 0, w_pre = 0, n_it = 0, t_begin = RT_NOW(), w_lds = 0, w_tail = 0, t_tail = RT_NOW());
 
-    // scales of the row: 8 groups (16 stages) per 128-bit load; when a block of 8 is taken into use the tile's next block
-    // is requested, so only a tile's first block is waited for (once per tile and warp; the per-stage cost is a compare)
-    uint4 sc[TERMS], scn[TERMS];
-    int cur_b = -1, nxt_b = -1;              // block of 8 groups held in sc / requested into scn, of the current tile
+    // scales of the row: 8 groups (8 units) per 128-bit load; when a block of 8 is taken into use the tile's next block is
+    // prefetched into L1 (held in registers instead, it cost the two-term forms their spills)
+    uint4 sc[TERMS];
+    int cur_b = -1;                          // block of 8 groups held in sc, of the current tile
     const __half* srow[TERMS];               // the row's scales of the current tile (null: a row beyond N, scales read as 0)
     auto load_scales = [&](int g0, uint4* dst) {
 #pragma unroll
@@ -798,10 +928,10 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
     bool in_tile = false;
     int n = 0;
     for (;;) {
-      if (!(in_tile && (int32_t)(own - it0) < kstages)) {
+      if (!(in_tile && (int32_t)(own - it0) < units)) {
         // past the end of the current tile (or before the first): look up the next one
         if (in_tile) {
-          it0 += (uint32_t)kstages;
+          it0 += (uint32_t)units;
           gs0 += (uint32_t)nsb;
           in_tile = false;
         }
@@ -812,114 +942,140 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
 #pragma unroll
         for (int i = 0; i < TERMS; ++i)
           if (i < p.n_terms) srow[i] = n < p.N ? p.scale[i] + ((int64_t)e * p.N + n) * p.G : nullptr;
-        cur_b = nxt_b = -1;
+        cur_b = -1;
         in_tile = true;
         continue;
       }
-      const int ks = (int)(own - it0);
-        RT_DECL(t_pre = RT_NOW());
-        RT_SPAN(w_tail, t_tail);
-        const int sb = ks / SPB, sbk = ks - sb * SPB;
-        const uint32_t gs = gs0 + (uint32_t)sb;
-        const uint32_t slot = p.nslab == 2 ? (gs & 1u) : gs % 3u, sround = p.nslab == 2 ? (gs >> 1) : gs / 3u;
-        // scales
-        const int blk = ks >> 4;
-        if (blk != cur_b) {
-          if (nxt_b == blk) {
+      const int g = (int)(own - it0);  // the unit inside the tile = its scale group
+      RT_DECL(t_pre = RT_NOW());
+      RT_SPAN(w_tail, t_tail);
+      // scales
+      const int blk = g >> 3;
+      if (blk != cur_b) {
+        load_scales(blk * 8, sc);
+        cur_b = blk;
+        if ((blk + 1) * 8 < p.G) {  // the tile's next block, needed a few of this warp's units from now
 #pragma unroll
-            for (int i = 0; i < TERMS; ++i) sc[i] = scn[i];
-          } else {
-            load_scales(blk * 8, sc);
-          }
-          cur_b = blk;
-          if ((blk + 1) * 8 < p.G) {  // the tile's next block, needed a few of this warp's stages from now
-            load_scales((blk + 1) * 8, scn);
-            nxt_b = blk + 1;
-          }
+          for (int i = 0; i < TERMS; ++i)
+            if (i < p.n_terms && srow[i] != nullptr) asm volatile("prefetch.global.L1 [%0];" ::"l"(srow[i] + (blk + 1) * 8));
         }
-        const int g = (ks >> 1) & 7;  // 64-trit stage -> 128-trit scale group, inside the 8 held in sc
+      }
+      RT_SPAN(w_pre, t_pre);
 
-        // packed words of this row for this stage, then the slab can go back to the producer
-        RT_SPAN(w_pre, t_pre);
-        if (!RT_WAIT(w_pfull, mbar_wait(smem_u32(&bar_pfull[slot]), sround & 1u, abort_flag))) { ok = false; break; }
+      // packed words of this row for a piece, then (after the superblock's last piece of this group) the slab can go back to
+      // the producer. One term: both pieces' words up front; more: a piece at a time (registers).
+      constexpr int WX = TERMS == 1 ? 2 : 1;
+      uint32_t w[WX][TERMS][4];
+      int sbk[2];
+      auto load_piece = [&](int x, uint32_t (&dst)[TERMS][4]) -> bool {
+        const int ks = 2 * g + x, sb = ks / SPB;
+        sbk[x] = ks - sb * SPB;
+        const uint32_t gs = gs0 + (uint32_t)sb;
+        const uint32_t slot = p.nslab == 2 ? (gs & 1u) : gs % 3u;
+        const bool same = x == 1 && sbk[1] != 0;  // the first piece's slab
+        if (!same && !RT_WAIT(w_pfull, mbar_wait(smem_u32(&bar_pfull[gs % PF_BARS]), gs / PF_BARS & 1u, abort_flag))) return false;
         RT_DECL(t_lds = RT_NOW());
-        uint32_t w[TERMS][4];
 #pragma unroll
         for (int i = 0; i < TERMS; ++i) {
           if (i < p.n_terms) {
-            const uint32_t* wp = reinterpret_cast<const uint32_t*>(slabs + ((size_t)slot * p.n_terms + i) * PF_SLAB + r * 64);
+            const uint32_t wp = slabs_a + ((uint32_t)slot * p.n_terms + i) * PF_SLAB;
+            if (FMT == 2) {  // word 4 sbk + j
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int lw = FMT == 2 ? 4 * sbk + j : (j < 3 ? 3 * sbk + j : 15);  // logical word of the row-superblock
-              w[i][j] = wp[(((lw & 3) ^ swz) << 2) | (lw >> 2)];
+              for (int j = 0; j < 4; ++j) dst[i][j] = lds32(wp + unit_off[j] + sbk[x] * 4);
+            } else {         // words 3 sbk, 3 sbk + 1, 3 sbk + 2 and 15
+              switch (sbk[x]) {
+                case 0: dst[i][0] = lds32(wp + unit_off[0]); dst[i][1] = lds32(wp + unit_off[1]); dst[i][2] = lds32(wp + unit_off[2]); break;
+                case 1: dst[i][0] = lds32(wp + unit_off[3]); dst[i][1] = lds32(wp + unit_off[0] + 4); dst[i][2] = lds32(wp + unit_off[1] + 4); break;
+                case 2: dst[i][0] = lds32(wp + unit_off[2] + 4); dst[i][1] = lds32(wp + unit_off[3] + 4); dst[i][2] = lds32(wp + unit_off[0] + 8); break;
+                case 3: dst[i][0] = lds32(wp + unit_off[1] + 8); dst[i][1] = lds32(wp + unit_off[2] + 8); dst[i][2] = lds32(wp + unit_off[3] + 8); break;
+                default: dst[i][0] = lds32(wp + unit_off[0] + 12); dst[i][1] = lds32(wp + unit_off[1] + 12); dst[i][2] = lds32(wp + unit_off[2] + 12); break;
+              }
+              dst[i][3] = lds32(wp + unit_off[3] + 12);
             }
           }
         }
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(smem_u32(&bar_pempty[slot]));
-          // the tile's last superblock may hold fewer than SPB stages: make up for the stages that do not exist
-          if (ks == kstages - 1)
-            for (int x = nsb * SPB - kstages; x > 0; --x) mbar_arrive(smem_u32(&bar_pempty[slot]));
+          // the tile's last superblock may hold fewer than SPB pieces: make up for those that do not exist
+          const int n_arrive = 1 + (ks == kstages - 1 ? nsb * SPB - kstages : 0);
+          for (int y = 0; y < n_arrive; ++y) mbar_arrive(smem_u32(&bar_pempty[gs % PF_BARS]));
         }
-
 #ifdef DST_ROLE_TIMERS
 #pragma unroll
         for (int i = 0; i < TERMS; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) asm volatile("" : "+r"(w[i][j]));
+          for (int j = 0; j < 4; ++j) asm volatile("" : "+r"(dst[i][j]));
 #endif
         RT_SPAN(w_lds, t_lds);
+        return true;
+      };
+      if (TERMS == 1 && (!load_piece(0, w[0]) || !load_piece(1, w[WX - 1]))) break;
+
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int wx = TERMS == 1 ? x : 0;
+        if (TERMS > 1 && !load_piece(x, w[0])) { ok = false; break; }
+        if (!SMALL || x == 0) {
+          // the A slot must be free (the MMAs that last read it are done); waited for before the arithmetic, so that the
+          // dequantised words go to TMEM eight by eight as they come and need not all stay in registers
+          // no sleep between polls here: these warps are the critical path, and a sleeping lane wakes up to a
+          // microsecond late (the whole warp then waits for it at the next convergence point)
+          const uint32_t prev = gst - NA;  // the stage whose A slot this is
+          if (gst >= NA && !RT_WAIT(w_dempty, mbar_wait(smem_u32(&bar_empty[prev % PF_BARS]), prev / PF_BARS & 1u, abort_flag))) { ok = false; break; }
+          __syncwarp();  // re-converge after the polling loop: tcgen05.st is .sync.aligned
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
         RT_DECL(t_c = RT_NOW());
-        __half2 acc[32];
+        const uint32_t taddr = tmem + lane_base + (uint32_t)p.tn_max + s * (PF_A_COLS * KH) + (SMALL ? x * PF_A_COLS : 0);
+        if constexpr (FMT == 1) {
+          uint32_t pool[TERMS];
 #pragma unroll
-        for (int i = 0; i < TERMS; ++i) {
-          if (i < p.n_terms) {
-            const __half2 s2 = pick_scale(sc[i], g);
-            if (FMT == 2) {
+          for (int i = 0; i < TERMS; ++i) pool[i] = i < p.n_terms ? tq1_select_pool(pick_scale_bits(sc[i], g & 7)) : 0u;
+          tq1_stage_select<TABLE, TERMS>(w[wx], TERMS <= 2 ? TERMS : p.n_terms, table_a, table_a + tq1_select_place<TABLE>(sbk[x]), pool, taddr);
+        } else {
+          __half2 s2[TERMS];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                if (i == 0) tq2_word<true>(w[i][j], s2, acc + 8 * j);
-                else tq2_word<false>(w[i][j], s2, acc + 8 * j);
+          for (int i = 0; i < TERMS; ++i) s2[i] = i < p.n_terms ? pick_scale(sc[i], g & 7) : __float2half2_rn(0.f);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {  // word by word, all terms, so eight words at a time are live
+            __half2 acc[8];
+#pragma unroll
+            for (int i = 0; i < TERMS; ++i) {
+              if (i < p.n_terms) {
+                if (i == 0) tq2_word<true>(w[wx][i][j], s2[i], acc);
+                else tq2_word<false>(w[wx][i][j], s2[i], acc);
               }
-            } else {
-              if (i == 0) tq1_stage<true>(w[i], sbk, lut_addr, s2, acc);
-              else tq1_stage<false>(w[i], sbk, lut_addr, s2, acc);
             }
+            uint32_t v[8];
+#pragma unroll
+            for (int y = 0; y < 8; ++y) v[y] = h2_bits(acc[y]);
+            tmem_st_8(taddr + 8 * j, v);
           }
         }
-        uint32_t v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = h2_bits(acc[j]);
-#ifdef DST_ROLE_TIMERS
-#pragma unroll
-        for (int j = 0; j < 32; ++j) asm volatile("" : "+r"(v[j]));
         RT_SPAN(w_comp, t_c);
-        ++n_it;
-#endif
-        // the A slot must be free (the MMAs that last read it are done) before the store into it
-        // no sleep between polls here: these warps are the critical path, and a sleeping lane wakes up to a
-        // microsecond late (the whole warp then waits for it at the next convergence point)
-        if (!RT_WAIT(w_dempty, mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_flag))) { ok = false; break; }
-        __syncwarp();  // re-converge after the polling loop: tcgen05.st is .sync.aligned
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t taddr = tmem + lane_base + (uint32_t)p.tn_max + s * PF_A_COLS;
-        RT_DECL(t_st = RT_NOW());
-        tmem_st_8(taddr, v);
-        tmem_st_8(taddr + 8, v + 8);
-        tmem_st_8(taddr + 16, v + 16);
-        tmem_st_8(taddr + 24, v + 24);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_full[s]));
-        RT_SPAN(w_st, t_st);
+        if (!SMALL || x == 1) {
+          RT_DECL(t_st = RT_NOW());
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_full[gst % PF_BARS]));
+          RT_SPAN(w_st, t_st);
+        }
+        if (!SMALL && x == 0) {
+          ++gst;
+          if (++s == NA) s = 0;
+        }
+      }
+      if (!ok) break;
 #ifdef DST_ROLE_TIMERS
-        t_tail = RT_NOW();
+      ++n_it;
+      t_tail = RT_NOW();
 #endif
-        own += n_groups;
-        s += n_groups;
-        while (s >= NB) { s -= NB; ph ^= 1u; }
+      own += n_groups;
+      constexpr uint32_t jump = SMALL ? n_groups : 2 * n_groups - 1;  // to the first stage of the group's next unit
+      gst += jump;
+      s += jump;
+      while (s >= NA) s -= NA;
     }
     if (warp == PF_DQ_WARP0 && lane == 0) {
       RT_ADD(24, RT_NOW() - t_begin); RT_ADD(25, w_pfull); RT_ADD(26, w_dempty); RT_ADD(27, n_it); RT_ADD(28, 1);
@@ -989,33 +1145,9 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-template <int FMT, int TERMS>
-int launch_fmt(const TmaMaps& maps, PrefillParams p, cudaStream_t st) {
-  // Shared-memory and TMEM plan: the token tile is as large as the experts are expected to need (up to 320 rows) as
-  // long as a stage ring of depth 4 fits; smaller tiles leave room for a deeper ring (each B stage is tn_max * 128
-  // bytes, each A slot 32 TMEM columns next to tn_max accumulator columns), which is what hides the TMA latency
-  // when the MMAs of a stage are short. Then a third packed-slab slot if there is room for it.
-  const long long budget = PF_SMEM_MAX - PF_SMEM_STATIC;
-  const long long fixed = 1024 + (FMT == 1 ? PF_LUT_BYTES : 0) + 2 * (PF_MAX_E + 1) * 4 + (p.wide_drain ? 128 + PF_EPI_WARPS * PF_EPI_TILE : 0);
-  const long long slab2 = 2LL * p.n_terms * PF_SLAB;
-  int tn_cap = (p.rows_hint + 31) / 32 * 32;
-  tn_cap = tn_cap < 64 ? 64 : (tn_cap > PF_TN_MAX ? PF_TN_MAX : tn_cap);
-  p.tn_max = 0;
-  for (int tn = tn_cap; tn >= 64; tn -= 32) {
-    long long nb = (budget - fixed - slab2) / (tn * 128LL);
-    if (nb >= 4 || tn == 64) {
-      const long long tmem_fit = (512 - tn) / PF_A_COLS;
-      nb = nb > tmem_fit ? tmem_fit : nb;
-      p.tn_max = tn;
-      p.nb = (int)(nb > PF_MAX_STAGES ? PF_MAX_STAGES : nb);
-      break;
-    }
-  }
-  if (p.tn_max == 0 || p.nb < 2) return DST_ERR_UNSUPPORTED;
-  p.nslab = fixed + 3LL * p.n_terms * PF_SLAB + (long long)p.nb * p.tn_max * 128 <= budget ? 3 : 2;
-  p.small = p.tn_max <= 128 ? 1 : 0;
-  const size_t smem = (size_t)(fixed + (long long)p.nslab * p.n_terms * PF_SLAB + (long long)p.nb * p.tn_max * 128);
-  auto kernel = prefill_kernel<FMT, TERMS>;
+template <int FMT, int TERMS, bool SMALL>
+int launch_plan(const TmaMaps& maps, const PrefillParams& p, size_t smem, cudaStream_t st) {
+  auto kernel = prefill_kernel<FMT, TERMS, SMALL>;
   DST_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 148;
   DST_CUDA_TRY(cudaGetDevice(&dev));
@@ -1026,9 +1158,63 @@ int launch_fmt(const TmaMaps& maps, PrefillParams p, cudaStream_t st) {
   if (tiles_upper < 1) tiles_upper = 1;
   unsigned grid = (unsigned)(tiles_upper < sms ? tiles_upper : sms);
   if (g_debug_max_ctas > 0 && grid > (unsigned)g_debug_max_ctas) grid = (unsigned)g_debug_max_ctas;
-  prefill_kernel<FMT, TERMS><<<grid, PF_THREADS, smem, st>>>(maps, p);
+  kernel<<<grid, PF_THREADS, smem, st>>>(maps, p);
   DST_CUDA_TRY(cudaGetLastError());
   return DST_OK;
+}
+
+// Places the parts of a CTA's shared memory for p.tn_max, with at least min_nb B stages: sets nb, na, nslab and the
+// addresses, returns the dynamic bytes (0: does not fit).
+template <int FMT, int TERMS, bool SMALL>
+size_t plan_smem(PrefillParams& p, int min_nb) {
+  constexpr int TABLE = pf_table(FMT, TERMS, SMALL), KH = SMALL ? 2 : 1;
+  const long long stage = p.tn_max * 128LL * KH, slab = (long long)p.n_terms * PF_SLAB;
+  const long long front = 2 * (PF_MAX_E + 1) * 4 + (p.row_target ? 2 * (SMALL ? PF_SMALL_TN : PF_TN_MAX) * 8 : 0) +
+                          (p.wide_drain ? (SMALL ? 4 : PF_EPI_WARPS) * PF_EPI_TILE : 0);
+  const long long na = (512 - p.tn_max) / (PF_A_COLS * KH);
+  p.na = (int)(na < PF_MAX_STAGES ? na : PF_MAX_STAGES);
+  for (p.nslab = 3; p.nslab >= 2; --p.nslab) {
+    const long long slabs = p.nslab * slab;
+    long long ring_at, room;  // start of the ring, bytes for it
+    if (TABLE == PF_TABLE_64K) {  // slabs, front | table at 64 KB | ring
+      if (PF_SMEM_START + slabs + front > 0x10000) continue;
+      ring_at = 0x20000;
+      room = PF_SMEM_END - ring_at;
+    } else if (TABLE == PF_TABLE_32K) {  // front | table at 32 KB | ring, slabs
+      if (PF_SMEM_START + front > 0x8000) continue;
+      ring_at = 0x10000;
+      room = PF_SMEM_END - ring_at - slabs;
+    } else {  // ring, slabs, front
+      ring_at = PF_SMEM_START;
+      room = PF_SMEM_END - ring_at - slabs - front;
+    }
+    long long nb = room / stage;
+    if (nb > p.na) nb = p.na;
+    if (nb < min_nb) continue;
+    p.nb = (int)nb;
+    const long long ring_end = ring_at + nb * stage;
+    p.a_ring = (uint32_t)ring_at;
+    p.a_table = TABLE == PF_TABLE_64K ? 0x10000u : 0x8000u;
+    p.a_slabs = TABLE == PF_TABLE_64K ? PF_SMEM_START : (uint32_t)ring_end;
+    p.a_front = TABLE == PF_TABLE_64K ? (uint32_t)(PF_SMEM_START + slabs) : TABLE == PF_TABLE_32K ? PF_SMEM_START : (uint32_t)(ring_end + slabs);
+    const long long end = TABLE == PF_TABLE_64K ? ring_end : TABLE == PF_TABLE_32K ? ring_end + slabs : ring_end + slabs + front;
+    return (size_t)(end - PF_SMEM_FIRST);
+  }
+  return 0;
+}
+
+template <int FMT, int TERMS>
+int launch_fmt(const TmaMaps& maps, PrefillParams p, cudaStream_t st) {
+  // The token tile is as large as the experts are expected to need (up to 320 rows) as long as a B ring of four 64-K stages
+  // fits: that much hides the latency of the copies behind the MMAs of a stage. Then a third packed-slab slot if there is
+  // room for it.
+  int tn_cap = (p.rows_hint + 31) / 32 * 32;
+  tn_cap = tn_cap < 64 ? 64 : (tn_cap > PF_TN_MAX ? PF_TN_MAX : tn_cap);
+  for (p.tn_max = tn_cap; p.tn_max > PF_SMALL_TN; p.tn_max -= 32)
+    if (const size_t smem = plan_smem<FMT, TERMS, false>(p, 4)) return launch_plan<FMT, TERMS, false>(maps, p, smem, st);
+  for (; p.tn_max >= 64; p.tn_max -= 32)
+    if (const size_t smem = plan_smem<FMT, TERMS, true>(p, 2)) return launch_plan<FMT, TERMS, true>(maps, p, smem, st);
+  return DST_ERR_UNSUPPORTED;
 }
 
 }  // namespace
@@ -1120,8 +1306,12 @@ int launch_prefill(const GemmArgs& a, cudaStream_t stream) {
   p.NT = (int)cdiv64(a.N, 128);
   p.S = (int)tiled_superblocks(a.fmt, a.K);
   p.kstages = (int)(a.K / 64);
-  // rows per expert: known when the caller passed host offsets, else assumed below twice the mean
-  p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : 2 * cdiv64(a.T, a.E));
+  // Rows per expert: known when the caller passed host offsets, else three standard deviations of an even routing above the
+  // mean (an expert with more is split into two tiles, which dequantises its weights twice; a tile sized for twice the mean
+  // costs every expert the form of the kernel for larger tiles: 96 rows on 96 experts of 4096 x 4096, TQ1, 428 against
+  // 596 us)
+  const int64_t mean = cdiv64(a.T, a.E);
+  p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : mean + (int64_t)ceil(3.0 * sqrt((double)mean)));
   if (p.rows_hint < 1) p.rows_hint = 1;
 #define DST_PF_LAUNCH(FMT_)                                                            \
   (a.terms.n == 1 ? launch_fmt<FMT_, 1>(maps, p, stream)                               \

@@ -412,6 +412,35 @@ def test_prefill_many_tiles_per_cta(kb, fmt):
         check_gemm(y[a:b], x[a:b], [(terms[0][0][e], terms[0][1][e])], K, 128, fmt)
 
 
+@pytest.mark.parametrize("fmt", ["tq1", "tq2"])
+@pytest.mark.parametrize("k_terms", [1, 2, 3])
+@pytest.mark.parametrize("K", [128, 384, 640, 2048])
+def test_prefill_both_forms_at_their_edges(kb, fmt, k_terms, K):
+    """The tcgen05 kernel's two forms (token tiles up to 128 rows and above) with every table and term count, from one unit of
+    128 trits per tile on (the dequant groups then jump over several tiles), tiles of 1 to 320 rows and one expert that is
+    split, a ragged N, few CTAs so that each walks many tiles."""
+    N = 300
+    lib = kb.ext()
+    for counts in ([1, 0, 33, 128, 7], [16, 129, 320, 0, 321]):
+        E = len(counts)
+        rng = np.random.default_rng(K + k_terms + counts[0])
+        terms = make_terms(rng, N, K, 128, fmt, k_terms, lead=(E,))
+        offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+        x = O.synth_acts(rng, (int(offsets[-1]), K))
+        tiled = [kb.tile_weights(torch.from_numpy(p).to(DEV), fmt, K) for p, _ in terms]
+        try:
+            assert lib.dst_debug_prefill_timeout(0, 0, 2) == 0  # two CTAs
+            y = kb.grouped_ternary_gemm_bf16(bf16_tensor(x, DEV), offsets, tiled, [torch.from_numpy(s).to(DEV) for _, s in terms], K, 128, fmt,
+                                             algo="prefill").cpu().numpy()
+            assert lib.dst_check_device_status(None) == 0
+        finally:
+            lib.dst_debug_prefill_timeout(0, 0, 0)
+        for e in range(E):
+            a, b = int(offsets[e]), int(offsets[e + 1])
+            if b > a:
+                check_gemm(y[a:b], x[a:b], [(p[e], s[e]) for p, s in terms], K, 128, fmt)
+
+
 @pytest.mark.parametrize("N", [200, 196, 384])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16])
 def test_prefill_sixteen_bit_outputs_equal_rounded_fp32_outputs(kb, N, out_dtype):
