@@ -16,7 +16,7 @@ from pathlib import Path
 CSRC = Path(__file__).resolve().parent / "csrc"
 LIB_PATH = CSRC / "libdst_b200.so"
 SOURCES = ["api.cu", "format_kernels.cu", "layout_kernels.cu", "gemm_generic.cu", "gemm_decode.cu", "gemm_decode_tq1.cu", "gemm_prefill.cu", "ep_kernels.cu",
-           "moe_kernels.cu"]
+           "moe_kernels.cu", "moe_layer.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-shared",
               "-Xcompiler", "-fPIC"]
 
@@ -61,6 +61,13 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB_PATH
 
 
+class ExpertWeightsC(ctypes.Structure):
+    """``dst_expert_weights`` of ``include/dst_b200.h``."""
+
+    _fields_ = [(name, ctypes.c_void_p * MAX_TERMS) for name in ("w13", "s13", "w2", "s2", "w13_decode", "w2_decode")] + \
+               [(name, ctypes.c_int64) for name in ("experts", "hidden", "inter")] + [("n_terms", ctypes.c_int), ("fmt", ctypes.c_int)]
+
+
 _SIGNATURES = {
     # name: (restype, argtypes)
     "dst_abi_version": (ctypes.c_int, []),
@@ -74,6 +81,10 @@ _SIGNATURES = {
     "dst_quant_act_int8_f16": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p,
                                               ctypes.c_void_p, ctypes.c_void_p]),
     "dst_decode_row_limit": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int64, ctypes.c_int64]),
+    "dst_moe_layer_workspace_bytes": (ctypes.c_size_t, [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]),
+    "dst_moe_layer": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_float,
+                                     ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]),
+    "dst_decode_auto_rows": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64]),
     "dst_ternary_grouped_gemm": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
                                                 ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
                                                 ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int64,

@@ -52,7 +52,20 @@ struct GemmArgs {
   void* peer_out[DST_MAX_PEERS];
   int n_peer_out;     // targets naming a buffer >= n_peer_out or a row >= peer_rows are not stored
   int64_t peer_rows;
+  // decode GEMV with a workspace only: row r of the problem is row (gather_order[r] / gather_top_k) of x (null: row r)
+  const int64_t* gather_order;
+  int gather_top_k;
+  int quantised;      // ... and the workspace already holds the quantised rows (decode_swiglu_quant): x is not read
 };
+
+// Every kernel that follows `order` clamps the entry to [0, n): an order array that was not produced by the routing
+// sort (or one whose tail belongs to dropped ids) can then make a row wrong, but cannot make an access leave the buffers.
+__device__ __forceinline__ int64_t clamp_slot(int64_t f, int64_t n) { return f < 0 ? 0 : (f >= n ? n - 1 : f); }
+
+__device__ __forceinline__ float silu_fast(float g) {
+  // g * sigmoid(g) with the hardware's exp2 and reciprocal approximations (2 ulp each; the result is rounded to bf16)
+  return __fdividef(g, 1.f + __expf(-g));
+}
 
 int64_t tiled_superblocks(int fmt, int64_t K);
 size_t prefill_workspace_bytes(int act_dtype, int64_t T, int64_t K);
@@ -62,11 +75,21 @@ int launch_generic(const GemmArgs& a, cudaStream_t stream);
 int launch_decode(const GemmArgs& a, cudaStream_t stream);    // DST_ERR_UNSUPPORTED when not covered
 int launch_prefill(const GemmArgs& a, cudaStream_t stream);   // DST_ERR_UNSUPPORTED when not covered
 bool decode_supports(const GemmArgs& a);
-int64_t decode_row_limit(int fmt, int64_t E, int64_t N);  // rows per expert up to which AUTO prefers the decode GEMV
+int64_t decode_row_limit(int fmt, int64_t E, int64_t N);
+int64_t decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N);  // rows per expert up to which AUTO prefers the decode GEMV
 int launch_decode_tq1(const GemmArgs& a, cudaStream_t stream);  // TQ1 decode kernel (gemm_decode_tq1.cu); reached through launch_decode
 bool decode_tq1_supports(const GemmArgs& a);
 bool prefill_supports(const GemmArgs& a);
+// SwiGLU of gate / up rows straight into the decode GEMV's quantised form (in `workspace`, as launch_decode lays it out for T
+// rows of K = inter); standard: the OLMoE rounding points, no weight, no clamp
+int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const int64_t* order, int64_t T, int64_t inter, float limit,
+                        bool standard, void* workspace, cudaStream_t stream);
 int decode_take_status(int* status);
+// moe_kernels.cu: the routing sort with the inverse order (inv may be null), and the combine from it
+int sort_rows(const void* ids, int ids_are_i32, int64_t n, int64_t E, int64_t* order, int64_t* offsets, int32_t* bad_count, void* workspace,
+              int64_t* inv, cudaStream_t st);
+int combine_rows(const void* down_bf16, const int64_t* inv, const int32_t* ids, const float* weights, int64_t T, int top_k, int64_t hidden,
+                 const void* add_bf16, void* y_bf16, cudaStream_t st);
 int ep_take_status(int* status);      // the same for the expert-parallel barrier kernel  // reads and clears the decode kernel's status word (0 or DST_ERR_TIMEOUT)
 
 // ---------------------------------------------------------------------------------------------

@@ -37,7 +37,9 @@
 //
 // Coverage: TQ2 tiled weights, group 128, K % 512 == 0 (a ring slot is two 256-trit superblocks), fp16 scales, bf16 / fp16 / int8 activations, any row
 // count per expert (rows are processed up to 16 at a time; beyond that the weights are streamed again, from L2).
-#include "dst_common.cuh"
+#include <cstring>
+
+#include "decode_units.cuh"
 
 namespace dst {
 namespace {
@@ -56,9 +58,6 @@ __host__ __device__ constexpr int dc_slot(int cw) { return dc_slot_data(cw) + 16
 constexpr int DC_RING_MAX = DC_RING_SLOTS;        // slots of the slab ring (fewer, at least 2, when shared memory is short)
 #ifndef DC_PRODUCER_SLEEP
 #define DC_PRODUCER_SLEEP true
-#endif
-#ifndef DC_PREQ_ABOVE
-#define DC_PREQ_ABOVE 0
 #endif
 constexpr int DC_ZERO = 512;                      // bytes of zeros the lanes without a column read
 constexpr long long DC_WAIT_CYCLES = 4000000000LL;  // ~2 s
@@ -141,111 +140,6 @@ __device__ __forceinline__ void mma_u8s8(int* d, uint32_t a0, uint32_t a1, uint3
   else
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// ------------------------------------------------------------------------------------------ work units
-// A work unit is (expert, pass, block of RI = 64, 128 or 256 weight rows): pass i covers the expert's token rows
-// ra + i MT .. (MT at most). Only experts with rows have units; they are numbered expert by expert, pass by pass, row
-// block by row block, and every CTA takes an equal, contiguous run of them, so a pass's token rows are staged once per CTA.
-// Experts without rows get no share of the grid: a decode step that reaches 6 of 384 experts ran on ten of the 592 CTAs
-// when the runs were cut over all experts' row blocks (one token, two stacked terms: 563 us for both GEMVs).
-template <int RI>
-__host__ __device__ __forceinline__ int blocks_per_expert(int NT) { return (NT * 128 + RI - 1) / RI; }
-
-struct Unit {
-  int e, n0;           // expert and first weight row
-  int64_t ra, rb, m0;  // the expert's token rows [ra, rb) and the pass's first one
-};
-
-// A warp's position in the unit sequence (the same in all its lanes; every call is made by the whole warp).
-template <int MT, int RI>
-struct UnitWalk {
-  int block, blocks;  // row block inside the pass
-  Unit u;
-  // local = the unit's index among the units of expert e (which has rows)
-  __device__ __forceinline__ void start(const DecodeParams& p, int e, long long local) {
-    blocks = blocks_per_expert<RI>(p.NT);
-    u.e = e;
-    row_range(p.offsets, e, p.T, u.ra, u.rb);
-    const long long pass = local / blocks;
-    block = (int)(local - pass * blocks);
-    u.m0 = u.ra + pass * MT;
-    u.n0 = block * RI;
-  }
-  __device__ __forceinline__ void next(const DecodeParams& p) {
-    if (++block == blocks) {
-      block = 0;
-      u.m0 += MT;
-      if (u.m0 >= u.rb) {
-        // the next expert with rows, 32 at a time (an empty or inverted range has none)
-        const int lane = threadIdx.x & 31;
-        for (int e0 = u.e + 1; e0 < p.E; e0 += 32) {
-          int64_t a = 0, b = 0;
-          if (e0 + lane < p.E) row_range(p.offsets, e0 + lane, p.T, a, b);
-          const uint32_t some = __ballot_sync(0xffffffffu, b > a);
-          if (some) {
-            const int src = __ffs(some) - 1;
-            u.e = e0 + src;
-            u.ra = __shfl_sync(0xffffffffu, a, src);
-            u.rb = __shfl_sync(0xffffffffu, b, src);
-            break;
-          }
-        }
-        u.m0 = u.ra;
-      }
-    }
-    u.n0 = block * RI;
-  }
-};
-
-// The CTA's run of units, found by all its threads together: every thread counts the units of a contiguous run of experts,
-// a block-wide scan gives their number and the expert that holds the CTA's first unit. scratch: one long long per warp.
-struct UnitRun {
-  long long count;    // units of this CTA
-  long long local;    // the first one's index among the units of expert e
-  int e;
-};
-template <int MT, int RI, int THREADS>
-__device__ __forceinline__ void find_run(const DecodeParams& p, long long* scratch, UnitRun* run) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (p.E + THREADS - 1) / THREADS;
-  const int e0 = threadIdx.x * per, e1 = e0 + per < p.E ? e0 + per : p.E;
-  const int blocks = blocks_per_expert<RI>(p.NT);
-  auto units_of = [&](int e) -> long long {
-    int64_t a, b;
-    row_range(p.offsets, e, p.T, a, b);
-    return (b - a + MT - 1) / MT * blocks;
-  };
-  long long sum = 0;
-  for (int e = e0; e < e1; ++e) sum += units_of(e);
-  long long incl = sum;
-  for (int d = 1; d < 32; d <<= 1) {
-    const long long up = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += up;
-  }
-  if (lane == 31) scratch[warp] = incl;
-  if (threadIdx.x == 0) run->count = 0;
-  __syncthreads();
-  long long before = incl - sum, total = 0;
-  for (int w = 0; w < THREADS / 32; ++w) {
-    if (w < warp) before += scratch[w];
-    total += scratch[w];
-  }
-  const long long u0 = total * blockIdx.x / gridDim.x, u1 = total * (blockIdx.x + 1) / gridDim.x;
-  if (u0 < u1 && u0 >= before && u0 < before + sum) {
-    long long left = u0 - before;
-    for (int e = e0; e < e1; ++e) {
-      const long long n = units_of(e);
-      if (left < n) {
-        run->e = e;
-        run->local = left;
-        run->count = u1 - u0;
-        break;
-      }
-      left -= n;
-    }
-  }
-  __syncthreads();
 }
 
 // ------------------------------------------------------------------------------------------ staging
@@ -381,18 +275,62 @@ __device__ bool stage_tokens(const DecodeParams& p, const XT* __restrict__ x, in
 
 // The staging above done ONCE per token, ahead of the GEMV, into global memory: with more than a few rows per expert
 // the GEMV's CTAs would otherwise repeat it for every expert they touch (measured at 8 rows: a quarter to a half of
-// their instructions). One block of DC_QWARPS warps per token row.
+// their instructions). One block of DC_QWARPS warps per row; `order`: the row is row order[t] / top_k of x (a MoE step's
+// gather, which needs no pass of its own then).
 template <typename XT>
 __global__ void __launch_bounds__(DC_QWARPS * 32)
-decode_quant_kernel(const DecodeParams p, uint8_t* __restrict__ q_rows, int* __restrict__ q_xsum4, float* __restrict__ q_xexp) {
+decode_quant_kernel(const DecodeParams p, const int64_t* __restrict__ order, int top_k, uint8_t* __restrict__ q_rows, int* __restrict__ q_xsum4,
+                    float* __restrict__ q_xexp) {
   __shared__ float xinv[DC_QWARPS];
   const int64_t t = blockIdx.x;
+  const int64_t src = order ? clamp_slot(order[t], (int64_t)p.T) / top_k : t;
   auto sync = []() -> bool {
     __syncthreads();
     return true;
   };
-  // token t as a "pass" of one row: row_scale, the row pointer and the outputs are all indexed by t through m0 = t
-  stage_tokens<1, DC_QWARPS>(p, static_cast<const XT*>(p.x), t, 1, q_rows + (size_t)t * 2 * p.K, (size_t)p.K, q_xsum4 + t * p.G, p.G, q_xexp + t, xinv, sync);
+  // token t as a "pass" of one row: row_scale and the row pointer are indexed by its source row
+  stage_tokens<1, DC_QWARPS>(p, static_cast<const XT*>(p.x), src, 1, q_rows + (size_t)t * 2 * p.K, (size_t)p.K, q_xsum4 + t * p.G, p.G, q_xexp + t, xinv, sync);
+}
+
+// SwiGLU of one row (the rounding points of the layer's SwiGLU kernels), kept in shared memory as bf16, then quantised as
+// above: one pass over gate and up where a SwiGLU kernel wrote the row and the quantisation read it back.
+template <bool STANDARD>
+__global__ void __launch_bounds__(DC_QWARPS * 32)
+decode_swiglu_quant_kernel(const DecodeParams p, const __nv_bfloat16* __restrict__ gu, const float* __restrict__ route_weights,
+                           const int64_t* __restrict__ order, float limit, uint8_t* __restrict__ q_rows, int* __restrict__ q_xsum4,
+                           float* __restrict__ q_xexp) {
+  extern __shared__ __align__(16) uint8_t sq_smem[];
+  __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(sq_smem);
+  __shared__ float xinv[DC_QWARPS];
+  const int64_t t = blockIdx.x;
+  const float w = route_weights ? route_weights[order ? clamp_slot(order[t], (int64_t)p.T) : t] : 1.f;
+  const __nv_bfloat16* g = gu + t * 2 * p.K;
+  const __nv_bfloat16* u = g + p.K;
+  for (int i = threadIdx.x * 2; i < p.K; i += DC_QWARPS * 64) {
+    const float2 gate = load_pair(g + i), up = load_pair(u + i);
+    float v[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float ga = j ? gate.y : gate.x, uu = j ? up.y : up.x;
+      if (STANDARD) {
+        v[j] = __bfloat162float(__float2bfloat16_rn(silu_fast(ga))) * uu;
+      } else {
+        if (limit > 0.f) {
+          uu = fminf(fmaxf(uu, -limit), limit);
+          ga = fminf(ga, limit);
+        }
+        v[j] = silu_fast(ga) * uu;
+        if (route_weights) v[j] = w * v[j];
+      }
+    }
+    reinterpret_cast<__nv_bfloat162*>(h)[i >> 1] = __floats2bfloat162_rn(v[0], v[1]);
+  }
+  __syncthreads();
+  auto sync = []() -> bool {
+    __syncthreads();
+    return true;
+  };
+  stage_tokens<1, DC_QWARPS>(p, h, 0, 1, q_rows + (size_t)t * 2 * p.K, (size_t)p.K, q_xsum4 + t * p.G, p.G, q_xexp + t, xinv, sync);
 }
 
 // ------------------------------------------------------------------------------------------ the kernel
@@ -895,18 +833,60 @@ int launch_rows(const DecodeParams& p, int64_t rows_hint, bool rows_known, int s
 }  // namespace
 
 // Scratch of the pre-quantised activations: [T][2][K] s8 rows, [T][G] int32 sums, [T] float factors (each part 256-byte aligned).
+namespace {
+size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
+struct QuantRows {
+  uint8_t* rows;
+  int* xsum4;
+  float* xexp;
+  QuantRows(void* base, int64_t T, int64_t K) {
+    rows = static_cast<uint8_t*>(base);
+    uint8_t* sums = rows + up256((size_t)T * 2 * (size_t)K);
+    xsum4 = reinterpret_cast<int*>(sums);
+    xexp = reinterpret_cast<float*>(sums + up256((size_t)T * (size_t)(K / 128) * 4));
+  }
+};
+}  // namespace
 size_t decode_workspace_bytes(int64_t T, int64_t K) {
-  const size_t G = (size_t)(K / 128);
-  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  return up((size_t)T * 2 * (size_t)K) + up((size_t)T * G * 4) + up((size_t)T * 4);
+  return up256((size_t)T * 2 * (size_t)K) + up256((size_t)T * (size_t)(K / 128) * 4) + up256((size_t)T * 4);
 }
 
-// Up to how many token rows per expert the decode GEMV beats the tcgen05 kernel (measured on 4096 x 4096 experts): 32
+int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const int64_t* order, int64_t T, int64_t inter, float limit,
+                        bool standard, void* workspace, cudaStream_t stream) {
+  if (inter % 128 != 0 || inter > 16384 || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0 || (reinterpret_cast<uintptr_t>(gu_bf16) & 3) != 0)
+    return DST_ERR_UNSUPPORTED;  // a row is kept in 32 KB of shared memory at most
+  DecodeParams p;
+  memset(&p, 0, sizeof(p));
+  p.T = (int)T;
+  p.K = (int)inter;
+  p.G = (int)(inter / 128);
+  const QuantRows q(workspace, T, inter);
+  auto gu = static_cast<const __nv_bfloat16*>(gu_bf16);
+  const size_t smem = (size_t)inter * 2;
+  if (standard) decode_swiglu_quant_kernel<true><<<(unsigned)T, DC_QWARPS * 32, smem, stream>>>(p, gu, nullptr, nullptr, 0.f, q.rows, q.xsum4, q.xexp);
+  else decode_swiglu_quant_kernel<false><<<(unsigned)T, DC_QWARPS * 32, smem, stream>>>(p, gu, route_weights, order, limit, q.rows, q.xsum4, q.xexp);
+  DST_CUDA_TRY(cudaGetLastError());
+  return DST_OK;
+}
+
+// Up to how many token rows per expert the decode GEMV can beat the tcgen05 kernel (measured on 4096 x 4096 experts): 32
 // where the many-row CTAs apply (TQ2 tiles, a 256-row unit for every SM; two passes of 16 rows), else 16.
-int64_t decode_row_limit(int fmt, int64_t E, int64_t N) {
+static int sm_count() {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return fmt == DST_FMT_TQ2 && E * ((N + 255) / 256) >= sms ? 32 : 16;
+  return sms;
+}
+int64_t decode_row_limit(int fmt, int64_t E, int64_t N) {
+  return fmt == DST_FMT_TQ2 && E * ((N + 255) / 256) >= sm_count() ? 32 : 16;
+}
+
+// ... and up to how many AUTO takes it for T rows. One TQ1 term: the GEMV runs at 1.0 TB/s of packed bytes with one row per
+// expert and 0.6 with eight, the tcgen05 kernel at 1.03 whatever the rows (48 experts of 4096 x 4096: 172 / 270 us against 167 / 169), so the
+// GEMV is left the steps whose units all run at once (6 experts, one row each: 45 against 58 us) and not a single matrix
+// (11008 x 4096, four rows: 61 against 32 us). More terms: the tcgen05 kernel adds them in fp16, the GEMV one by one in fp32.
+int64_t decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N) {
+  if (fmt != DST_FMT_TQ1 || n_terms > 1) return decode_row_limit(fmt, E, N);
+  return E > 1 && T * ((N + 255) / 256) <= sm_count() ? 8 : 0;
 }
 
 bool decode_supports(const GemmArgs& a) {
@@ -924,7 +904,7 @@ int launch_decode(const GemmArgs& a, cudaStream_t stream) {
   for (int i = 0; i < a.terms.n; ++i)
     if ((reinterpret_cast<uintptr_t>(a.terms.packed[i]) & 15) != 0 || (reinterpret_cast<uintptr_t>(a.terms.scale[i]) & 3) != 0)
       return DST_ERR_ALIGNMENT;  // slabs are bulk-copied (16 bytes); scales are read two groups (32 bits) at a time
-  if ((reinterpret_cast<uintptr_t>(a.x) & 15) != 0) return DST_ERR_ALIGNMENT;  // rows are read with 128-bit loads
+  if (!a.quantised && (reinterpret_cast<uintptr_t>(a.x) & 15) != 0) return DST_ERR_ALIGNMENT;  // rows are read with 128-bit loads
   DecodeParams p;
   for (int i = 0; i < DST_MAX_TERMS; ++i) {
     p.tiled[i] = i < a.terms.n ? a.terms.packed[i] : nullptr;
@@ -955,21 +935,24 @@ int launch_decode(const GemmArgs& a, cudaStream_t stream) {
   int dev = 0, sms = 148;
   DST_CUDA_TRY(cudaGetDevice(&dev));
   DST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // More than two rows per expert and a workspace: quantise every token once, ahead of the GEMV
-  if (rows_hint > DC_PREQ_ABOVE && a.workspace != nullptr && a.workspace_bytes >= decode_workspace_bytes(a.T, a.K) &&
-      (reinterpret_cast<uintptr_t>(a.workspace) & 255) == 0) {
-    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    uint8_t* base = static_cast<uint8_t*>(a.workspace);
-    uint8_t* q_rows = base;
-    int* q_xsum4 = reinterpret_cast<int*>(base + up((size_t)a.T * 2 * (size_t)a.K));
-    float* q_xexp = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(q_xsum4) + up((size_t)a.T * (size_t)a.G * 4));
-    if (a.act_dtype == DST_ACT_BF16) decode_quant_kernel<__nv_bfloat16><<<(unsigned)a.T, DC_QWARPS * 32, 0, stream>>>(p, q_rows, q_xsum4, q_xexp);
-    else if (a.act_dtype == DST_ACT_F16) decode_quant_kernel<__half><<<(unsigned)a.T, DC_QWARPS * 32, 0, stream>>>(p, q_rows, q_xsum4, q_xexp);
-    else decode_quant_kernel<int8_t><<<(unsigned)a.T, DC_QWARPS * 32, 0, stream>>>(p, q_rows, q_xsum4, q_xexp);
-    DST_CUDA_TRY(cudaGetLastError());
-    p.q_rows = q_rows;
-    p.q_xsum4 = q_xsum4;
-    p.q_xexp = q_xexp;
+  // A workspace: quantise every token once, ahead of the GEMV
+  if (a.workspace != nullptr && a.workspace_bytes >= decode_workspace_bytes(a.T, a.K) && (reinterpret_cast<uintptr_t>(a.workspace) & 255) == 0) {
+    const QuantRows q(a.workspace, a.T, a.K);
+    if (!a.quantised) {
+      const unsigned grid = (unsigned)a.T;
+      if (a.act_dtype == DST_ACT_BF16)
+        decode_quant_kernel<__nv_bfloat16><<<grid, DC_QWARPS * 32, 0, stream>>>(p, a.gather_order, a.gather_top_k, q.rows, q.xsum4, q.xexp);
+      else if (a.act_dtype == DST_ACT_F16)
+        decode_quant_kernel<__half><<<grid, DC_QWARPS * 32, 0, stream>>>(p, a.gather_order, a.gather_top_k, q.rows, q.xsum4, q.xexp);
+      else
+        decode_quant_kernel<int8_t><<<grid, DC_QWARPS * 32, 0, stream>>>(p, a.gather_order, a.gather_top_k, q.rows, q.xsum4, q.xexp);
+      DST_CUDA_TRY(cudaGetLastError());
+    }
+    p.q_rows = q.rows;
+    p.q_xsum4 = q.xsum4;
+    p.q_xexp = q.xexp;
+  } else if (a.gather_order != nullptr || a.quantised) {
+    return DST_ERR_BAD_ARG;  // both need the workspace
   }
   if (a.act_dtype == DST_ACT_BF16) return launch_rows<__nv_bfloat16>(p, rows_hint, a.max_rows >= 0, sms, stream);
   if (a.act_dtype == DST_ACT_F16) return launch_rows<__half>(p, rows_hint, a.max_rows >= 0, sms, stream);

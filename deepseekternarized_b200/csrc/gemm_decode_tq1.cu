@@ -27,10 +27,12 @@
 // One warp owns 16 weight rows of a 128-row tile; a CTA of 16 warps works on two neighbouring row tiles of one
 // expert at a time, so 8 staged token rows (up to ~17 KB each for K = 4096: the slots are laid out in the order
 // the lanes consume them, zeros included) serve 256 weight rows. Up to 8 token rows per pass; an expert with
-// more rows is processed in several passes (the weights are re-read, from L2).
+// more rows is processed in several passes (the weights are re-read, from L2). The CTAs' runs of units are cut over the
+// experts that have rows (decode_units.cuh): 8 tokens on 384 experts, both GEMVs 1213 us cut over all experts, ~260 now.
+// AUTO leaves it the steps that decode_auto_rows (gemm_decode.cu) names: the tcgen05 kernel is as fast for many units.
 //
 // Coverage: TQ1 tiled weights, group 128, K % 128 == 0, fp16 scales, bf16 or fp16 activations.
-#include "dst_common.cuh"
+#include "decode_units.cuh"
 
 namespace dst {
 namespace {
@@ -305,21 +307,23 @@ decode_tq1_kernel(const Decode1Params p) {
   }
   const uint32_t lut_addr = (uint32_t)__cvta_generic_to_shared(lut) + (uint32_t)lane * 4u;
 
-  // work items: (expert, pair of neighbouring 128-row tiles); a contiguous range per CTA
-  const int NTP = (p.NT + 1) >> 1;
-  const long long items = (long long)p.E * NTP;
-  const long long per = (items + gridDim.x - 1) / gridDim.x;
-  const long long i0 = (long long)blockIdx.x * per, i1 = i0 + per < items ? i0 + per : items;
+  // work units: (expert, pass of D1_MT token rows, pair of neighbouring 128-row tiles), a contiguous run per CTA
+  __shared__ long long scan_s[D1_WARPS];
+  __shared__ UnitRun run_s;
+  find_run<D1_MT, 256, D1_THREADS>(p, scan_s, &run_s);
+  const long long n_units = run_s.count;
   int staged_e = -1;
   int64_t staged_m0 = -1;
 
-  for (long long item = i0; item < i1; ++item) {
-    const int e = (int)(item / NTP), ntp = (int)(item - (long long)e * NTP);
-    const int nt = ntp * 2 + (warp >> 3);  // warps 0-7: first tile of the pair, warps 8-15: second
-    int64_t ra, rb;
-    row_range(p.offsets, e, p.T, ra, rb);
-    for (int64_t m0 = ra; m0 < rb; m0 += D1_MT) {
-      const int mc = (int)(rb - m0 < D1_MT ? rb - m0 : D1_MT);
+  UnitWalk<D1_MT, 256> walk;
+  if (n_units > 0) walk.start(p, run_s.e, run_s.local);
+  for (long long unit = 0; unit < n_units; ++unit) {
+    if (unit > 0) walk.next(p);
+    const int e = walk.u.e;
+    const int64_t m0 = walk.u.m0;
+    const int nt = (walk.u.n0 >> 7) + (warp >> 3);  // warps 0-7: first tile of the pair, warps 8-15: second
+    const int mc = (int)(walk.u.rb - m0 < D1_MT ? walk.u.rb - m0 : D1_MT);
+    {
       if (staged_e != e || staged_m0 != m0) {
         __syncthreads();  // everyone is done with the previous rows (and the table is written)
         if (p.act_dtype == DST_ACT_BF16) d1_stage_tokens(p, static_cast<const __nv_bfloat16*>(p.x), m0, mc, xs, xsum, xexp, xex);
@@ -459,7 +463,9 @@ int launch_decode_tq1(const GemmArgs& a, cudaStream_t stream) {
   int dev = 0, sms = 148;
   DST_CUDA_TRY(cudaGetDevice(&dev));
   DST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const long long items = (long long)p.E * ((p.NT + 1) >> 1);
+  // units at most: every token row a pass of its own, or every expert with rows in them and full passes
+  const long long passes = p.T < p.E ? (long long)p.T : (long long)p.E + p.T / D1_MT;
+  const long long items = passes * ((p.NT + 1) >> 1);
   const size_t smem = d1_smem(p.S, p.G);
   int per_sm = (int)((220 * 1024) / (smem + 1024));
   per_sm = per_sm < 1 ? 1 : (per_sm > 2 ? 2 : per_sm);

@@ -18,10 +18,12 @@ namespace {
 // rows included: their weights are NaN, their ids 0..k-1).
 constexpr int ROUTE_MAX_PER_LANE = 32;  // E <= 1024
 
-// a ranks above b: NaN above everything, NaNs equal among themselves
-__device__ __forceinline__ bool route_above(float a, float b) {
-  const bool an = a != a, bn = b != b;
-  return an ? !bn : (!bn && a > b);
+// A key as an unsigned number of the same order: NaN above everything, NaNs and zeros of either sign equal among
+// themselves; 0 is below every key (no candidate).
+__device__ __forceinline__ uint32_t route_rank(float key) {
+  if (key != key) return 0xffffffffu;
+  const uint32_t u = __float_as_uint(key + 0.f);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
 // PL: experts per lane (E <= 32 PL); the loops over a lane's experts are unrolled to that count
@@ -61,128 +63,203 @@ __global__ void route_kernel(const float* __restrict__ logits, const float* __re
 #pragma unroll
     for (int j = 0; j < PL; ++j) v[j] = sqrtf(v[j] > 20.f ? v[j] : log1pf(expf(v[j])));
   }
-  uint32_t taken = 0;  // bit j: expert j * 32 + lane has been picked
-  float wsel[8];
-  int isel[8];
+  // Rounds of arg-max: the largest rank by one warp reduction, the lowest id that has it by another (15 shuffles and
+  // comparisons of (key, weight, id) took their place before: 16 384 tokens of 384 experts 71 us).
+  uint32_t rank[PL];
+#pragma unroll
+  for (int j = 0; j < PL; ++j) {
+    const int e = j * 32 + lane;
+    rank[j] = e < E ? route_rank(bias ? v[j] + bias[e] : v[j]) : 0u;
+  }
+  float my_w = 0.f;  // of pick `lane`
+  int my_id = 0;
   float wsum = 0.f;
   for (int r = 0; r < top_k; ++r) {
-    float best = 0.f, best_w = 0.f;
-    int bi = 0x7fffffff;  // no candidate in this lane yet
+    uint32_t best = 0u;
 #pragma unroll
-    for (int j = 0; j < PL; ++j) {
-      const int e = j * 32 + lane;
-      if (e < E && !((taken >> j) & 1u)) {
-        const float key = bias ? v[j] + bias[e] : v[j];
-        if (bi == 0x7fffffff || route_above(key, best)) {  // ascending e within a lane: the first maximum is the lowest id
-          best = key;
-          best_w = v[j];
-          bi = e;
-        }
+    for (int j = 0; j < PL; ++j) best = rank[j] > best ? rank[j] : best;
+    best = __reduce_max_sync(0xffffffffu, best);
+    uint32_t id = 0x7fffffffu;  // top_k <= E: some expert has the rank, unless all that are left are below every key
+#pragma unroll
+    for (int j = PL - 1; j >= 0; --j)
+      if (rank[j] == best && j * 32 + lane < E) id = (uint32_t)(j * 32 + lane);
+    id = __reduce_min_sync(0xffffffffu, id);
+    float w = 0.f;
+#pragma unroll
+    for (int j = 0; j < PL; ++j)
+      if ((uint32_t)(j * 32 + lane) == id) {
+        w = v[j];
+        rank[j] = 0u;  // picked
       }
+    w = __shfl_sync(0xffffffffu, w, (int)(id & 31u));
+    if (lane == r) {
+      my_w = w;
+      my_id = (int)id;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-      const float ow = __shfl_xor_sync(0xffffffffu, best_w, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-      const bool take = oi != 0x7fffffff && (bi == 0x7fffffff || route_above(ob, best) || (!route_above(best, ob) && oi < bi));
-      if (take) {
-        best = ob;
-        best_w = ow;
-        bi = oi;
-      }
-    }
-    // top_k <= E, so some lane always had a candidate: 0 <= bi < E
-    if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
-    wsel[r] = best_w;
-    isel[r] = bi;
-    wsum += best_w;
+    wsum += w;
   }
-  if (lane == 0) {
+  if (lane < top_k) {
     const float d = (renorm && top_k > 1) ? 1.f / (wsum + 1e-20f) : 1.f;
-    for (int r = 0; r < top_k; ++r) {
-      weights[t * top_k + r] = ((renorm && top_k > 1) ? wsel[r] * d : wsel[r]) * route_scale;
-      ids[t * top_k + r] = isel[r];
-    }
+    weights[t * top_k + lane] = ((renorm && top_k > 1) ? my_w * d : my_w) * route_scale;
+    ids[t * top_k + lane] = my_id;
   }
 }
 
 // ------------------------------------------------------------------------------------ routing sort
-// Stable counting sort in three steps over chunks of SORT_CHUNK consecutive ids, one warp per chunk:
-//   1. per-chunk histogram               hist[c][e]; also presets order[] to -1, so the tail that dropped ids leave
+// Stable counting sort of n ids, also giving the inverse order when asked for (inv[i] = position of id i, -1: dropped).
+// Up to SORT_SMALL ids: one block, everything in shared memory (the three steps below take ~14 us for six ids).
+// More, in three steps over chunks of SORT_CHUNK consecutive ids, four warps per chunk:
+//   1. per-chunk histogram               hist[c][e]; also presets order[] (and inv[]) to -1, so the tail that dropped ids leave
 //                                         unwritten is recognisable (every reader clamps or skips it) instead of
 //                                         holding whatever was in memory
 //   2. one block: offsets[e] and the start of every (chunk, expert) run, in place in hist
-//   3. per chunk, in input order: warp match on the expert id gives each entry its rank among equal
-//      ids of the same 32-entry step; a per-expert cursor in shared memory carries across steps.
-constexpr int SORT_CHUNK = 1024;
+//   3. per chunk, in input order: every warp counts its quarter, the quarters' counts become per-warp cursors in shared
+//      memory, and a warp match on the expert id gives each entry its rank among equal ids of the same 32-entry step.
+constexpr int SORT_CHUNK = 1024, SORT_WARPS = 4, SORT_SMALL = 1024;
+
+// Exclusive prefix sum of val[0 .. E) in shared memory, in place, by the whole block; val[E] = the total. E + 1 entries.
+__device__ __forceinline__ void block_exclusive_scan(int32_t* val, int E, int32_t* warp_sums /* 32 */) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = (blockDim.x + 31) >> 5;
+  const int per = (E + blockDim.x - 1) / blockDim.x, e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
+  int sum = 0;
+  for (int e = e0; e < e1; ++e) sum += val[e];
+  int incl = sum;
+  for (int d = 1; d < 32; d <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += up;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  int run = incl - sum, total = 0;
+  for (int w = 0; w < warps; ++w) {
+    if (w < warp) run += warp_sums[w];
+    total += warp_sums[w];
+  }
+  for (int e = e0; e < e1; ++e) {
+    const int v = val[e];
+    val[e] = run;
+    run += v;
+  }
+  if (tid == 0) val[E] = total;
+  __syncthreads();
+}
 
 template <typename IdT>
-__global__ void sort_hist_kernel(const IdT* __restrict__ ids, int64_t n, int E, int32_t* __restrict__ hist,
-                                 int32_t* __restrict__ bad_count, int64_t* __restrict__ order) {
+__global__ void __launch_bounds__(SORT_SMALL)
+sort_small_kernel(const IdT* __restrict__ ids, int n, int E, int64_t* __restrict__ order, int64_t* __restrict__ offsets,
+                  int32_t* __restrict__ bad_count, int64_t* __restrict__ inv) {
+  extern __shared__ int32_t count[];  // [E + 1]
+  __shared__ int32_t id_s[SORT_SMALL], sums[32];
+  const int tid = threadIdx.x;
+  for (int e = tid; e <= E; e += blockDim.x) count[e] = 0;
+  __syncthreads();
+  int id = -1;
+  if (tid < n) {
+    const int64_t e = (int64_t)ids[tid];
+    id = e >= 0 && e < E ? (int)e : -1;
+    id_s[tid] = id;
+    order[tid] = -1;  // rewritten below, after the barrier, where the sorted ids end
+    if (id >= 0) atomicAdd(&count[id], 1);
+  }
+  const int bad = __syncthreads_count(tid < n && id < 0);
+  if (bad_count && tid == 0) *bad_count = bad;
+  block_exclusive_scan(count, E, sums);
+  for (int e = tid; e <= E; e += blockDim.x) offsets[e] = count[e];
+  if (tid < n) {
+    int64_t pos = -1;
+    if (id >= 0) {
+      int rank = 0;  // equal ids before this one
+      for (int j = 0; j < tid; ++j) rank += id_s[j] == id;
+      pos = count[id] + rank;
+      order[pos] = tid;
+    }
+    if (inv) inv[tid] = pos;
+  }
+}
+
+template <typename IdT>
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+sort_hist_kernel(const IdT* __restrict__ ids, int64_t n, int E, int32_t* __restrict__ hist, int32_t* __restrict__ bad_count,
+                 int64_t* __restrict__ order, int64_t* __restrict__ inv) {
   extern __shared__ int32_t sh[];
-  for (int e = threadIdx.x; e < E; e += 32) sh[e] = 0;
-  __syncwarp();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) sh[e] = 0;
+  __syncthreads();
   const int64_t c = blockIdx.x, i0 = c * SORT_CHUNK;
   int bad = 0;
-  for (int s = 0; s < SORT_CHUNK; s += 32) {
-    const int64_t i = i0 + s + threadIdx.x;
+  for (int s = threadIdx.x; s < SORT_CHUNK; s += SORT_WARPS * 32) {
+    const int64_t i = i0 + s;
     if (i < n) {
       const int64_t e = (int64_t)ids[i];
       if (e >= 0 && e < E) atomicAdd(&sh[e], 1);
       else ++bad;
       order[i] = -1;
+      if (inv) inv[i] = -1;
     }
   }
-  __syncwarp();
-  for (int e = threadIdx.x; e < E; e += 32) hist[c * E + e] = sh[e];
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) hist[c * E + e] = sh[e];
   if (bad && bad_count) atomicAdd(bad_count, bad);
 }
 
 __global__ void sort_scan_kernel(int32_t* __restrict__ hist, int64_t chunks, int E, int64_t* __restrict__ offsets) {
-  // thread e: total of expert e; then an exclusive scan over experts; then run starts per chunk.
-  extern __shared__ int64_t tot[];
+  // thread e: total of expert e; an exclusive scan over the experts; then the run starts per chunk (total rows < 2^31)
+  extern __shared__ int32_t tot[];  // [E + 1]
+  __shared__ int32_t sums[32];
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int64_t s = 0;
+    int32_t s = 0;
     for (int64_t c = 0; c < chunks; ++c) s += hist[c * E + e];
     tot[e] = s;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t run = 0;
-    for (int e = 0; e < E; ++e) {
-      const int64_t v = tot[e];
-      tot[e] = run;
-      offsets[e] = run;
-      run += v;
-    }
-    offsets[E] = run;
-  }
-  __syncthreads();
+  block_exclusive_scan(tot, E, sums);
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = tot[e];
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int64_t run = tot[e];
+    int32_t run = tot[e];
     for (int64_t c = 0; c < chunks; ++c) {
       const int32_t v = hist[c * E + e];
-      hist[c * E + e] = (int32_t)run;  // total rows < 2^31
+      hist[c * E + e] = run;
       run += v;
     }
   }
 }
 
 template <typename IdT>
-__global__ void sort_place_kernel(const IdT* __restrict__ ids, int64_t n, int E, const int32_t* __restrict__ hist,
-                                  int64_t* __restrict__ order) {
-  extern __shared__ int32_t cur[];
-  const int lane = threadIdx.x;
-  const int64_t c = blockIdx.x, i0 = c * SORT_CHUNK;
-  for (int e = lane; e < E; e += 32) cur[e] = hist[c * E + e];
-  __syncwarp();
-  for (int s = 0; s < SORT_CHUNK; s += 32) {
-    const int64_t i = i0 + s + lane;
-    int64_t e = i < n ? (int64_t)ids[i] : -1;
-    const bool ok = e >= 0 && e < E;
-    const unsigned active = __ballot_sync(0xffffffffu, ok);
-    if (ok) {
-      const unsigned peers = __match_any_sync(active, (int)e);
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+sort_place_kernel(const IdT* __restrict__ ids, int64_t n, int E, const int32_t* __restrict__ hist, int64_t* __restrict__ order,
+                  int64_t* __restrict__ inv) {
+  extern __shared__ int32_t cur_all[];  // [SORT_WARPS][E]
+  constexpr int STEPS = SORT_CHUNK / SORT_WARPS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t c = blockIdx.x, i0 = c * SORT_CHUNK + warp * (STEPS * 32);
+  for (int e = threadIdx.x; e < SORT_WARPS * E; e += blockDim.x) cur_all[e] = 0;
+  __syncthreads();
+  int32_t* cur = cur_all + warp * E;
+  int id[STEPS];
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+    const int64_t i = i0 + s * 32 + lane;
+    const int64_t e = i < n ? (int64_t)ids[i] : -1;
+    id[s] = e >= 0 && e < E ? (int)e : -1;
+    if (id[s] >= 0) atomicAdd(&cur[id[s]], 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int32_t run = hist[c * E + e];
+#pragma unroll
+    for (int w = 0; w < SORT_WARPS; ++w) {
+      const int32_t v = cur_all[w * E + e];
+      cur_all[w * E + e] = run;
+      run += v;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+    const int64_t i = i0 + s * 32 + lane;
+    const int e = id[s];
+    const unsigned active = __ballot_sync(0xffffffffu, e >= 0);
+    if (e >= 0) {
+      const unsigned peers = __match_any_sync(active, e);
       const int rank = __popc(peers & ((1u << lane) - 1u));
       const int leader = __ffs(peers) - 1;
       int base = 0;
@@ -192,16 +269,13 @@ __global__ void sort_place_kernel(const IdT* __restrict__ ids, int64_t n, int E,
       }
       base = __shfl_sync(peers, base, leader);
       order[base + rank] = i;
+      if (inv) inv[i] = base + rank;
     }
     __syncwarp();
   }
 }
 
 // ------------------------------------------------------------------------------------------ gather
-// Every kernel that follows `order` clamps the entry to [0, n): an order array that was not produced by the routing
-// sort (or one whose tail belongs to dropped ids) can then make a row wrong, but cannot make an access leave the buffers.
-__device__ __forceinline__ int64_t clamp_slot(int64_t f, int64_t n) { return f < 0 ? 0 : (f >= n ? n - 1 : f); }
-
 // dst[p, :] = src[order[p] / top_k, :], 16-byte vectors where the row length allows.
 __global__ void gather_rows_kernel(const uint16_t* __restrict__ src, const int64_t* __restrict__ order, int64_t n_rows,
                                    int64_t K, int top_k, uint16_t* __restrict__ dst) {
@@ -220,11 +294,6 @@ __global__ void gather_rows_kernel(const uint16_t* __restrict__ src, const int64
 }
 
 // ------------------------------------------------------------------------------------------ swiglu
-__device__ __forceinline__ float silu_fast(float g) {
-  // g * sigmoid(g) with the hardware's exp2 and reciprocal approximations (2 ulp each; the result is rounded to bf16)
-  return __fdividef(g, 1.f + __expf(-g));
-}
-
 // gu[p, 0:I] = gate (bf16), gu[p, I:2I] = up (bf16); h = bf16(w * silu(gate) * up), fp32 in between.
 __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, const float* __restrict__ route_weights,
                               const int64_t* __restrict__ order, int64_t n_rows, int64_t inter, float limit,
@@ -560,32 +629,25 @@ __global__ void invert_order_kernel(const int64_t* __restrict__ order, int64_t n
   }
 }
 
-// A token's positions in `down` in increasing expert id (the ids of one token are distinct) -> pos[0 .. top_k) in
-// shared memory; positions that are negative (dropped ids) or beyond the n_pos rows of `down` are marked -1. One
-// thread sorts (its arrays are indexed at run time, so they live in local memory: one thread's worth, not a block's).
+// A token's positions in `down` in increasing expert id (equal ids, which only dropped slots have: in slot order) ->
+// pos[0 .. top_k) in shared memory; positions that are negative (dropped ids) or beyond the n_pos rows of `down` are marked
+// -1. One lane per slot, ranked by counting. w_shared (optional): the slots' routing weights rounded to bf16, same order.
 __device__ __forceinline__ void token_slots(const int64_t* __restrict__ inv, const int32_t* __restrict__ ids, int64_t t, int top_k,
-                                            int64_t n_pos, int64_t* pos_shared) {
-  if (threadIdx.x == 0) {
-    int64_t pos[8];
-    int eid[8];
-    for (int s = 0; s < top_k; ++s) {
-      const int64_t q = inv[t * top_k + s];
-      pos[s] = (q >= 0 && q < n_pos) ? q : -1;
-      eid[s] = ids[t * top_k + s];
+                                            int64_t n_pos, int64_t* pos_shared, const float* __restrict__ weights = nullptr,
+                                            float* w_shared = nullptr) {
+  if (threadIdx.x < 32) {
+    const int s = threadIdx.x < top_k ? threadIdx.x : 0;
+    const int64_t q = inv[t * top_k + s];
+    const int e = ids[t * top_k + s];
+    int rank = 0;
+    for (int j = 0; j < top_k; ++j) {
+      const int o = __shfl_sync(0xffffffffu, e, j);
+      rank += o < e || (o == e && j < s);
     }
-    for (int i = 1; i < top_k; ++i) {  // insertion sort by expert id
-      const int e = eid[i];
-      const int64_t q = pos[i];
-      int j = i - 1;
-      while (j >= 0 && eid[j] > e) {
-        eid[j + 1] = eid[j];
-        pos[j + 1] = pos[j];
-        --j;
-      }
-      eid[j + 1] = e;
-      pos[j + 1] = q;
+    if (threadIdx.x < top_k) {
+      pos_shared[rank] = (q >= 0 && q < n_pos) ? q : -1;
+      if (w_shared) w_shared[rank] = __bfloat162float(__float2bfloat16_rn(weights[t * top_k + s]));
     }
-    for (int s = 0; s < top_k; ++s) pos_shared[s] = pos[s];
   }
   __syncthreads();
 }
@@ -685,45 +747,93 @@ __global__ void swiglu_std_kernel(const __nv_bfloat16* __restrict__ gu, int64_t 
   if (threadIdx.x == 0) factor[p] = ldexpf(1.f, ex);
 }
 
+// The normalised form for inter % 8 == 0, inter <= 256 J: a warp per row, its chunks in registers (as swiglu_norm_warp_kernel;
+// 6216 rows of 1024: 26 us with a block per row, the values computed twice).
+template <int J>
+__global__ void __launch_bounds__(256)
+swiglu_std_norm_warp_kernel(const __nv_bfloat16* __restrict__ gu, int64_t n_rows, int64_t inter, __half* __restrict__ h, float* __restrict__ factor) {
+  const int lane = threadIdx.x & 31, chunks = (int)(inter >> 3);
+  for (int64_t p = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); p < n_rows; p += (int64_t)gridDim.x * 8) {
+    const uint4* g = reinterpret_cast<const uint4*>(gu + p * 2 * inter);
+    const uint4* u = reinterpret_cast<const uint4*>(gu + p * 2 * inter + inter);
+    uint4 rg[J], ru[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int c = lane + j * 32;
+      rg[j] = c < chunks ? g[c] : make_uint4(0u, 0u, 0u, 0u);
+      ru[j] = c < chunks ? u[c] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint4 hv[J];
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      float gate[8], up[8], x[8];
+      bf16x8_to_float(rg[j], gate);
+      bf16x8_to_float(ru[j], up);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = __bfloat162float(__float2bfloat16_rn(silu_fast(gate[i]))) * up[i];
+      hv[j] = float8_to_bf16(x);
+      bf16x8_to_float(hv[j], x);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(x[i]));
+    }
+    const int ex = norm_exponent(warp_max(amax));
+    const float down = ldexpf(1.f, -ex);
+    uint4* d = reinterpret_cast<uint4*>(h + p * inter);
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int c = lane + j * 32;
+      if (c < chunks) {
+        float x[8];
+        bf16x8_to_float(hv[j], x);
+        d[c] = float8_to_f16(x, down);
+      }
+    }
+    if (lane == 0) factor[p] = ldexpf(1.f, ex);
+  }
+}
+
 // One block per token: y = sum over its slots in increasing expert id of bf16(down * bf16(weight)), every partial
-// sum rounded to bf16 (the reference accumulates with index_add_ into a bf16 tensor).
-__global__ void combine_weighted_kernel(const __nv_bfloat16* __restrict__ down, const int64_t* __restrict__ inv,
-                                        const int32_t* __restrict__ ids, const float* __restrict__ weights, int top_k, int64_t hidden,
-                                        __nv_bfloat16* __restrict__ y) {
+// sum rounded to bf16 (the reference accumulates with index_add_ into a bf16 tensor). VEC: hidden % 8 == 0, 128-bit loads of
+// all the token's rows before any is added (777 tokens of 2048 x 8: 37 us element by element).
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+combine_weighted_kernel(const __nv_bfloat16* __restrict__ down, const int64_t* __restrict__ inv, const int32_t* __restrict__ ids,
+                        const float* __restrict__ weights, int top_k, int64_t hidden, __nv_bfloat16* __restrict__ y) {
   const int64_t t = blockIdx.x;
-  int64_t pos[8];
-  int eid[8];
-  float wv[8];
-  const int64_t n_pos = (int64_t)gridDim.x * top_k;
-  for (int s = 0; s < top_k; ++s) {
-    const int64_t q = inv[t * top_k + s];
-    pos[s] = (q >= 0 && q < n_pos) ? q : -1;  // -1: the slot's expert id was dropped by the routing sort
-    eid[s] = ids[t * top_k + s];
-    wv[s] = __bfloat162float(__float2bfloat16_rn(weights[t * top_k + s]));
-  }
-  for (int i = 1; i < top_k; ++i) {  // insertion sort by expert id (ids of one token are distinct)
-    const int e = eid[i];
-    const int64_t p = pos[i];
-    const float w = wv[i];
-    int j = i - 1;
-    while (j >= 0 && eid[j] > e) {
-      eid[j + 1] = eid[j];
-      pos[j + 1] = pos[j];
-      wv[j + 1] = wv[j];
-      --j;
+  __shared__ int64_t pos[8];
+  __shared__ float wv[8];
+  token_slots(inv, ids, t, top_k, (int64_t)gridDim.x * top_k, pos, weights, wv);
+  auto add = [&](float acc, float d, float w) {
+    const float r = __bfloat162float(__float2bfloat16_rn(d * w));
+    return __bfloat162float(__float2bfloat16_rn(acc + r));
+  };
+  if constexpr (VEC) {
+    const int chunks = (int)(hidden >> 3);
+    for (int c = threadIdx.x; c < chunks; c += 256) {
+      uint4 raw[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s < top_k && pos[s] >= 0) raw[s] = reinterpret_cast<const uint4*>(down + pos[s] * hidden)[c];
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        if (s < top_k && pos[s] >= 0) {
+          float f[8];
+          bf16x8_to_float(raw[s], f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i] = add(acc[i], f[i], wv[s]);
+        }
+      }
+      reinterpret_cast<uint4*>(y + t * hidden)[c] = float8_to_bf16(acc);
     }
-    eid[j + 1] = e;
-    pos[j + 1] = p;
-    wv[j + 1] = w;
-  }
-  for (int64_t c = threadIdx.x; c < hidden; c += blockDim.x) {
+  } else {
+  for (int64_t c = threadIdx.x; c < hidden; c += 256) {
     float acc = 0.f;
-    for (int s = 0; s < top_k; ++s) {
-      if (pos[s] < 0) continue;
-      const float r = __bfloat162float(__float2bfloat16_rn(__bfloat162float(down[pos[s] * hidden + c]) * wv[s]));
-      acc = __bfloat162float(__float2bfloat16_rn(acc + r));
-    }
+    for (int s = 0; s < top_k; ++s)
+      if (pos[s] >= 0) acc = add(acc, __bfloat162float(down[pos[s] * hidden + c]), wv[s]);
     y[t * hidden + c] = __float2bfloat16_rn(acc);
+  }
   }
 }
 
@@ -768,33 +878,48 @@ extern "C" size_t dst_sort_workspace_bytes(int64_t n, int64_t E) {
   return (size_t)(chunks * E) * sizeof(int32_t);
 }
 
-extern "C" int dst_sort_by_expert(const void* ids, int ids_are_i32, int64_t n, int64_t E, int64_t* order,
-                                  int64_t* offsets, int32_t* bad_count, void* workspace, dst_stream_t stream) {
+int dst::sort_rows(const void* ids, int ids_are_i32, int64_t n, int64_t E, int64_t* order, int64_t* offsets, int32_t* bad_count,
+                   void* workspace, int64_t* inv, cudaStream_t st) {
   if (n < 0 || E <= 0 || !offsets) return DST_ERR_BAD_ARG;
   if (E > 4096 || n > 0x7fffffff) return DST_ERR_BAD_SHAPE;  // per-expert tables live in shared memory
-  auto st = static_cast<cudaStream_t>(stream);
-  if (bad_count) DST_CUDA_TRY(cudaMemsetAsync(bad_count, 0, sizeof(int32_t), st));
   if (n == 0) {
+    if (bad_count) DST_CUDA_TRY(cudaMemsetAsync(bad_count, 0, sizeof(int32_t), st));
     DST_CUDA_TRY(cudaMemsetAsync(offsets, 0, (size_t)(E + 1) * sizeof(int64_t), st));
     return DST_OK;
   }
   if (!ids || !order || !workspace) return DST_ERR_BAD_ARG;
-  const int64_t chunks = cdiv64(n, SORT_CHUNK);
+  const size_t sh32 = (size_t)(E + 1) * sizeof(int32_t);
+  auto i32 = static_cast<const int32_t*>(ids);
+  auto i64 = static_cast<const int64_t*>(ids);
+  if (n <= SORT_SMALL) {
+    const unsigned threads = (unsigned)(cdiv64(n, 32) * 32 < 256 ? 256 : cdiv64(n, 32) * 32);  // at least eight warps for the scan over the experts
+    if (ids_are_i32) sort_small_kernel<int32_t><<<1, threads, sh32, st>>>(i32, (int)n, (int)E, order, offsets, bad_count, inv);
+    else sort_small_kernel<int64_t><<<1, threads, sh32, st>>>(i64, (int)n, (int)E, order, offsets, bad_count, inv);
+    DST_CUDA_TRY(cudaGetLastError());
+    return DST_OK;
+  }
+  if (bad_count) DST_CUDA_TRY(cudaMemsetAsync(bad_count, 0, sizeof(int32_t), st));
+  const unsigned chunks = (unsigned)cdiv64(n, SORT_CHUNK);
   int32_t* hist = static_cast<int32_t*>(workspace);
-  const size_t sh32 = (size_t)E * sizeof(int32_t);
-  if (ids_are_i32)
-    sort_hist_kernel<int32_t><<<(unsigned)chunks, 32, sh32, st>>>(static_cast<const int32_t*>(ids), n, (int)E, hist, bad_count, order);
-  else
-    sort_hist_kernel<int64_t><<<(unsigned)chunks, 32, sh32, st>>>(static_cast<const int64_t*>(ids), n, (int)E, hist, bad_count, order);
+  if (ids_are_i32) sort_hist_kernel<int32_t><<<chunks, SORT_WARPS * 32, sh32, st>>>(i32, n, (int)E, hist, bad_count, order, inv);
+  else sort_hist_kernel<int64_t><<<chunks, SORT_WARPS * 32, sh32, st>>>(i64, n, (int)E, hist, bad_count, order, inv);
   DST_CUDA_TRY(cudaGetLastError());
-  sort_scan_kernel<<<1, 512, (size_t)E * sizeof(int64_t), st>>>(hist, chunks, (int)E, offsets);
+  sort_scan_kernel<<<1, 512, sh32, st>>>(hist, chunks, (int)E, offsets);
   DST_CUDA_TRY(cudaGetLastError());
-  if (ids_are_i32)
-    sort_place_kernel<int32_t><<<(unsigned)chunks, 32, sh32, st>>>(static_cast<const int32_t*>(ids), n, (int)E, hist, order);
-  else
-    sort_place_kernel<int64_t><<<(unsigned)chunks, 32, sh32, st>>>(static_cast<const int64_t*>(ids), n, (int)E, hist, order);
+  const size_t place = (size_t)SORT_WARPS * (size_t)E * sizeof(int32_t);  // above 48 KB for more than 3072 experts
+  if (place > 48 * 1024) {
+    DST_CUDA_TRY(cudaFuncSetAttribute(sort_place_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)place));
+    DST_CUDA_TRY(cudaFuncSetAttribute(sort_place_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)place));
+  }
+  if (ids_are_i32) sort_place_kernel<int32_t><<<chunks, SORT_WARPS * 32, place, st>>>(i32, n, (int)E, hist, order, inv);
+  else sort_place_kernel<int64_t><<<chunks, SORT_WARPS * 32, place, st>>>(i64, n, (int)E, hist, order, inv);
   DST_CUDA_TRY(cudaGetLastError());
   return DST_OK;
+}
+
+extern "C" int dst_sort_by_expert(const void* ids, int ids_are_i32, int64_t n, int64_t E, int64_t* order,
+                                  int64_t* offsets, int32_t* bad_count, void* workspace, dst_stream_t stream) {
+  return dst::sort_rows(ids, ids_are_i32, n, E, order, offsets, bad_count, workspace, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int dst_gather_rows(const void* src, const int64_t* order, int64_t n_rows, int64_t K, int top_k,
@@ -895,6 +1020,29 @@ extern "C" int dst_swiglu_norm_dev(const void* gu_bf16, const float* route_weigh
                             static_cast<cudaStream_t>(stream));
 }
 
+// The combine of both flavours from the inverse order (weights null: V4 with the optional `add`; else the standard one)
+int dst::combine_rows(const void* down_bf16, const int64_t* inv, const int32_t* ids, const float* weights, int64_t T, int top_k,
+                      int64_t hidden, const void* add_bf16, void* y_bf16, cudaStream_t st) {
+  auto down = static_cast<const __nv_bfloat16*>(down_bf16);
+  auto add = static_cast<const __nv_bfloat16*>(add_bf16);
+  auto y = static_cast<__nv_bfloat16*>(y_bf16);
+  const bool vec = hidden % 8 == 0 && (reinterpret_cast<uintptr_t>(down) & 15) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(add) & 15) == 0;
+  if (weights && vec) combine_weighted_kernel<true><<<(unsigned)T, 256, 0, st>>>(down, inv, ids, weights, top_k, hidden, y);
+  else if (weights) combine_weighted_kernel<false><<<(unsigned)T, 256, 0, st>>>(down, inv, ids, weights, top_k, hidden, y);
+  else if (vec) combine_vec_kernel<<<(unsigned)T, 256, 0, st>>>(down, inv, ids, top_k, hidden, add, y);
+  else combine_kernel<<<(unsigned)T, 256, 0, st>>>(down, inv, ids, top_k, hidden, add, y);
+  DST_CUDA_TRY(cudaGetLastError());
+  return DST_OK;
+}
+
+static int invert_rows(const int64_t* order, int64_t n, int64_t* inv, cudaStream_t st) {
+  DST_CUDA_TRY(cudaMemsetAsync(inv, 0xff, (size_t)n * sizeof(int64_t), st));  // -1: no row (see invert_order_kernel)
+  invert_order_kernel<<<(unsigned)cdiv64(n, 256), 256, 0, st>>>(order, n, inv);
+  DST_CUDA_TRY(cudaGetLastError());
+  return DST_OK;
+}
+
 extern "C" int dst_combine_add(const void* down_bf16, const int64_t* order, const int32_t* ids, int64_t T, int top_k,
                                int64_t hidden, int64_t* inv, const void* add_bf16, void* y_bf16, dst_stream_t stream) {
   if (T < 0 || top_k <= 0 || top_k > 8 || hidden <= 0) return DST_ERR_BAD_ARG;
@@ -902,20 +1050,8 @@ extern "C" int dst_combine_add(const void* down_bf16, const int64_t* order, cons
   if (!down_bf16 || !order || !ids || !inv || !y_bf16) return DST_ERR_BAD_ARG;
   if (T > 0x7fffffff / top_k) return DST_ERR_BAD_SHAPE;
   auto st = static_cast<cudaStream_t>(stream);
-  const int64_t n = T * top_k;
-  DST_CUDA_TRY(cudaMemsetAsync(inv, 0xff, (size_t)n * sizeof(int64_t), st));  // -1: no row (see invert_order_kernel)
-  invert_order_kernel<<<(unsigned)cdiv64(n, 256), 256, 0, st>>>(order, n, inv);
-  DST_CUDA_TRY(cudaGetLastError());
-  auto add = static_cast<const __nv_bfloat16*>(add_bf16);
-  if (hidden % 8 == 0 && (reinterpret_cast<uintptr_t>(down_bf16) & 15) == 0 && (reinterpret_cast<uintptr_t>(y_bf16) & 15) == 0 &&
-      (reinterpret_cast<uintptr_t>(add_bf16) & 15) == 0)
-    combine_vec_kernel<<<(unsigned)T, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(down_bf16), inv, ids, top_k, hidden, add,
-                                                   static_cast<__nv_bfloat16*>(y_bf16));
-  else
-    combine_kernel<<<(unsigned)T, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(down_bf16), inv, ids, top_k, hidden, add,
-                                               static_cast<__nv_bfloat16*>(y_bf16));
-  DST_CUDA_TRY(cudaGetLastError());
-  return DST_OK;
+  const int rc = invert_rows(order, T * top_k, inv, st);
+  return rc != DST_OK ? rc : dst::combine_rows(down_bf16, inv, ids, nullptr, T, top_k, hidden, add_bf16, y_bf16, st);
 }
 
 extern "C" int dst_ep_combine_returned(const void* rows_bf16, const int64_t* order, const int64_t* row_dest, const int32_t* ids, int64_t T,
@@ -961,6 +1097,16 @@ extern "C" int dst_swiglu_std_norm(const void* gu_bf16, int64_t n_rows, int64_t 
   if (n_rows == 0) return DST_OK;
   if (!gu_bf16 || !h_f16 || !row_factor) return DST_ERR_BAD_ARG;
   if (n_rows > 0x7fffffff) return DST_ERR_BAD_SHAPE;
+  if (inter % 8 == 0 && inter <= 2048 && (reinterpret_cast<uintptr_t>(gu_bf16) & 15) == 0 && (reinterpret_cast<uintptr_t>(h_f16) & 15) == 0) {
+    auto g = static_cast<const __nv_bfloat16*>(gu_bf16);
+    auto d = static_cast<__half*>(h_f16);
+    auto st = static_cast<cudaStream_t>(stream);
+    const unsigned grid = (unsigned)std::min<int64_t>((n_rows + 7) / 8, 148 * 64);
+    if (inter <= 1024) swiglu_std_norm_warp_kernel<4><<<grid, 256, 0, st>>>(g, n_rows, inter, d, row_factor);
+    else swiglu_std_norm_warp_kernel<8><<<grid, 256, 0, st>>>(g, n_rows, inter, d, row_factor);
+    DST_CUDA_TRY(cudaGetLastError());
+    return DST_OK;
+  }
   swiglu_std_kernel<true><<<(unsigned)n_rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(gu_bf16), inter, nullptr, static_cast<__half*>(h_f16), row_factor);
   DST_CUDA_TRY(cudaGetLastError());
@@ -974,12 +1120,6 @@ extern "C" int dst_combine_weighted(const void* down_bf16, const int64_t* order,
   if (!down_bf16 || !order || !ids || !weights || !inv || !y_bf16) return DST_ERR_BAD_ARG;
   if (T > 0x7fffffff / top_k) return DST_ERR_BAD_SHAPE;
   auto st = static_cast<cudaStream_t>(stream);
-  const int64_t n = T * top_k;
-  DST_CUDA_TRY(cudaMemsetAsync(inv, 0xff, (size_t)n * sizeof(int64_t), st));  // -1: no row
-  invert_order_kernel<<<(unsigned)cdiv64(n, 256), 256, 0, st>>>(order, n, inv);
-  DST_CUDA_TRY(cudaGetLastError());
-  combine_weighted_kernel<<<(unsigned)T, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(down_bf16), inv, ids, weights, top_k, hidden,
-                                                      static_cast<__nv_bfloat16*>(y_bf16));
-  DST_CUDA_TRY(cudaGetLastError());
-  return DST_OK;
+  const int rc = invert_rows(order, T * top_k, inv, st);
+  return rc != DST_OK ? rc : dst::combine_rows(down_bf16, inv, ids, weights, T, top_k, hidden, nullptr, y_bf16, st);
 }

@@ -158,12 +158,17 @@ int dst_ternary_grouped_gemm(void* out, int out_dtype, int accumulate, const voi
 /* Scratch bytes dst_ternary_grouped_gemm needs for `algo` (AUTO: the largest any kernel may need). */
 size_t dst_gemm_workspace_bytes(int algo, int act_dtype, int64_t T, int64_t K);
 
-/* Token rows per expert up to which DST_ALGO_AUTO sends tiled weights of `fmt` (E experts of N rows) to the
- * decode GEMV rather than the tcgen05 kernel: 16, or 32 where the decode GEMV's many-row form applies. A caller
+/* Token rows per expert up to which the decode GEMV can be the faster kernel for tiled weights of `fmt` (E experts of N
+ * rows): 16, or 32 where its many-row form applies. A caller
  * that keeps a second, decode-friendly copy of its weights (the Python layer's 2-bit copy of TQ1 trits) picks
  * the copy by the same rule. No reference counterpart: the reference has one kernel for every row count
  * (boilerplate/kernels/csrc/ternary_cuda_kernel.cu:44-99). */
 int64_t dst_decode_row_limit(int fmt, int64_t E, int64_t N);
+
+/* Token rows per expert up to which DST_ALGO_AUTO takes the decode GEMV for T rows in all over E experts of N rows and
+ * n_terms stacked terms: the limit above, except for single-term TQ1 tiles (8 when T rows leave every CTA at most one
+ * work unit and E > 1, else 0). No reference counterpart. */
+int64_t dst_decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N);
 
 /*
  * Routing sort: flattened expert ids [n] (int64 or int32) -> the stable order that sorts them by
@@ -241,6 +246,30 @@ int dst_swiglu_norm_dev(const void* gu_bf16, const float* route_weights, const i
  */
 int dst_combine(const void* down_bf16, const int64_t* order, const int32_t* ids, int64_t T, int top_k,
                 int64_t hidden, int64_t* inv, void* y_bf16, dst_stream_t stream);
+/* A whole routed-expert layer on one device from one call (boilerplate/engine/model.py:407-422 from the routing weights
+ * on; engine/standard.py:154-176 with standard != 0): the routing sort, the gather, both expert GEMMs with SwiGLU between
+ * them, the shared expert (V4, one expert, may be null) and the combine, on one stream. The kernels and their choice are
+ * those of the single entry points with DST_ALGO_AUTO. Tiled weights, group 128, fp16 scales, hidden and inter multiples
+ * of 128; anything else is DST_ERR_UNSUPPORTED (dst_moe_layer_workspace_bytes then returns 0).
+ *   x [T, hidden] bf16, weights [T, top_k] f32, ids [T, top_k] int32 (an id outside [0, experts) drops that slot)
+ *   w13, s13     per term: [experts, 2 inter, ...] tiled weights and scales; w2, s2 [experts, hidden, ...]
+ *   w13_decode, w2_decode   optional: the trits of TQ1 weights once more as tiled TQ2 (all terms or none)
+ *   workspace    256-byte aligned, dst_moe_layer_workspace_bytes bytes */
+typedef struct dst_expert_weights {
+  const void* w13[DST_MAX_TERMS];
+  const void* s13[DST_MAX_TERMS];
+  const void* w2[DST_MAX_TERMS];
+  const void* s2[DST_MAX_TERMS];
+  const void* w13_decode[DST_MAX_TERMS];
+  const void* w2_decode[DST_MAX_TERMS];
+  int64_t experts, hidden, inter;
+  int n_terms, fmt;
+} dst_expert_weights;
+size_t dst_moe_layer_workspace_bytes(int64_t T, int top_k, int standard, const dst_expert_weights* w, const dst_expert_weights* shared);
+int dst_moe_layer(const void* x_bf16, const float* weights, const int32_t* ids, int64_t T, int top_k, int standard, float limit,
+                  const dst_expert_weights* w, const dst_expert_weights* shared, void* y_bf16, void* workspace, size_t workspace_bytes,
+                  dst_stream_t stream);
+
 /* The same with one more bf16 row per token added in fp32 after the experts' rows and before the cast: the shared
  * expert's output, `y += self.swiglu(L.shared, x)` of boilerplate/engine/model.py:421. add_bf16 [T, hidden] or NULL.
  * A (token, slot) whose expert id the routing sort dropped (outside [0, E)) contributes nothing. */
