@@ -20,6 +20,7 @@ does (``ternary_cuda.py:76-77``).
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from functools import lru_cache
@@ -87,7 +88,7 @@ class TiledWeights:
     def untile(self) -> torch.Tensor:
         lib = _require("auto")
         out = torch.empty(self.E, self.N, packed_cols(self.fmt, self.K), dtype=torch.uint8, device=self.data.device)
-        with torch.cuda.device(self.data.device):
+        with _guard(self.data.device):
             _lib.check(lib.dst_untile_weights(self.data.data_ptr(), self.E, self.N, self.K, _fmt_code(self.fmt), out.data_ptr(),
                                               _stream(self.data)))
         return out
@@ -124,7 +125,7 @@ def tile_weights(packed: torch.Tensor, fmt: str, K: int, decode_copy: bool = Fal
     E, N, _ = packed.shape
     nbytes = lib.dst_tiled_bytes(code, E, N, K)
     data = torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=packed.device)
-    with torch.cuda.device(packed.device):
+    with _guard(packed.device):
         _lib.check(lib.dst_tile_weights(packed.data_ptr(), E, N, K, code, data.data_ptr(), _stream(packed)))
     dec = None
     if decode_copy and fmt == "tq1" and K % 512 == 0:
@@ -140,7 +141,7 @@ def _reencode_tq2_tiled(lib, packed_tq1: torch.Tensor, K: int) -> torch.Tensor:
     out = torch.empty(max(int(lib.dst_tiled_bytes(_lib.FMT_TQ2, E, N, K)), 16), dtype=torch.uint8, device=dev)
     per_expert = int(lib.dst_tiled_bytes(_lib.FMT_TQ2, 1, N, K))
     step = max(1, (256 << 20) // max(N * K, 1))
-    with torch.cuda.device(dev):
+    with _guard(dev):
         st = _stream(packed_tq1)
         for e0 in range(0, E, step):
             n = min(step, E - e0)
@@ -157,8 +158,16 @@ def fast_path_covers(K: int, group: int, scale_dtype, act_dtype=torch.bfloat16) 
     return group == 128 and K % 128 == 0 and scale_dtype == torch.float16 and act_dtype in (torch.bfloat16, torch.float16, torch.int8)
 
 
-def _stream(t: torch.Tensor):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+def _stream(t: torch.Tensor) -> int:
+    return torch._C._cuda_getCurrentRawStream(t.device.index)  # torch.cuda.current_stream() builds an object per call (~2 us)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def _guard(device: torch.device):
+    """``torch.cuda.device(device)``, or nothing where that device is the current one already (~3 us per call)."""
+    return _NO_GUARD if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _check_dev(ts: Sequence[torch.Tensor]):
@@ -170,19 +179,25 @@ def _check_dev(ts: Sequence[torch.Tensor]):
             raise RuntimeError("ternary GEMM tensors must share one device")
 
 
-def _offsets(offsets, E: int, T: int, device, validate: bool):
+def _offsets(offsets, E: int, T: int, device, validate: bool, checked=None):
     """(device int64 tensor, host ctypes array or None). Host validation as ``ternary_cuda.py:94-97``."""
     if isinstance(offsets, torch.Tensor) and offsets.is_cuda and not validate:
         if offsets.dtype != torch.int64 or offsets.numel() != E + 1:
             raise ValueError("offsets must be nondecreasing, start at 0, end at the row count, one per expert + 1")
         return offsets.contiguous(), None
-    offs = torch.as_tensor(offsets, dtype=torch.int64).cpu().contiguous()
-    if offs.dim() != 1 or offs.numel() != E + 1 or int(offs[0]) != 0 or int(offs[-1]) != T or bool((offs.diff() < 0).any()):
-        raise ValueError("offsets must be nondecreasing, start at 0, end at the row count, one per expert + 1")
-    host = (ctypes.c_int64 * (E + 1))(*offs.tolist())
+    offs, host = checked if checked is not None else _host_offsets(offsets, E, T)
     dev = offsets.contiguous() if isinstance(offsets, torch.Tensor) and offsets.is_cuda and offsets.dtype == torch.int64 \
         else offs.to(device)
     return dev, host
+
+
+def _host_offsets(offsets, E: int, T: int):
+    """(int64 CPU tensor, ctypes array) of offsets that are in order, else ValueError (``ternary_cuda.py:94-97``)."""
+    offs = torch.as_tensor(offsets, dtype=torch.int64).cpu().contiguous()
+    values = offs.tolist() if offs.dim() == 1 and offs.numel() == E + 1 else [1]
+    if values[0] != 0 or values[-1] != T or any(b < a for a, b in zip(values, values[1:])):
+        raise ValueError("offsets must be nondecreasing, start at 0, end at the row count, one per expert + 1")
+    return offs, (ctypes.c_int64 * (E + 1))(*values)
 
 
 def _decode_row_limit(E: int, N: int) -> int:
@@ -192,7 +207,7 @@ def _decode_row_limit(E: int, N: int) -> int:
 
 
 def _grouped(lib, x, row_scale, offsets, packed_terms, scale_terms, K, group, fmt, out, accumulate, algo,
-             validate_offsets=True, act_code=None):
+             validate_offsets=True, act_code=None, checked=None):
     """Shared launcher. packed_terms[i] [E, N, Kp] uint8, scale_terms[i] [E, N, G]."""
     code = _fmt_code(fmt)
     n_terms = len(packed_terms)
@@ -242,21 +257,19 @@ def _grouped(lib, x, row_scale, offsets, packed_terms, scale_terms, K, group, fm
     if E == 1 and offsets is None:
         offs_dev, offs_host = None, None
     else:
-        offs_dev, offs_host = _offsets(offsets, E, T, x.device, validate_offsets)
+        offs_dev, offs_host = _offsets(offsets, E, T, x.device, validate_offsets, checked)
     pk = (ctypes.c_void_p * n_terms)(*[p.data_ptr() for p in raw])
     sc = (ctypes.c_void_p * n_terms)(*[s.data_ptr() for s in scale_terms])
     act = _ACT[x.dtype] if act_code is None else act_code
     ws_bytes = int(lib.dst_gemm_workspace_bytes(_ALGO[algo], act, T, K)) if tiled and act != _lib.ACT_F16_NORM else 0
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
-    with torch.cuda.device(x.device):
+    with _guard(x.device):
         rc = lib.dst_ternary_grouped_gemm(
             out.data_ptr(), _OUT[out.dtype], int(bool(accumulate)), x.data_ptr(), act,
             row_scale.data_ptr() if row_scale is not None else None,
             offs_dev.data_ptr() if offs_dev is not None else None, offs_host,
             pk, _lib.LAYOUT_TILED if tiled else _lib.LAYOUT_CANONICAL, sc, n_terms, _SCALE[sdt], E, T, N, K, group, code,
             _ALGO[algo], ws.data_ptr() if ws is not None else None, ws_bytes, _stream(x))
-    if ws is not None:
-        ws.record_stream(torch.cuda.current_stream(x.device))
     _lib.check(rc)
     return out
 
@@ -279,8 +292,9 @@ def grouped_ternary_gemm(x: torch.Tensor, x_scale: torch.Tensor, offsets, packed
     (reference ``ternary_cuda.py:90-111``)."""
     _fmt_code(fmt)
     E = packed.size(0)
+    checked = None
     if offsets is not None and not (isinstance(offsets, torch.Tensor) and offsets.is_cuda):
-        _offsets(offsets, E, x.size(0), "cpu", True)  # host offsets are validated before anything else, as the reference does
+        checked = _host_offsets(offsets, E, x.size(0))  # host offsets are validated before anything else, as the reference does
     lib = _require(backend)
     if not x.is_cuda:
         raise RuntimeError(_UNAVAILABLE + ": activations are not on a CUDA device and this backend has no CPU path")
@@ -290,7 +304,7 @@ def grouped_ternary_gemm(x: torch.Tensor, x_scale: torch.Tensor, offsets, packed
     # fp32 accumulation); anything else to the generic kernel with the reference's integer group sums
     fast = isinstance(packed, TiledWeights) or fast_path_covers(K, group, ws.dtype, x.dtype)
     return _grouped(lib, x.contiguous(), x_scale.float().contiguous(), offsets, [packed if isinstance(packed, TiledWeights) else packed.contiguous()],
-                    [ws.contiguous()], K, group, fmt, out, False, ("auto" if fast else "generic") if algo == "auto" else algo)
+                    [ws.contiguous()], K, group, fmt, out, False, ("auto" if fast else "generic") if algo == "auto" else algo, checked=checked)
 
 
 def sort_by_expert(expert_ids: torch.Tensor, n_experts: int) -> tuple[torch.Tensor, torch.Tensor]:
@@ -306,10 +320,9 @@ def sort_by_expert(expert_ids: torch.Tensor, n_experts: int) -> tuple[torch.Tens
     order = torch.empty(n, dtype=torch.int64, device=ids.device)
     offsets = torch.empty(n_experts + 1, dtype=torch.int64, device=ids.device)
     ws = torch.empty(max(1, lib.dst_sort_workspace_bytes(n, n_experts)), dtype=torch.uint8, device=ids.device)
-    bad = torch.zeros(1, dtype=torch.int32, device=ids.device)
-    with torch.cuda.device(ids.device):
+    with _guard(ids.device):
         rc = lib.dst_sort_by_expert(ids.data_ptr(), int(ids.dtype == torch.int32), n, n_experts, order.data_ptr(),
-                                    offsets.data_ptr(), bad.data_ptr(), ws.data_ptr(), _stream(ids))
+                                    offsets.data_ptr(), None, ws.data_ptr(), _stream(ids))
     _lib.check(rc)
     return order, offsets
 

@@ -108,7 +108,7 @@ class B200Ops:
                 raise ValueError("the gate bias holds one value per expert")
         w = torch.empty(T, top_k, dtype=torch.float32, device=logits.device)
         ids = torch.empty(T, top_k, dtype=torch.int32, device=logits.device)
-        with torch.cuda.device(logits.device):
+        with kb._guard(logits.device):
             _lib.check(lib.dst_route_topk(logits.data_ptr(), bias.data_ptr() if bias is not None else None, T, E, top_k,
                                           _lib.SCORE_FUNCS[score_func], ctypes.c_float(gate_temp), 1 if renorm else 0,
                                           ctypes.c_float(route_scale), w.data_ptr(), ids.data_ptr(), kb._stream(logits)))
@@ -121,8 +121,9 @@ class B200Ops:
         if not (self.fused_norm and self.algo in ("auto", "prefill") and isinstance(weights[0], kb.TiledWeights)):
             return False
         w = weights[0]
-        # few rows per expert stay bf16 for the decode GEMV (TQ2 tiles, or TQ1 with its 2-bit decode copy)
-        decode_rows = kb._decode_row_limit(w.E, w.N) if self.algo == "auto" and (w.fmt == "tq2" or w.decode is not None) else 16
+        # few rows per expert stay bf16 for the decode GEMV (TQ2 tiles, TQ1's 2-bit decode copy, or TQ1 tiles)
+        fmt = "tq2" if w.decode is not None else w.fmt
+        decode_rows = int(self._lib().dst_decode_auto_rows(kb._fmt_code(fmt), len(weights), w.E, rows, w.N)) if self.algo == "auto" else 16
         return rows > decode_rows * w.E
 
     def gather(self, x: torch.Tensor, order: torch.Tensor | None, top_k: int, for_weights=None):
@@ -133,14 +134,14 @@ class B200Ops:
         if for_weights is not None and x.dtype == torch.bfloat16 and self._norm_ok(for_weights, n):
             out = torch.empty(n, x.size(1), dtype=torch.float16, device=x.device)
             fac = torch.empty(n, dtype=torch.float32, device=x.device)
-            with torch.cuda.device(x.device):
+            with kb._guard(x.device):
                 _lib.check(lib.dst_gather_rows_norm(x.data_ptr(), order.data_ptr() if order is not None else None, n, x.size(1), top_k,
                                                     out.data_ptr(), fac.data_ptr(), kb._stream(x)))
             return kb.NormRows(out, fac)
         if order is None:
             return x
         out = torch.empty(order.numel(), x.size(1), dtype=x.dtype, device=x.device)
-        with torch.cuda.device(x.device):
+        with kb._guard(x.device):
             _lib.check(lib.dst_gather_rows(x.data_ptr(), order.data_ptr(), order.numel(), x.size(1), top_k, out.data_ptr(),
                                            kb._stream(x)))
         return out
@@ -161,7 +162,7 @@ class B200Ops:
         pk = (ctypes.c_void_p * n)(*[p.data.data_ptr() for p in packed])
         sc = (ctypes.c_void_p * n)(*[t.data_ptr() for t in scales])
         E, N = packed[0].E, packed[0].N
-        with torch.cuda.device(x.data.device):
+        with kb._guard(x.data.device):
             _lib.check(lib.dst_ternary_grouped_gemm_scatter(peer_out, n_peers, peer_rows, row_target.data_ptr(), kb._OUT[torch.bfloat16], x.data.data_ptr(),
                                                             _lib.ACT_F16_NORM, x.factor.data_ptr(), offsets.data_ptr(), None, pk, sc, n,
                                                             kb._SCALE[scales[0].dtype], E, x.data.size(0), N, K, group, kb._fmt_code(fmt),
@@ -174,7 +175,7 @@ class B200Ops:
         if n_rows_dev is not None:
             h = torch.empty(gu.size(0), inter, dtype=torch.float16, device=gu.device)
             fac = torch.empty(gu.size(0), dtype=torch.float32, device=gu.device)
-            with torch.cuda.device(gu.device):
+            with kb._guard(gu.device):
                 _lib.check(lib.dst_swiglu_norm_dev(gu.data_ptr(), row_weights.data_ptr() if row_weights is not None else None,
                                                    order.data_ptr() if order is not None else None, gu.size(0), n_rows_dev.data_ptr(), inter,
                                                    ctypes.c_float(limit), h.data_ptr(), fac.data_ptr(), kb._stream(gu)))
@@ -182,13 +183,13 @@ class B200Ops:
         if for_weights is not None and self._norm_ok(for_weights, gu.size(0)):
             h = torch.empty(gu.size(0), inter, dtype=torch.float16, device=gu.device)
             fac = torch.empty(gu.size(0), dtype=torch.float32, device=gu.device)
-            with torch.cuda.device(gu.device):
+            with kb._guard(gu.device):
                 _lib.check(lib.dst_swiglu_norm(gu.data_ptr(), row_weights.data_ptr() if row_weights is not None else None,
                                                order.data_ptr() if order is not None else None, gu.size(0), inter,
                                                ctypes.c_float(limit), h.data_ptr(), fac.data_ptr(), kb._stream(gu)))
             return kb.NormRows(h, fac)
         h = torch.empty(gu.size(0), inter, dtype=torch.bfloat16, device=gu.device)
-        with torch.cuda.device(gu.device):
+        with kb._guard(gu.device):
             _lib.check(lib.dst_swiglu(gu.data_ptr(), row_weights.data_ptr() if row_weights is not None else None,
                                       order.data_ptr() if order is not None else None, gu.size(0), inter,
                                       ctypes.c_float(limit), h.data_ptr(), kb._stream(gu)))
@@ -200,11 +201,11 @@ class B200Ops:
         if for_weights is not None and self._norm_ok(for_weights, gu.size(0)):
             h = torch.empty(gu.size(0), inter, dtype=torch.float16, device=gu.device)
             fac = torch.empty(gu.size(0), dtype=torch.float32, device=gu.device)
-            with torch.cuda.device(gu.device):
+            with kb._guard(gu.device):
                 _lib.check(lib.dst_swiglu_std_norm(gu.data_ptr(), gu.size(0), inter, h.data_ptr(), fac.data_ptr(), kb._stream(gu)))
             return kb.NormRows(h, fac)
         h = torch.empty(gu.size(0), inter, dtype=torch.bfloat16, device=gu.device)
-        with torch.cuda.device(gu.device):
+        with kb._guard(gu.device):
             _lib.check(lib.dst_swiglu_std(gu.data_ptr(), gu.size(0), inter, h.data_ptr(), kb._stream(gu)))
         return h
 
@@ -217,7 +218,7 @@ class B200Ops:
         y = torch.empty(T, hidden, dtype=torch.bfloat16, device=down.device)
         ids32 = ids.reshape(-1).to(torch.int32).contiguous()
         w = weights.reshape(-1).float().contiguous()
-        with torch.cuda.device(down.device):
+        with kb._guard(down.device):
             _lib.check(lib.dst_combine_weighted(down.data_ptr(), order.data_ptr(), ids32.data_ptr(), w.data_ptr(), T, top_k, hidden,
                                                 inv.data_ptr(), y.data_ptr(), kb._stream(down)))
         return y
@@ -234,7 +235,7 @@ class B200Ops:
             add = add.contiguous()
             if tuple(add.shape) != (T, hidden) or add.dtype != torch.bfloat16:
                 raise RuntimeError("the added rows must be bf16 [tokens, hidden]")
-        with torch.cuda.device(down.device):
+        with kb._guard(down.device):
             _lib.check(lib.dst_combine_add(down.data_ptr(), order.data_ptr(), ids32.data_ptr(), T, top_k, hidden, inv.data_ptr(),
                                            add.data_ptr() if add is not None else None, y.data_ptr(), kb._stream(down)))
         return y
@@ -327,12 +328,66 @@ class MoELayer:
         xs = self.gather_for_experts(x, None, 1, weights=self.shared)
         return self.experts_forward(xs, None, None, None, weights=self.shared)
 
+    @staticmethod
+    def _c_weights(w: ExpertWeights, device):
+        """``w`` as the C struct, or None where ``dst_moe_layer`` does not cover its shapes or layout."""
+        n, E, H, I = len(w.w13_packed), w.n_experts, w.hidden, w.inter
+        if w.group != 128 or not 1 <= n <= _lib.MAX_TERMS or not len(w.w13_scale) == len(w.w2_packed) == len(w.w2_scale) == n:
+            return None
+        c = _lib.ExpertWeightsC(experts=E, hidden=H, inter=I, n_terms=n, fmt=kb._fmt_code(w.fmt))
+        copies = w.fmt == "tq1" and all(getattr(p, "decode", None) is not None for ps in (w.w13_packed, w.w2_packed) for p in ps)
+        for packed, scales, N, K, to, to_scale, to_decode in ((w.w13_packed, w.w13_scale, 2 * I, H, c.w13, c.s13, c.w13_decode),
+                                                              (w.w2_packed, w.w2_scale, H, I, c.w2, c.s2, c.w2_decode)):
+            for i in range(n):
+                p, s = packed[i], scales[i]
+                if not (isinstance(p, kb.TiledWeights) and p.E == E and p.N == N and p.K == K and p.fmt == w.fmt and p.data.device == device
+                        and s.dtype == torch.float16 and s.shape == (E, N, K // 128) and s.device == device and s.is_contiguous()):
+                    return None
+                to[i], to_scale[i] = p.data.data_ptr(), s.data_ptr()
+                if copies:
+                    to_decode[i] = p.decode.data.data_ptr()
+        return c
+
+    def _layer_call(self, x: torch.Tensor, weights: torch.Tensor, ids: torch.Tensor):
+        """The layer by one call into the library (``dst_moe_layer``), or None where the steps are called one by one: another
+        ops object or a forced kernel, activations that are not bf16 rows of this layer, weights or shapes it does not cover."""
+        if type(self.ops) is not B200Ops or self.ops.algo != "auto" or not self.ops.fused_norm:
+            return None
+        if not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or x.size(1) != self.w.hidden or not (weights.device == ids.device == x.device) \
+                or ids.dtype not in (torch.int32, torch.int64):
+            return None
+        dev, lib = x.device, self.ops._lib()
+        w = self._c_weights(self.w, dev)
+        shared = self._c_weights(self.shared, dev) if self.shared is not None else None
+        if w is None or (self.shared is not None and shared is None):
+            return None
+        T, standard = x.size(0), int(self.flavour == "standard")
+        pw, ps = ctypes.byref(w), ctypes.byref(shared) if shared is not None else None
+        x = x.contiguous()
+        if x.data_ptr() & 15:
+            return None
+        with kb._guard(dev):
+            nbytes = lib.dst_moe_layer_workspace_bytes(T, self.top_k, standard, pw, ps)
+            if nbytes == 0:
+                return None
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            y = torch.empty_like(x)
+            # an id outside [0, E) is dropped, also one that 32 bits would wrap into the range
+            ids32 = (ids if ids.dtype == torch.int32 else ids.clamp(-1, self.w.n_experts).to(torch.int32)).contiguous()
+            wts = weights.float().contiguous()
+            _lib.check(lib.dst_moe_layer(x.data_ptr(), wts.data_ptr(), ids32.data_ptr(), T, self.top_k, standard, ctypes.c_float(self.swiglu_limit),
+                                         pw, ps, y.data_ptr(), ws.data_ptr(), nbytes, kb._stream(x)))
+        return y
+
     def forward_routed(self, x: torch.Tensor, weights: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
         """x [T, hidden] bf16 with routing weights [T, k] f32 and expert ids [T, k] (int32 or int64) that the caller
         computed (``V4Model.route`` / the top-k of ``StandardDecoder._moe``) -> y [T, hidden] bf16. An id outside
         [0, E) drops that (token, slot)."""
         if tuple(weights.shape) != tuple(ids.shape) or weights.size(0) != x.size(0) or weights.size(-1) != self.top_k:
             raise ValueError("weights and ids are [tokens, top_k]")
+        y = self._layer_call(x, weights, ids)
+        if y is not None:
+            return y
         if self.flavour == "standard":
             return self._forward_standard(x, weights, ids)
         T = x.size(0)
@@ -518,7 +573,7 @@ class ExpertParallelMoE:
         row_dest = torch.empty(order.numel(), dtype=torch.int64, device=x.device)
         x = x.contiguous()
         wflat = weights.reshape(-1).contiguous()
-        with torch.cuda.device(x.device):
+        with kb._guard(x.device):
             _lib.check(lib.dst_ep_placement(offs_all.data_ptr(), W, self.E, El, self.rank, dst_start.data_ptr(), offsets2.data_ptr(),
                                             kb._stream(x)))
             ev("offsets all-gather+placement")
@@ -542,7 +597,7 @@ class ExpertParallelMoE:
         inv = torch.empty(T * self.top_k, dtype=torch.int64, device=x.device)
         y = torch.empty(T, hidden, dtype=torch.bfloat16, device=x.device)
         ids32 = ids.reshape(-1).to(torch.int32).contiguous()
-        with torch.cuda.device(x.device):
+        with kb._guard(x.device):
             if fused:
                 _lib.check(lib.dst_ep_combine_returned(buf.back.data_ptr(), order.data_ptr(), row_dest.data_ptr(), ids32.data_ptr(), T,
                                                        self.top_k, hidden, inv.data_ptr(), shared.data_ptr() if shared is not None else None,
@@ -557,7 +612,7 @@ class ExpertParallelMoE:
     def _barrier(self, x: torch.Tensor) -> None:
         """Stream-ordered barrier among the ranks: one small kernel over the symmetric flag words (bounded wait)."""
         self._barrier_seq += 1
-        with torch.cuda.device(x.device):
+        with kb._guard(x.device):
             _lib.check(B200Ops._lib().dst_ep_barrier(self._flag_ptrs, self.world, self.rank, self._barrier_seq, kb._stream(x)))
 
     def _phase_events(self):

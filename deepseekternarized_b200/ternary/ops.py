@@ -11,6 +11,7 @@ contract. Both modes keep their weights in the tiled device layout. There is no 
 
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 
 import torch
@@ -34,7 +35,7 @@ def quant_act_int8(x: torch.Tensor, as_f16: bool = False) -> tuple[torch.Tensor,
     q = torch.empty(x2.shape, dtype=torch.float16 if as_f16 else torch.int8, device=x.device)
     s = torch.empty(x2.size(0), dtype=torch.float32, device=x.device)
     fn = lib.dst_quant_act_int8_f16 if as_f16 else lib.dst_quant_act_int8
-    with torch.cuda.device(x.device):
+    with kb._guard(x.device):
         _lib.check(fn(x2.data_ptr(), int(x2.dtype == torch.float32), x2.size(0), x2.size(1), q.data_ptr(), s.data_ptr(), kb._stream(x2)))
     return q.view(*lead, -1), s.view(lead)
 
@@ -68,6 +69,7 @@ class TernaryLinear:
         self.backend, self.algo = backend, algo
         self.decode_copy = decode_copy  # TQ1: keep a tiled TQ2 copy of the trits on the device for few-row calls
         self._dev = None
+        self._direct = None  # pointer tables of the tiled weights in _dev
 
     def _on(self, device):
         """([packed], [scale [1,N,G]]) on ``device``, copied once and kept. Shapes the fast kernels cover
@@ -86,7 +88,36 @@ class TernaryLinear:
             if self.algo != "generic" and kb.fast_path_covers(self.K, self.group, scales[0].dtype):
                 packed = [kb.tile_weights(p, self.fmt, self.K, self.decode_copy) for p in packed]
             self._dev = (device, packed, scales)
+            self._direct = self._pointers(packed, scales)
         return self._dev[1], self._dev[2]
+
+    def _pointers(self, packed, scales):
+        """What the C entry takes of the weights kept in ``_dev`` (None: the general path): pointer tables of the tiles, the
+        scales and, where every term has one, the 2-bit decode copies."""
+        n, N = len(packed), self.out_features
+        if not (1 <= n <= _lib.MAX_TERMS and all(isinstance(p, kb.TiledWeights) and p.E == 1 and p.N == N for p in packed)
+                and all(tuple(s.shape) == (1, N, self.K // self.group) for s in scales)):
+            return None
+        table = ctypes.c_void_p * n
+        dec = table(*[p.decode.data.data_ptr() for p in packed]) if self.fmt == "tq1" and all(p.decode is not None for p in packed) else None
+        return table(*[p.data.data_ptr() for p in packed]), dec, table(*[s.data_ptr() for s in scales])
+
+    def _gemm(self, x: torch.Tensor, act: int, row_scale, out: torch.Tensor, algo: str) -> None:
+        """The launch of ``kb._grouped`` for weights that ``_on`` laid out and checked: rows [T, K] of this layer's K, no offsets."""
+        lib = kb._require(self.backend)
+        x = x.contiguous()
+        T, N = out.shape
+        pk, dec, sc = self._direct
+        code = kb._fmt_code(self.fmt)
+        if dec is not None and algo in ("auto", "decode") and act != _lib.ACT_F16_NORM and T <= kb._decode_row_limit(1, N):
+            pk, code, algo = dec, _lib.FMT_TQ2, "decode"
+        ws_bytes = int(lib.dst_gemm_workspace_bytes(kb._ALGO[algo], act, T, self.K)) if act != _lib.ACT_F16_NORM else 0
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
+        with kb._guard(x.device):
+            _lib.check(lib.dst_ternary_grouped_gemm(
+                out.data_ptr(), kb._OUT[out.dtype], 0, x.data_ptr(), act, row_scale.data_ptr() if row_scale is not None else None, None, None,
+                pk, _lib.LAYOUT_TILED, sc, len(pk), _lib.SCALE_F16, 1, T, N, self.K, self.group, code, kb._ALGO[algo],
+                ws.data_ptr() if ws is not None else None, ws_bytes, kb._stream(x)))
 
     @property
     def out_features(self) -> int:
@@ -113,19 +144,30 @@ class TernaryLinear:
             lib = kb._require(self.backend)
             out = torch.empty(x2.size(0), self.out_features, dtype=torch.float32, device=x2.device)
             tiled = isinstance(packed[0], kb.TiledWeights)
-            if tiled and self.algo in ("auto", "prefill") and x2.size(0) > 16:
-                # many rows: quantise straight into the tcgen05 kernel's row format (2 launches per linear)
+            if tiled and self.algo in ("auto", "prefill") and (x2.size(0) > 16 or (self.fmt == "tq1" and packed[0].decode is None)):
+                # many rows, or weights whose decode GEMV takes no int8 rows: quantise straight into the tcgen05 kernel's row
+                # format (2 launches per linear)
                 qh, s = quant_act_int8(x2, as_f16=True)
-                kb.grouped_ternary_gemm_bf16(kb.NormRows(qh, s), None, packed, scales, self.K, self.group, self.fmt, out=out,
-                                             backend=self.backend)
+                if self._direct is not None:
+                    self._gemm(qh, _lib.ACT_F16_NORM, s, out, "prefill")
+                else:
+                    kb.grouped_ternary_gemm_bf16(kb.NormRows(qh, s), None, packed, scales, self.K, self.group, self.fmt, out=out,
+                                                 backend=self.backend)
             else:
                 q, s = quant_act_int8(x2)
-                kb._grouped(lib, q, s, None, packed, scales, self.K, self.group, self.fmt, out, False, self.algo)
+                if self._direct is not None:
+                    self._gemm(q, _lib.ACT_I8, s, out, self.algo)
+                else:
+                    kb._grouped(lib, q, s, None, packed, scales, self.K, self.group, self.fmt, out, False, self.algo)
         else:
             xa = x2 if x2.dtype in (torch.bfloat16, torch.float16) else x2.bfloat16()
             od = out_dtype if out_dtype in (torch.float32, torch.bfloat16, torch.float16) else torch.float32
-            out = kb.grouped_ternary_gemm_bf16(xa, None, packed, scales, self.K, self.group, self.fmt, out_dtype=od,
-                                               algo=self.algo, backend=self.backend)
+            if self._direct is not None:
+                out = torch.empty(xa.size(0), self.out_features, dtype=od, device=xa.device)
+                self._gemm(xa, kb._ACT[xa.dtype], None, out, self.algo)
+            else:
+                out = kb.grouped_ternary_gemm_bf16(xa, None, packed, scales, self.K, self.group, self.fmt, out_dtype=od,
+                                                   algo=self.algo, backend=self.backend)
         return out.view(*shape[:-1], -1).to(out_dtype)
 
 
@@ -143,7 +185,7 @@ def _gather_call(packed_ptrs, scale_ptrs, sdt, ids: torch.Tensor, V: int, K: int
     n = len(packed_ptrs)
     pk = (ctypes.c_void_p * n)(*packed_ptrs)
     sc = (ctypes.c_void_p * n)(*scale_ptrs)
-    with torch.cuda.device(flat.device):
+    with kb._guard(flat.device):
         _lib.check(lib.dst_gather_dequant_rows_strided(pk, sc, n, kb._SCALE[sdt], flat.data_ptr(), flat.numel(), V, K, group, kb._fmt_code(fmt),
                                                        pstride, sstride, out.data_ptr(), bad.data_ptr() if check else None, kb._stream(flat)))
     if check and int(bad.item()):

@@ -584,6 +584,79 @@ def test_moe_layer_steps_against_oracle(fmt, k_terms):
     assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("fmt,k_terms,copy", [("tq1", 1, False), ("tq1", 2, True), ("tq2", 2, False)])
+@pytest.mark.parametrize("flavour", ["v4", "standard"])
+def test_moe_layer_in_one_call_equals_its_steps(fmt, k_terms, copy, flavour):
+    """The library's whole-layer entry against the same layer by single steps, bit for bit: one token up to many rows per
+    expert (quantised rows gathered and written by SwiGLU, the TQ1 GEMV, the tcgen05 kernel), clamp and shared expert, ids
+    that are dropped or do not fit 32 bits."""
+    from deepseekternarized_b200.moe import B200Ops, ExpertWeights, MoELayer
+
+    class Steps(B200Ops):  # any other ops object gets the steps one by one
+        pass
+
+    E, hidden, inter, top_k = 40, 512, 512, 3
+    rng = np.random.default_rng(k_terms)
+
+    def experts(n):
+        gen = torch.Generator(device=DEV).manual_seed(n)
+        sizes = {"w13": (n, 2 * inter, hidden), "w2": (n, hidden, inter)}
+        from deepseekternarized_b200.ternary.pack import pack
+        packed = {k: [pack(torch.randint(-1, 2, (a * b, c), generator=gen, device=DEV, dtype=torch.int8), fmt).view(a, b, -1) for _ in range(k_terms)]
+                  for k, (a, b, c) in sizes.items()}
+        scale = {k: [(torch.rand(a, b, c // 128, generator=gen, device=DEV) * 0.02 + 0.005).half() for _ in range(k_terms)] for k, (a, b, c) in sizes.items()}
+        return ExpertWeights(packed["w13"], scale["w13"], packed["w2"], scale["w2"], hidden, inter, 128, fmt).prepare(decode_copy=copy)
+
+    w, shared = experts(E), experts(1)
+    kw = {"flavour": flavour} if flavour == "standard" else {"flavour": flavour, "swiglu_limit": 1.5, "shared": shared, "score_func": "sqrtsoftplus"}
+    for T in (1, 2, 13, 100, 700, 2600):
+        x = torch.from_numpy(rng.standard_normal((T, hidden)).astype(np.float32)).to(DEV).bfloat16()
+        logits = torch.from_numpy(rng.standard_normal((T, E)).astype(np.float32)).to(DEV)
+        one, steps = MoELayer(w, top_k, **kw), MoELayer(w, top_k, ops=Steps(), **kw)
+        wts, ids = one.route(logits)
+        assert one._layer_call(x, wts, ids) is not None and steps._layer_call(x, wts, ids) is None
+        assert torch.equal(one(x, logits), steps(x, logits))
+        wide = ids.to(torch.int64)
+        wide[0, 1], wide[T // 2, 0] = -1, (1 << 32) + 3
+        assert torch.equal(one.forward_routed(x, wts, wide), steps.forward_routed(x, wts, wide))
+
+
+@pytest.mark.parametrize("n,E", [(1, 1), (31, 5), (1023, 384), (1024, 4096), (1025, 384), (5000, 4096), (3000, 1)])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_sort_edges(kb, n, E, dtype):
+    """Both forms of the routing sort (one block, chunks) around their border, with ids that are dropped."""
+    rng = np.random.default_rng(n + E)
+    ids = rng.integers(-1, E + 1, n)
+    order, offsets = kb.sort_by_expert(torch.from_numpy(ids).to(DEV, dtype), E)
+    keep = np.flatnonzero((ids >= 0) & (ids < E))
+    want = keep[np.argsort(ids[keep], kind="stable")]
+    assert np.array_equal(order.cpu().numpy()[: len(want)], want) and (order.cpu().numpy()[len(want):] == -1).all()
+    assert np.array_equal(offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(ids[keep], minlength=E))]))
+
+
+@pytest.mark.parametrize("E", [8, 33, 384, 1000])
+def test_route_ties_and_non_finite_logits(E):
+    """Ranks of the router's keys: equal keys give the lowest id, NaN ranks above everything, -inf below, +0 and -0 tie."""
+    from deepseekternarized_b200.moe import B200Ops
+
+    rng = np.random.default_rng(E)
+    logits = rng.integers(-3, 4, (64, E)).astype(np.float32)
+    logits[1], logits[2] = -np.inf, np.nan
+    logits[3, E // 2], logits[4, ::2], logits[5, 3] = np.nan, -np.inf, np.inf
+    bias = np.where(np.arange(E) % 2 == 0, 0.0, -0.0).astype(np.float32)
+    for score in ("sigmoid", "softmax"):
+        w, ids = B200Ops().route(torch.from_numpy(logits).to(DEV), 6, 1.0, score_func=score, bias=torch.from_numpy(bias))
+        ids = ids.cpu().numpy()
+        assert ((ids >= 0) & (ids < E)).all() and all(len(set(r)) == 6 for r in ids)
+        for t in (0, 1, 2, 3 if score == "sigmoid" else 0, 4, 6, 63):
+            l = logits[t].astype(np.float64)
+            key = np.where(np.isnan(l), np.inf, l) if score == "sigmoid" or np.isfinite(l).all() else (l if not np.isnan(l).any() else np.zeros(E))
+            if t == 1:
+                key = np.zeros(E)
+            want = np.argsort(-key, kind="stable")[:6]
+            assert np.array_equal(ids[t], want), (score, t)
+
+
 def test_host_pipeline_equals_direct_calls():
     """Batches fed from pinned host buffers through the three-stream pipeline (ragged sizes, more batches than
     slots, distinct output buffers) equal the layer called on device-resident copies of the same batches."""
