@@ -1210,6 +1210,26 @@ int launch_fmt(const TmaMaps& maps, PrefillParams p, cudaStream_t st) {
   // room for it.
   int tn_cap = (p.rows_hint + 31) / 32 * 32;
   tn_cap = tn_cap < 64 ? 64 : (tn_cap > PF_TN_MAX ? PF_TN_MAX : tn_cap);
+  if (p.E == 1) {
+    // One matrix: the row count is known, and few, large tiles may leave SMs idle. The token tile that gives the least (waves of
+    // tiles) x (time of a 64-K stage, ns: fits of what 64 to 256 rows and one and two terms measured). 333 rows through
+    // 4096 x 4096: 4 x 32 tiles of 84 rows instead of 2 x 32 of 167, kernel 30 -> 26 us; 2048 rows through 4096 x 11008, two terms: 203 -> 199 us per call.
+    float best = 0.f;
+    int best_tn = 0;
+    for (int tn = 64; tn <= tn_cap; tn += 32) {
+      p.tn_max = tn;
+      const bool small = tn <= PF_SMALL_TN;
+      if ((small ? plan_smem<FMT, TERMS, true>(p, 2) : plan_smem<FMT, TERMS, false>(p, 4)) == 0) continue;
+      const long long tiles = cdiv64(p.T, tn), rows = cdiv64(p.T, tiles);
+      const float stage = (small ? 245.f + 0.9f * (float)(rows > 64 ? rows - 64 : 0) : 230.f + 0.9f * (float)rows) + 135.f * (float)(p.n_terms - 1);
+      const float cost = (float)cdiv64(tiles * p.NT, 148) * stage;
+      if (best_tn == 0 || cost < best) {
+        best = cost;
+        best_tn = tn;
+      }
+    }
+    if (best_tn != 0) tn_cap = best_tn;
+  }
   for (p.tn_max = tn_cap; p.tn_max > PF_SMALL_TN; p.tn_max -= 32)
     if (const size_t smem = plan_smem<FMT, TERMS, false>(p, 4)) return launch_plan<FMT, TERMS, false>(maps, p, smem, st);
   for (; p.tn_max >= 64; p.tn_max -= 32)
@@ -1269,7 +1289,8 @@ int launch_prefill(const GemmArgs& a, cudaStream_t stream) {
   const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.T};
   const cuuint64_t strides[1] = {(cuuint64_t)a.K * 2};
   const cuuint32_t estr[2] = {1, 1};
-  for (int i = 0; i < 16; ++i) {
+  const int heights = (int)((a.max_rows >= 0 && a.max_rows < 256 ? a.max_rows : 256) + 15) / 16;  // no tile has more rows than an expert
+  for (int i = 0; i < heights; ++i) {
     const cuuint32_t box[2] = {64, (cuuint32_t)(16 * (i + 1))};
     const CUresult cr = encode_fn()(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xh), dims, strides, box, estr,
                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
