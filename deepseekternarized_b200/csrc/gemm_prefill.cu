@@ -20,8 +20,8 @@
 // What bounds it: up to ~128 token rows the instruction streams of the dequant warps and of the MMA issuer (130 to 500
 // cycles of tensor work per 64 K, ~470 spent), above that the tensor pipe and the drain of the one accumulator. Measured
 // on 96 experts of 4096 x 4096, one launch, this form / the one before (one 64-trit piece per group and step, two issuing
-// warps on one ring of A and B slots, digit-field tables): TQ1 64 rows 326 / 629 us, 256 rows 615 / 736; TQ2 64 rows
-// 338 / 577, 256 rows 607 / 689; two TQ2 terms 64 rows 521 / 869.
+// warps on one ring of A and B slots, digit-field tables): TQ1 64 rows 310 / 629 us, 256 rows 599 / 736; TQ2 64 rows
+// 319 / 577, 256 rows 590 / 689; two TQ2 terms 64 rows 502 / 869.
 // Shared-memory bandwidth is what bounds this kernel when A goes through shared memory (measured: the MMA
 // issuer stalled ~1100 cycles per 512-cycle stage); with A in TMEM only B is written and read there.
 // bf16 activations are converted once to fp16 with a power-of-two factor per row (exact for every
@@ -161,6 +161,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -202,13 +205,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (mbar_test(bar, parity)) return true;
   const long long t0 = clock64();
   for (;;) {
-    if (BACKOFF ? mbar_test(bar, parity) : mbar_spin(bar, parity)) return true;
+    if (BACKOFF) {
+#pragma unroll 1
+      for (int i = 0; i < 16; ++i) {
+        __nanosleep(200);
+        if (mbar_test(bar, parity)) return true;
+      }
+    } else if (mbar_spin(bar, parity)) {
+      return true;
+    }
     if (*abort_flag) return false;
     if (clock64() - t0 > g_wait_cycles) {
       *abort_flag = 1;
       return false;
     }
-    if (BACKOFF) __nanosleep(200);
   }
 }
 
@@ -896,9 +906,9 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
     // A group takes 128 trits (two pieces: one scale group) at a time: unit `own`, counted over all tiles of this CTA. The
     // bookkeeping around a piece (barriers, slab slots, scale, loop) costs as much as its arithmetic and is paid once for two.
     const int units = kstages >> 1;
-    uint32_t own = grp;
-    uint32_t gst = grp * (2 / KH), s = gst % NA;  // the unit's (first) stage and its A slot
-    uint32_t it0 = 0, gs0 = 0;                     // first unit / first slab of the current tile
+    uint32_t gst = grp * (2 / KH), s = gst % NA;  // the group's next unit's (first) stage, counted over all tiles of this CTA, and its A slot
+    uint32_t gs0 = 0;                              // first slab of the current tile
+    int g = (int)grp;                              // the group's next unit, from the current tile's first on
     bool ok = true;
     RT_DECL(w_pfull = 0, w_dempty = 0, w_drain = 0, w_comp = 0, w_st = 0, w_pre = 0, n_it = 0, t_begin = RT_NOW(), w_lds = 0, w_tail = 0, t_tail = RT_NOW());
 
@@ -924,29 +934,34 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
         }
       }
     };
-    int t = (int)blockIdx.x - t_step;  // tile being dequantised; before the first one here
-    bool in_tile = false;
-    int n = 0;
-    for (;;) {
-      if (!(in_tile && (int32_t)(own - it0) < units)) {
-        // past the end of the current tile (or before the first): look up the next one
-        if (in_tile) {
-          it0 += (uint32_t)units;
-          gs0 += (uint32_t)nsb;
-          in_tile = false;
-        }
-        if (t + t_step >= n_tiles) break;
-        t += t_step;
-        tile_seek(p, offs, tpre, t, e, nt, row0, rows);
-        n = nt * 128 + r;
+    // SMALL TQ1: a group's units are ten pieces = two whole superblocks apart, so the pieces of all its units of a tile sit at
+    // the same place of their superblocks and the words' offsets are found once per tile
+    constexpr bool FIXED = SMALL && FMT == 1;
+    static_assert(!FIXED || 2 * n_groups % SPB == 0, "units of a group at the same place of a superblock");
+    uint32_t place[2][3] = {};  // FIXED: offsets of the words 3 sbk, 3 sbk + 1, 3 sbk + 2 of both pieces
+    int sbk[2], sb0 = 0;        // piece inside its superblock; FIXED: the unit's first piece's superblock
+    for (int t = (int)blockIdx.x; ok && t < n_tiles; t += t_step, g -= units, gs0 += (uint32_t)nsb) {
+      if (g >= units) continue;  // a tile with fewer units than groups: none of them is this group's
+      tile_seek(p, offs, tpre, t, e, nt, row0, rows);
+      const int n = nt * 128 + r;
 #pragma unroll
-        for (int i = 0; i < TERMS; ++i)
-          if (i < p.n_terms) srow[i] = n < p.N ? p.scale[i] + ((int64_t)e * p.N + n) * p.G : nullptr;
-        cur_b = -1;
-        in_tile = true;
-        continue;
+      for (int i = 0; i < TERMS; ++i)
+        if (i < p.n_terms) srow[i] = n < p.N ? p.scale[i] + ((int64_t)e * p.N + n) * p.G : nullptr;
+      cur_b = -1;
+      if (FIXED) {
+        sb0 = 2 * g / SPB;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          sbk[x] = (2 * g + x) % SPB;
+          const int k0 = 3 * sbk[x];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const int lw = k0 + j;
+            place[x][j] = (uint32_t)(r * 64 + (((lw & 3) ^ ((r >> 1) & 3)) << 4) + (lw >> 2) * 4);
+          }
+        }
       }
-      const int g = (int)(own - it0);  // the unit inside the tile = its scale group
+      for (; g < units; g += (int)n_groups) {
       RT_DECL(t_pre = RT_NOW());
       RT_SPAN(w_tail, t_tail);
       // scales
@@ -966,10 +981,15 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
       // the producer. One term: both pieces' words up front; more: a piece at a time (registers).
       constexpr int WX = TERMS == 1 ? 2 : 1;
       uint32_t w[WX][TERMS][4];
-      int sbk[2];
       auto load_piece = [&](int x, uint32_t (&dst)[TERMS][4]) -> bool {
-        const int ks = 2 * g + x, sb = ks / SPB;
-        sbk[x] = ks - sb * SPB;
+        const int ks = 2 * g + x;
+        int sb;
+        if (FIXED) {
+          sb = x == 0 ? sb0 : sb0 + (sbk[1] == 0);
+        } else {
+          sb = ks / SPB;
+          sbk[x] = ks - sb * SPB;
+        }
         const uint32_t gs = gs0 + (uint32_t)sb;
         const uint32_t slot = p.nslab == 2 ? (gs & 1u) : gs % 3u;
         const bool same = x == 1 && sbk[1] != 0;  // the first piece's slab
@@ -982,6 +1002,10 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
             if (FMT == 2) {  // word 4 sbk + j
 #pragma unroll
               for (int j = 0; j < 4; ++j) dst[i][j] = lds32(wp + unit_off[j] + sbk[x] * 4);
+            } else if (FIXED) {
+#pragma unroll
+              for (int j = 0; j < 3; ++j) dst[i][j] = lds32(wp + place[x][j]);
+              dst[i][3] = lds32(wp + unit_off[3] + 12);
             } else {         // words 3 sbk, 3 sbk + 1, 3 sbk + 2 and 15
               switch (sbk[x]) {
                 case 0: dst[i][0] = lds32(wp + unit_off[0]); dst[i][1] = lds32(wp + unit_off[1]); dst[i][2] = lds32(wp + unit_off[2]); break;
@@ -994,11 +1018,13 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
             }
           }
         }
-        __syncwarp();
-        if (lane == 0) {
-          // the tile's last superblock may hold fewer than SPB pieces: make up for those that do not exist
-          const int n_arrive = 1 + (ks == kstages - 1 ? nsb * SPB - kstages : 0);
-          for (int y = 0; y < n_arrive; ++y) mbar_arrive(smem_u32(&bar_pempty[gs % PF_BARS]));
+        // the slab goes back; the tile's last superblock may hold fewer than SPB pieces: make up for those that do not exist.
+        // One term: both pieces' arrivals at once where they share the slab
+        if (!(TERMS == 1 && x == 0 && sbk[0] != SPB - 1)) {
+          __syncwarp();
+          if (lane == 0)
+            mbar_arrive_n(smem_u32(&bar_pempty[gs % PF_BARS]),
+                          (uint32_t)((TERMS == 1 && same ? 2 : 1) + (ks == kstages - 1 ? nsb * SPB - kstages : 0)));
         }
 #ifdef DST_ROLE_TIMERS
 #pragma unroll
@@ -1009,7 +1035,7 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
         RT_SPAN(w_lds, t_lds);
         return true;
       };
-      if (TERMS == 1 && (!load_piece(0, w[0]) || !load_piece(1, w[WX - 1]))) break;
+      if (TERMS == 1 && (!load_piece(0, w[0]) || !load_piece(1, w[WX - 1]))) { ok = false; break; }
 
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
@@ -1071,11 +1097,12 @@ prefill_kernel(const __grid_constant__ TmaMaps xmaps, const PrefillParams p) {
       ++n_it;
       t_tail = RT_NOW();
 #endif
-      own += n_groups;
       constexpr uint32_t jump = SMALL ? n_groups : 2 * n_groups - 1;  // to the first stage of the group's next unit
       gst += jump;
       s += jump;
       while (s >= NA) s -= NA;
+      if (FIXED) sb0 += 2 * (int)n_groups / SPB;
+      }
     }
     if (warp == PF_DQ_WARP0 && lane == 0) {
       RT_ADD(24, RT_NOW() - t_begin); RT_ADD(25, w_pfull); RT_ADD(26, w_dempty); RT_ADD(27, n_it); RT_ADD(28, 1);
