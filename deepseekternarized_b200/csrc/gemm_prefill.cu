@@ -126,7 +126,7 @@ struct PrefillParams {
   int E, T, N, K, G, NT, S, kstages;
   // chosen by the host from the shared-memory budget
   int tn_max;       // token rows per tile at most (a multiple of 32, <= PF_TN_MAX): accumulator columns 0 .. tn_max - 1, the A ring after them
-  int rows_hint;    // most rows an expert is expected to have (host knowledge or twice the mean), sizes tn_max
+  int rows_hint;    // most rows an expert is expected to have (host knowledge or the mean and three deviations), sizes tn_max
   int nb;           // B stages in shared memory
   int na;           // A slots in TMEM = length of the barrier rings (nb <= na): stage g uses A slot g % na and B stage g % nb
   int nslab;        // slots of the packed-slab ring, 2 or 3

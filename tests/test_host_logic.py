@@ -218,3 +218,109 @@ def test_host_pipeline_has_no_cpu_path():
         HostPipeline(lambda x, lg: x, 8, 16, 4, "cpu")
     with pytest.raises(ValueError):
         HostPipeline(lambda x, lg: x, 8, 16, 4, "cpu", slots=1)
+
+
+def _prefill_roles(small, spb, pieces, tiles, na, nb, nslab, rnd):
+    """The barrier protocol of the tcgen05 kernel's roles (csrc/gemm_prefill.cu), restated: stage g's barriers are entry g % 16
+    of their rings whatever the number of A slots, B stages and slabs; a wait only sees a phase's parity. Interleaves the
+    roles at random; raises when a role reads a slot that does not hold its data, writes one that is still read, or hangs."""
+    kh, groups, ring = (2, 5, 16) if small else (1, 4, 16)
+    bar = {}
+
+    def count(kind):
+        return {"full": 2, "empty": 1, "pfull": 1, "pempty": spb}[kind]
+
+    def arrive(kind, g, n=1):
+        b = bar.setdefault((kind, g % ring), [0, count(kind)])  # phase, arrivals that are missing
+        for _ in range(n):
+            b[1] -= 1
+            if b[1] == 0:
+                b[0], b[1] = b[0] + 1, count(kind)
+
+    def wait(kind, g):
+        while (bar.setdefault((kind, g % ring), [0, count(kind)])[0] & 1) == (g // ring & 1):
+            yield
+
+    a_slot, b_slot, slab = [None] * na, [None] * nb, [None] * nslab
+    nsb, stages, done = -(-pieces // spb), tiles * pieces // kh, [0]
+
+    def copy_rows():
+        for g in range(stages):
+            if g >= nb:
+                yield from wait("empty", g - nb)
+            assert g < nb or done[0] > g - nb
+            b_slot[g % nb] = g
+            arrive("full", g)
+            yield
+
+    def copy_slabs():
+        for i in range(tiles * nsb):
+            if i >= nslab:
+                yield from wait("pempty", i - nslab)
+            yield
+            slab[i % nslab] = i
+            arrive("pfull", i)
+            yield
+
+    def mma():
+        for g in range(stages):
+            yield from wait("full", g)
+            assert a_slot[g % na] == [g * kh + h for h in range(kh)] and b_slot[g % nb] == g
+            yield
+            done[0] = g + 1
+            arrive("empty", g)
+            yield
+
+    def dequant(unit):
+        gst, gs0, g = unit * 2 // kh, 0, unit
+        for _ in range(tiles):
+            while g < pieces // 2:
+                for x in range(2):
+                    k = 2 * g + x
+                    gs = gs0 + k // spb
+                    if x == 0 or k % spb == 0:
+                        yield from wait("pfull", gs)
+                    assert slab[gs % nslab] == gs
+                    yield
+                    arrive("pempty", gs, 1 + (nsb * spb - pieces if k == pieces - 1 else 0))
+                for x in range(2):
+                    if not small or x == 0:
+                        if gst >= na:
+                            yield from wait("empty", gst - na)
+                        assert gst < na or done[0] > gst - na
+                        a_slot[gst % na] = []
+                    yield
+                    a_slot[gst % na].append(gst * kh + (x if small else 0))
+                    if not small or x == 1:
+                        arrive("full", gst)
+                    if not small and x == 0:
+                        gst += 1
+                gst += groups if small else 2 * groups - 1
+                g += groups
+            g -= pieces // 2
+            gs0 += nsb
+
+    roles = [copy_rows(), copy_slabs(), mma()] + [dequant(i) for i in range(groups)]
+    weight = [10 ** rnd.uniform(-0.5, 0.5) for _ in roles]
+    live = list(range(len(roles)))
+    for _ in range(60000):
+        i = rnd.choices(live, [weight[j] for j in live])[0]
+        try:
+            next(roles[i])
+        except StopIteration:
+            live.remove(i)
+        if not live:
+            break
+    assert not live and done[0] == stages
+
+
+@pytest.mark.parametrize("seed", range(30))
+def test_prefill_barrier_protocol_under_random_interleavings(seed):
+    """Every ring length that the host's plan can give, from one unit of 128 trits per tile on (a dequant group then jumps over
+    several tiles: with as many barriers as slots it came back two phases on)."""
+    import random
+
+    rnd = random.Random(seed)
+    small = bool(seed & 1)
+    na = rnd.choice([6, 7]) if small else rnd.choice([6, 7, 8, 9, 11])
+    _prefill_roles(small, rnd.choice([4, 5]), 2 * rnd.choice([1, 1, 2, 3, 5, 8]), rnd.randint(1, 7), na, rnd.randint(2, na), rnd.choice([2, 3]), rnd)
