@@ -48,6 +48,23 @@ class PackedTerm:
     scale: torch.Tensor  # [N, G] fp16/bf16 as stored
 
 
+class _Layout:
+    """A linear's weights on one device and the pointer tables that the C entry takes of exactly these tensors (``tables``
+    None: the general path): tiles, 2-bit decode copies (None unless every term has one), scales. Built whole and not
+    changed afterwards, so threads that share a linear see no table without the tensors it points into."""
+
+    def __init__(self, device, packed: list, scales: list, N: int, K: int, group: int):
+        self.device, self.packed, self.scales = device, packed, scales
+        n = len(packed)
+        self.tables = None
+        if 1 <= n <= _lib.MAX_TERMS and all(isinstance(p, kb.TiledWeights) and p.E == 1 and p.N == N for p in packed) \
+                and all(tuple(s.shape) == (1, N, K // group) for s in scales):
+            table = ctypes.c_void_p * n
+            copies = [p.decode for p in packed] if packed[0].fmt == "tq1" else [None]
+            dec = table(*[c.data.data_ptr() for c in copies]) if all(c is not None for c in copies) else None
+            self.tables = table(*[p.data.data_ptr() for p in packed]), dec, table(*[s.data_ptr() for s in scales])
+
+
 class TernaryLinear:
     """Drop-in for the reference class (``ops.py:34-86``): same constructor, same call.
 
@@ -68,14 +85,15 @@ class TernaryLinear:
         self.terms, self.K, self.fmt, self.group, self.act = terms, K, fmt, group, act
         self.backend, self.algo = backend, algo
         self.decode_copy = decode_copy  # TQ1: keep a tiled TQ2 copy of the trits on the device for few-row calls
-        self._dev = None
-        self._direct = None  # pointer tables of the tiled weights in _dev
+        self._dev = None  # the _Layout in use, replaced as a whole
 
-    def _on(self, device):
-        """([packed], [scale [1,N,G]]) on ``device``, copied once and kept. Shapes the fast kernels cover
-        (group 128, K % 128 == 0, fp16 scales; both activation modes) are kept in the tiled device layout,
-        everything else as the canonical ``[1, N, Kp]`` bytes."""
-        if self._dev is None or self._dev[0] != device:
+    def _layout(self, device) -> "_Layout":
+        """The weights on ``device``, copied once and kept. Shapes the fast kernels cover (group 128, K % 128 == 0, fp16
+        scales; both activation modes) are kept in the tiled device layout, everything else as the canonical ``[1, N, Kp]``
+        bytes. A caller works with the object it got here: another thread may put its own, also of another device, in its
+        place in ``_dev`` at any time."""
+        laid = self._dev
+        if laid is None or laid.device != device:
             packed = [t.packed.to(device).contiguous()[None] for t in self.terms]
             scales = []
             for t in self.terms:
@@ -87,27 +105,16 @@ class TernaryLinear:
                 scales = [s.float() for s in scales]
             if self.algo != "generic" and kb.fast_path_covers(self.K, self.group, scales[0].dtype):
                 packed = [kb.tile_weights(p, self.fmt, self.K, self.decode_copy) for p in packed]
-            self._dev = (device, packed, scales)
-            self._direct = self._pointers(packed, scales)
-        return self._dev[1], self._dev[2]
+            laid = _Layout(device, packed, scales, self.out_features, self.K, self.group)
+            self._dev = laid
+        return laid
 
-    def _pointers(self, packed, scales):
-        """What the C entry takes of the weights kept in ``_dev`` (None: the general path): pointer tables of the tiles, the
-        scales and, where every term has one, the 2-bit decode copies."""
-        n, N = len(packed), self.out_features
-        if not (1 <= n <= _lib.MAX_TERMS and all(isinstance(p, kb.TiledWeights) and p.E == 1 and p.N == N for p in packed)
-                and all(tuple(s.shape) == (1, N, self.K // self.group) for s in scales)):
-            return None
-        table = ctypes.c_void_p * n
-        dec = table(*[p.decode.data.data_ptr() for p in packed]) if self.fmt == "tq1" and all(p.decode is not None for p in packed) else None
-        return table(*[p.data.data_ptr() for p in packed]), dec, table(*[s.data_ptr() for s in scales])
-
-    def _gemm(self, x: torch.Tensor, act: int, row_scale, out: torch.Tensor, algo: str) -> None:
-        """The launch of ``kb._grouped`` for weights that ``_on`` laid out and checked: rows [T, K] of this layer's K, no offsets."""
+    def _gemm(self, laid: "_Layout", x: torch.Tensor, act: int, row_scale, out: torch.Tensor, algo: str) -> None:
+        """The launch of ``kb._grouped`` for weights that ``_layout`` laid out and checked: rows [T, K] of this layer's K, no offsets."""
         lib = kb._require(self.backend)
         x = x.contiguous()
         T, N = out.shape
-        pk, dec, sc = self._direct
+        pk, dec, sc = laid.tables
         code = kb._fmt_code(self.fmt)
         if dec is not None and algo in ("auto", "decode") and act != _lib.ACT_F16_NORM and T <= kb._decode_row_limit(1, N):
             pk, code, algo = dec, _lib.FMT_TQ2, "decode"
@@ -125,10 +132,11 @@ class TernaryLinear:
 
     def dequantized(self) -> torch.Tensor:
         """fp32 [N, K] ``sum_i unpack(packed_i) * scale_i`` (reference ``ops.py:51-58``), built with the unpack kernel."""
-        dev = self._dev[0] if self._dev is not None else "cuda"
-        packed, scales = self._on(torch.device(dev))
+        laid = self._dev
+        if laid is None:
+            laid = self._layout(torch.device("cuda"))
         w = None
-        for p, s in zip(packed, scales):
+        for p, s in zip(laid.packed, laid.scales):
             p = p.untile() if isinstance(p, kb.TiledWeights) else p
             d = unpack(p[0], self.fmt, self.K).float() * s[0].float().repeat_interleave(self.group, -1)[:, : self.K]
             w = d if w is None else w + d
@@ -139,7 +147,8 @@ class TernaryLinear:
             raise RuntimeError("B200 ternary kernel unavailable for CPU tensors (this backend has no CPU path)")
         shape = x.shape
         x2 = x.reshape(-1, self.K)
-        packed, scales = self._on(x2.device)
+        laid = self._layout(x2.device)
+        packed, scales = laid.packed, laid.scales
         if self.act == "int8":
             lib = kb._require(self.backend)
             out = torch.empty(x2.size(0), self.out_features, dtype=torch.float32, device=x2.device)
@@ -148,23 +157,23 @@ class TernaryLinear:
                 # many rows, or weights whose decode GEMV takes no int8 rows: quantise straight into the tcgen05 kernel's row
                 # format (2 launches per linear)
                 qh, s = quant_act_int8(x2, as_f16=True)
-                if self._direct is not None:
-                    self._gemm(qh, _lib.ACT_F16_NORM, s, out, "prefill")
+                if laid.tables is not None:
+                    self._gemm(laid, qh, _lib.ACT_F16_NORM, s, out, "prefill")
                 else:
                     kb.grouped_ternary_gemm_bf16(kb.NormRows(qh, s), None, packed, scales, self.K, self.group, self.fmt, out=out,
                                                  backend=self.backend)
             else:
                 q, s = quant_act_int8(x2)
-                if self._direct is not None:
-                    self._gemm(q, _lib.ACT_I8, s, out, self.algo)
+                if laid.tables is not None:
+                    self._gemm(laid, q, _lib.ACT_I8, s, out, self.algo)
                 else:
                     kb._grouped(lib, q, s, None, packed, scales, self.K, self.group, self.fmt, out, False, self.algo)
         else:
             xa = x2 if x2.dtype in (torch.bfloat16, torch.float16) else x2.bfloat16()
             od = out_dtype if out_dtype in (torch.float32, torch.bfloat16, torch.float16) else torch.float32
-            if self._direct is not None:
+            if laid.tables is not None:
                 out = torch.empty(xa.size(0), self.out_features, dtype=od, device=xa.device)
-                self._gemm(xa, kb._ACT[xa.dtype], None, out, self.algo)
+                self._gemm(laid, xa, kb._ACT[xa.dtype], None, out, self.algo)
             else:
                 out = kb.grouped_ternary_gemm_bf16(xa, None, packed, scales, self.K, self.group, self.fmt, out_dtype=od,
                                                    algo=self.algo, backend=self.backend)

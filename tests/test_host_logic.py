@@ -324,3 +324,138 @@ def test_prefill_barrier_protocol_under_random_interleavings(seed):
     small = bool(seed & 1)
     na = rnd.choice([6, 7]) if small else rnd.choice([6, 7, 8, 9, 11])
     _prefill_roles(small, rnd.choice([4, 5]), 2 * rnd.choice([1, 1, 2, 3, 5, 8]), rnd.randint(1, 7), na, rnd.randint(2, na), rnd.choice([2, 3]), rnd)
+
+
+class _CudaLike(torch.Tensor):
+    """A CPU tensor that says it is on a GPU: takes a linear's call to the (stubbed) library."""
+
+    is_cuda = property(lambda self: True)
+    device = property(lambda self: getattr(self, "says", torch.device("cpu")))
+
+
+def _cuda_like(x, device=None):
+    x = x.as_subclass(_CudaLike)
+    if device is not None:
+        x.says = device
+        x.reshape = lambda *shape: x  # the rows as they are: a view would forget its device
+    return x
+
+
+@pytest.fixture
+def stub_library(monkeypatch):
+    """The library as a stub on the CPU: tiling makes a fresh buffer, a GEMM records the pointers it is given. Returns (calls:
+    [(thread name, [packed pointers])], tiles: {thread name: [tile buffers]}, hooks: {"tile" | "gemm": callable})."""
+    import threading
+    from contextlib import nullcontext
+
+    calls, tiles, hooks = [], {}, {}
+
+    class Lib:
+        def dst_gemm_workspace_bytes(self, *a):
+            return 0
+
+        def dst_decode_row_limit(self, *a):
+            return 16
+
+        def dst_ternary_grouped_gemm(self, *a):
+            calls.append((threading.current_thread().name, list(a[8])))
+            return 0
+
+    def tile(packed, fmt, K, decode_copy=False):
+        hooks.get("tile", lambda: None)()
+        t = kb.TiledWeights(torch.zeros(packed.numel() + 64, dtype=torch.uint8), 1, packed.size(1), K, fmt)
+        tiles.setdefault(threading.current_thread().name, []).append(t.data)
+        return t
+
+    def require(backend):
+        hooks.get("gemm", lambda: None)()
+        return Lib()
+
+    monkeypatch.setattr(kb, "tile_weights", tile)
+    monkeypatch.setattr(kb, "_require", require)
+    monkeypatch.setattr(kb, "_guard", lambda device: nullcontext())
+    monkeypatch.setattr(kb, "_stream", lambda t: 0)
+    return calls, tiles, hooks
+
+
+def _linear(cls=ops.TernaryLinear):
+    return cls([ops.PackedTerm(torch.zeros(8, 32, dtype=torch.uint8), torch.ones(8, 1).half())], 128, "tq2", 128, act="bf16")
+
+
+def _kept(lin):
+    return [p.data.data_ptr() for p in (lin._dev[1] if isinstance(lin._dev, tuple) else lin._dev.packed)]
+
+
+def _run_threads(*named):
+    import threading
+
+    threads = [threading.Thread(target=fn, name=name, daemon=True) for name, fn in named]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(20)
+        assert not t.is_alive()
+
+
+def test_linear_two_threads_in_the_first_call(stub_library):
+    """Both threads find no weights and lay them out; the first one is held up until the second one's call is over. What the
+    linear keeps and what later calls point at are then the same tensors, whoever came last."""
+    import threading
+
+    calls, tiles, hooks = stub_library
+    both_inside, first_held, second_done = threading.Barrier(2), threading.Event(), threading.Event()
+
+    class Held(ops.TernaryLinear):
+        @property
+        def out_features(self):  # read between the first thread's tiling and the end of its layout
+            if threading.current_thread().name == "first":
+                first_held.set()
+                second_done.wait(10)
+            return super().out_features
+
+    lin, x = _linear(Held), _cuda_like(torch.zeros(4, 128).bfloat16())
+
+    def tile_hook():
+        if threading.current_thread().name in ("first", "second"):
+            both_inside.wait(10)
+        if threading.current_thread().name == "second":
+            first_held.wait(10)
+
+    hooks["tile"] = tile_hook
+
+    def second():
+        lin(x)
+        second_done.set()
+
+    _run_threads(("first", lambda: lin(x)), ("second", second))
+    by_thread = {n: p for n, p in calls}
+    assert by_thread["first"] == [tiles["first"][0].data_ptr()] and by_thread["second"] == [tiles["second"][0].data_ptr()]
+    calls.clear()
+    lin(x)
+    assert calls[0][1] == _kept(lin)
+
+
+def test_linear_threads_on_two_devices(stub_library):
+    """One linear used from two threads on two devices: a launch gets the pointers of its own device's weights although the
+    other thread lays out its own between this thread's layout and its launch."""
+    import threading
+
+    calls, tiles, hooks = stub_library
+    lin = _linear()
+    a_ready, b_done = threading.Event(), threading.Event()
+
+    def gemm_hook():
+        if threading.current_thread().name == "a":
+            a_ready.set()
+            b_done.wait(10)
+
+    hooks["gemm"] = gemm_hook
+
+    def b():
+        a_ready.wait(10)
+        lin(_cuda_like(torch.zeros(4, 128).bfloat16(), torch.device("cpu", 0)))
+        b_done.set()
+
+    _run_threads(("a", lambda: lin(_cuda_like(torch.zeros(4, 128).bfloat16()))), ("b", b))
+    by_thread = {n: p for n, p in calls}
+    assert by_thread["a"] == [tiles["a"][0].data_ptr()] and by_thread["b"] == [tiles["b"][0].data_ptr()]
