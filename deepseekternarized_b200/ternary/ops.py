@@ -55,6 +55,7 @@ class _Layout:
 
     def __init__(self, device, packed: list, scales: list, N: int, K: int, group: int):
         self.device, self.packed, self.scales = device, packed, scales
+        self.sizes = N, K, group
         n = len(packed)
         self.tables = None
         if 1 <= n <= _lib.MAX_TERMS and all(isinstance(p, kb.TiledWeights) and p.E == 1 and p.N == N for p in packed) \
@@ -63,6 +64,10 @@ class _Layout:
             copies = [p.decode for p in packed] if packed[0].fmt == "tq1" else [None]
             dec = table(*[c.data.data_ptr() for c in copies]) if all(c is not None for c in copies) else None
             self.tables = table(*[p.data.data_ptr() for p in packed]), dec, table(*[s.data_ptr() for s in scales])
+
+    def __reduce__(self):
+        # copy and pickle take the tensors; the copy's tables are made anew from the copied tensors
+        return _Layout, (self.device, self.packed, self.scales, *self.sizes)
 
 
 class TernaryLinear:
@@ -86,6 +91,11 @@ class TernaryLinear:
         self.backend, self.algo = backend, algo
         self.decode_copy = decode_copy  # TQ1: keep a tiled TQ2 copy of the trits on the device for few-row calls
         self._dev = None  # the _Layout in use, replaced as a whole
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        if not isinstance(self._dev, _Layout):  # saved with its device weights as a plain tuple: laid out again at the next call
+            self._dev = None
 
     def _layout(self, device) -> "_Layout":
         """The weights on ``device``, copied once and kept. Shapes the fast kernels cover (group 128, K % 128 == 0, fp16

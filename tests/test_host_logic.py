@@ -459,3 +459,24 @@ def test_linear_threads_on_two_devices(stub_library):
     _run_threads(("a", lambda: lin(_cuda_like(torch.zeros(4, 128).bfloat16()))), ("b", b))
     by_thread = {n: p for n, p in calls}
     assert by_thread["a"] == [tiles["a"][0].data_ptr()] and by_thread["b"] == [tiles["b"][0].data_ptr()]
+
+
+@pytest.mark.parametrize("copies", ["deepcopy", "pickle"])
+def test_linear_copies_after_a_call(stub_library, copies):
+    """A linear that has laid out its weights can be copied and pickled; the copy's calls point at the copy's own tensors, and
+    one saved with the device weights as the plain (device, tiles, scales) tuple of earlier versions still loads."""
+    import copy
+    import pickle
+
+    calls, _, _ = stub_library
+    lin, x = _linear(), _cuda_like(torch.zeros(4, 128).bfloat16())
+    lin(x)
+    other = copy.deepcopy(lin) if copies == "deepcopy" else pickle.loads(pickle.dumps(lin))
+    other(x)
+    assert calls[1][1] == _kept(other) and calls[1][1] != calls[0][1]
+    lin(x)
+    assert calls[2][1] == calls[0][1] == _kept(lin)
+    old = ops.TernaryLinear.__new__(ops.TernaryLinear)
+    old.__setstate__({**lin.__dict__, "_dev": (torch.device("cpu"), lin._dev.packed, lin._dev.scales)})
+    old(x)
+    assert calls[3][1] == _kept(old)
