@@ -82,6 +82,7 @@ bool decode_tq1_supports(const GemmArgs& a);
 bool prefill_supports(const GemmArgs& a);
 // SwiGLU of gate / up rows straight into the decode GEMV's quantised form (in `workspace`, as launch_decode lays it out for T
 // rows of K = inter); standard: the OLMoE rounding points, no weight, no clamp
+bool decode_swiglu_quant_supports(int64_t inter);
 int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const int64_t* order, int64_t T, int64_t inter, float limit,
                         bool standard, void* workspace, cudaStream_t stream);
 int decode_take_status(int* status);

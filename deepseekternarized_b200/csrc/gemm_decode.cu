@@ -851,10 +851,14 @@ size_t decode_workspace_bytes(int64_t T, int64_t K) {
   return up256((size_t)T * 2 * (size_t)K) + up256((size_t)T * (size_t)(K / 128) * 4) + up256((size_t)T * 4);
 }
 
+// A row is kept in shared memory (2 bytes per element): every row length that the decode GEMV takes (25 088 at most)
+constexpr int64_t DC_SWIGLU_MAX = 32768;
+bool decode_swiglu_quant_supports(int64_t inter) { return inter % 128 == 0 && inter <= DC_SWIGLU_MAX; }
+
 int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const int64_t* order, int64_t T, int64_t inter, float limit,
                         bool standard, void* workspace, cudaStream_t stream) {
-  if (inter % 128 != 0 || inter > 16384 || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0 || (reinterpret_cast<uintptr_t>(gu_bf16) & 3) != 0)
-    return DST_ERR_UNSUPPORTED;  // a row is kept in 32 KB of shared memory at most
+  if (!decode_swiglu_quant_supports(inter) || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0 || (reinterpret_cast<uintptr_t>(gu_bf16) & 3) != 0)
+    return DST_ERR_UNSUPPORTED;
   DecodeParams p;
   memset(&p, 0, sizeof(p));
   p.T = (int)T;
@@ -863,6 +867,10 @@ int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const i
   const QuantRows q(workspace, T, inter);
   auto gu = static_cast<const __nv_bfloat16*>(gu_bf16);
   const size_t smem = (size_t)inter * 2;
+  if (smem + 1024 > 48 * 1024) {  // with the static part above what a launch gets unasked
+    DST_CUDA_TRY(cudaFuncSetAttribute(decode_swiglu_quant_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DST_CUDA_TRY(cudaFuncSetAttribute(decode_swiglu_quant_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  }
   if (standard) decode_swiglu_quant_kernel<true><<<(unsigned)T, DC_QWARPS * 32, smem, stream>>>(p, gu, nullptr, nullptr, 0.f, q.rows, q.xsum4, q.xexp);
   else decode_swiglu_quant_kernel<false><<<(unsigned)T, DC_QWARPS * 32, smem, stream>>>(p, gu, route_weights, order, limit, q.rows, q.xsum4, q.xexp);
   DST_CUDA_TRY(cudaGetLastError());

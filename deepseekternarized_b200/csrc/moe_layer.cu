@@ -66,6 +66,11 @@ Gemm make_gemm(const dst_expert_weights& w, bool second, int64_t n, const int64_
   }
   a.act_dtype = DST_ACT_BF16;
   if (few && decode_supports(a)) {
+    // the second GEMV's rows come quantised from decode_swiglu_quant: a row length it does not take is not covered here
+    if (second && a.fmt == DST_FMT_TQ2 && !decode_swiglu_quant_supports(a.K)) {
+      g.path = PATH_NONE;
+      return g;
+    }
     g.path = a.fmt == DST_FMT_TQ2 ? PATH_DECODE : PATH_DECODE_TQ1;
   } else {
     static const float one = 1.f;  // any non-null pointer: only asked whether the shape is covered

@@ -621,6 +621,40 @@ def test_moe_layer_in_one_call_equals_its_steps(fmt, k_terms, copy, flavour):
         assert torch.equal(one.forward_routed(x, wts, wide), steps.forward_routed(x, wts, wide))
 
 
+def _random_experts(n, hidden, inter, fmt, seed, k_terms=1, copy=False):
+    """Random prepared ``ExpertWeights``, packed on the GPU."""
+    from deepseekternarized_b200.moe import ExpertWeights
+    from deepseekternarized_b200.ternary.pack import pack
+
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    packed, scale = {}, {}
+    for k, (rows, K) in {"w13": (2 * inter, hidden), "w2": (hidden, inter)}.items():
+        packed[k] = [pack(torch.randint(-1, 2, (n * rows, K), generator=gen, device=DEV, dtype=torch.int8), fmt).view(n, rows, -1) for _ in range(k_terms)]
+        scale[k] = [(torch.rand(n, rows, K // 128, generator=gen, device=DEV) * 0.02 + 0.005).half() for _ in range(k_terms)]
+    return ExpertWeights(packed["w13"], scale["w13"], packed["w2"], scale["w2"], hidden, inter, 128, fmt).prepare(decode_copy=copy)
+
+
+@pytest.mark.parametrize("fmt,copy", [("tq2", False), ("tq1", True), ("tq1", False)])
+@pytest.mark.parametrize("inter", [16384, 16896, 18432, 24576, 25088, 25600])
+def test_moe_layer_in_one_call_wide_experts(fmt, copy, inter):
+    """Intermediate sizes up to and beyond the longest row that the decode GEMV takes (25 088), a decode-sized step, routed and
+    as the shared expert: the call gives what the single steps give, bit for bit."""
+    from deepseekternarized_b200.moe import B200Ops, MoELayer
+
+    class Steps(B200Ops):
+        pass
+
+    if copy and inter > 25088:
+        pytest.skip("the single steps read a decode copy with the GEMV only")
+    hidden, T = 512, 3
+    w, shared = _random_experts(4, hidden, inter, fmt, 1, copy=copy), _random_experts(1, hidden, inter, fmt, 2, copy=copy)
+    gen = torch.Generator(device=DEV).manual_seed(inter)
+    x, logits = torch.randn(T, hidden, generator=gen, device=DEV).bfloat16(), torch.randn(T, 4, generator=gen, device=DEV)
+    for kw in ({"shared": shared}, {"flavour": "standard"}):
+        y = MoELayer(w, 2, **kw)(x, logits)
+        assert torch.equal(y, MoELayer(w, 2, ops=Steps(), **kw)(x, logits)) and bool(y.isfinite().all()) and float(y.float().abs().max()) > 0
+
+
 @pytest.mark.parametrize("n,E", [(1, 1), (31, 5), (1023, 384), (1024, 4096), (1025, 384), (5000, 4096), (3000, 1)])
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
 def test_sort_edges(kb, n, E, dtype):
