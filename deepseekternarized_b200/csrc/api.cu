@@ -116,8 +116,7 @@ static int grouped_gemm(void* out, int out_dtype, int accumulate, const void* x,
   }
   if (act_dtype == DST_ACT_F16_NORM) return launch_prefill(a, st);  // only the tcgen05 kernel reads this format
   // AUTO: few rows per expert -> decode GEMV; many -> tcgen05 grouped GEMM; otherwise generic.
-  const int64_t avg_rows = a.max_rows >= 0 ? a.max_rows : cdiv64(T, E);
-  if (avg_rows <= decode_auto_rows(fmt, n_terms, E, T, N) && decode_supports(a)) return launch_decode(a, st);
+  if (auto_takes_decode(a)) return launch_decode(a, st);
   if (prefill_supports(a)) return launch_prefill(a, st);
   if (decode_supports(a)) return launch_decode(a, st);
   if (weight_layout == DST_LAYOUT_TILED) return DST_ERR_UNSUPPORTED;

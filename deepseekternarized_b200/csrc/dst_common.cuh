@@ -77,9 +77,11 @@ int launch_prefill(const GemmArgs& a, cudaStream_t stream);   // DST_ERR_UNSUPPO
 bool decode_supports(const GemmArgs& a);
 int64_t decode_row_limit(int fmt, int64_t E, int64_t N);
 int64_t decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N);  // rows per expert up to which AUTO prefers the decode GEMV
+bool auto_takes_decode(const GemmArgs& a);  // AUTO's choice for this call: the decode GEMV (which then covers it)
 int launch_decode_tq1(const GemmArgs& a, cudaStream_t stream);  // TQ1 decode kernel (gemm_decode_tq1.cu); reached through launch_decode
 bool decode_tq1_supports(const GemmArgs& a);
 bool prefill_supports(const GemmArgs& a);
+bool prefill_aligned(const GemmArgs& a);  // the alignments that launch_prefill asks for, else DST_ERR_ALIGNMENT
 // SwiGLU of gate / up rows straight into the decode GEMV's quantised form (in `workspace`, as launch_decode lays it out for T
 // rows of K = inter); standard: the OLMoE rounding points, no weight, no clamp
 bool decode_swiglu_quant_supports(int64_t inter);

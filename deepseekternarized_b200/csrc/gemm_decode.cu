@@ -897,6 +897,14 @@ int64_t decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N) 
   return E > 1 && T * ((N + 255) / 256) <= sm_count() ? 8 : 0;
 }
 
+// The choice itself. A call whose tensors the tcgen05 kernel does not take as they lie in memory (scales that are a view at an
+// odd offset, say) keeps the GEMV up to its own limit.
+bool auto_takes_decode(const GemmArgs& a) {
+  const int64_t rows = a.max_rows >= 0 ? a.max_rows : cdiv64(a.T, a.E);
+  const int64_t limit = prefill_aligned(a) ? decode_auto_rows(a.fmt, a.terms.n, a.E, a.T, a.N) : decode_row_limit(a.fmt, a.E, a.N);
+  return rows <= limit && decode_supports(a);
+}
+
 bool decode_supports(const GemmArgs& a) {
   if (a.fmt == DST_FMT_TQ1) return decode_tq1_supports(a);
   return a.weight_layout == DST_LAYOUT_TILED && a.fmt == DST_FMT_TQ2 && a.group == 128 && a.K % 512 == 0 &&

@@ -1280,15 +1280,20 @@ bool prefill_supports(const GemmArgs& a) {
          a.N <= (int64_t(1) << 22) && encode_fn() != nullptr;
 }
 
+bool prefill_aligned(const GemmArgs& a) {
+  const bool prenorm = a.act_dtype == DST_ACT_F16_NORM;
+  if (!prenorm && (reinterpret_cast<uintptr_t>(a.workspace) & 255) != 0) return false;
+  if (prenorm && (reinterpret_cast<uintptr_t>(a.x) & 15) != 0) return false;
+  for (int i = 0; i < a.terms.n; ++i)
+    if ((reinterpret_cast<uintptr_t>(a.terms.packed[i]) & 15) != 0 || (reinterpret_cast<uintptr_t>(a.terms.scale[i]) & 15) != 0) return false;
+  return true;
+}
+
 int launch_prefill(const GemmArgs& a, cudaStream_t stream) {
   if (a.T == 0 || a.N == 0 || a.E == 0) return DST_OK;
   if (!prefill_supports(a)) return DST_ERR_UNSUPPORTED;
+  if (!prefill_aligned(a)) return DST_ERR_ALIGNMENT;
   const bool prenorm = a.act_dtype == DST_ACT_F16_NORM;
-  if (!prenorm && (reinterpret_cast<uintptr_t>(a.workspace) & 255) != 0) return DST_ERR_ALIGNMENT;
-  if (prenorm && (reinterpret_cast<uintptr_t>(a.x) & 15) != 0) return DST_ERR_ALIGNMENT;
-  for (int i = 0; i < a.terms.n; ++i)
-    if ((reinterpret_cast<uintptr_t>(a.terms.packed[i]) & 15) != 0 || (reinterpret_cast<uintptr_t>(a.terms.scale[i]) & 15) != 0)
-      return DST_ERR_ALIGNMENT;
 
   // 1. activations -> fp16 rows + per-row power-of-two factor, in the workspace
   //    (skipped when the caller hands in rows that are in that format already)

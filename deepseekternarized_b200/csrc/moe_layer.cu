@@ -51,11 +51,7 @@ Gemm make_gemm(const dst_expert_weights& w, bool second, int64_t n, const int64_
   a.weight_layout = DST_LAYOUT_TILED;
   a.out_dtype = DST_OUT_BF16;
   // the 2-bit decode copy takes the place of TQ1 weights by the rule of TQ2 tiles
-  const int64_t mean = cdiv64(n, a.E);
-  const bool copy = w.fmt == DST_FMT_TQ1 && dec[0] != nullptr;
-  const int few_fmt = copy ? DST_FMT_TQ2 : w.fmt;
-  const bool few = mean <= decode_auto_rows(few_fmt, w.n_terms, a.E, n, a.N);
-  if (few && copy) {
+  if (w.fmt == DST_FMT_TQ1 && dec[0] != nullptr && cdiv64(n, a.E) <= decode_row_limit(DST_FMT_TQ2, a.E, a.N)) {
     a.fmt = DST_FMT_TQ2;
     packed = dec;
   }
@@ -65,7 +61,7 @@ Gemm make_gemm(const dst_expert_weights& w, bool second, int64_t n, const int64_
     a.terms.scale[i] = scale[i];
   }
   a.act_dtype = DST_ACT_BF16;
-  if (few && decode_supports(a)) {
+  if (auto_takes_decode(a)) {
     // the second GEMV's rows come quantised from decode_swiglu_quant: a row length it does not take is not covered here
     if (second && a.fmt == DST_FMT_TQ2 && !decode_swiglu_quant_supports(a.K)) {
       g.path = PATH_NONE;

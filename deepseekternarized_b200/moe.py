@@ -286,7 +286,7 @@ class MoELayer:
         order, offsets = self.ops.sort(ids, w.n_experts)
         xs = self.gather_for_experts(x, order, self.top_k)
         gu = self.ops.gemm(xs, offsets, w.w13_packed, w.w13_scale, w.hidden, w.group, w.fmt)
-        h = self.ops.swiglu_std(gu, w.inter, for_weights=w.w2_packed)
+        h = self.ops.swiglu_std(gu, w.inter, for_weights=self._for_weights(w.w2_packed, w.w2_scale))
         down = self.ops.gemm(h, offsets, w.w2_packed, w.w2_scale, w.inter, w.group, w.fmt)
         return self.ops.combine_weighted(down, order, ids, weights, T, self.top_k)
 
@@ -306,7 +306,7 @@ class MoELayer:
                 self.ops.gemm_scatter(h, offsets, w.w2_packed, w.w2_scale, w.inter, w.group, w.fmt, *scatter)
                 return None
         elif getattr(self.ops, "fused_norm", False):
-            h = self.ops.swiglu(gu, row_weights, order, w.inter, self.swiglu_limit, for_weights=w.w2_packed)
+            h = self.ops.swiglu(gu, row_weights, order, w.inter, self.swiglu_limit, for_weights=self._for_weights(w.w2_packed, w.w2_scale))
         else:
             h = self.ops.swiglu(gu, row_weights, order, w.inter, self.swiglu_limit)
         if out is None:
@@ -317,8 +317,14 @@ class MoELayer:
         """Rows in expert-sorted order, in the format the first expert GEMM reads fastest."""
         w = self.w if weights is None else weights
         if getattr(self.ops, "fused_norm", False):
-            return self.ops.gather(x, order, top_k, for_weights=w.w13_packed)
+            return self.ops.gather(x, order, top_k, for_weights=self._for_weights(w.w13_packed, w.w13_scale))
         return self.ops.gather(x, order, top_k)
+
+    @staticmethod
+    def _for_weights(packed, scales):
+        """The weights that gather and SwiGLU prepare their rows for, or None (bf16 rows) where the scales are not aligned as
+        the tcgen05 kernel reads them (16 bytes): only the decode GEMV takes such a call, and it reads bf16 rows."""
+        return None if any(s.is_cuda and s.data_ptr() & 15 for s in scales) else packed
 
     def shared_forward(self, x: torch.Tensor):
         """``swiglu(L.shared, x)`` of boilerplate/engine/model.py:421 as bf16 rows [T, hidden] (None without a shared

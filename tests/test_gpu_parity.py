@@ -6,6 +6,7 @@ quantisation; for GEMM outputs the north-star tolerance (relative Frobenius erro
 
 from __future__ import annotations
 
+import ctypes
 import os
 
 import numpy as np
@@ -653,6 +654,64 @@ def test_moe_layer_in_one_call_wide_experts(fmt, copy, inter):
     for kw in ({"shared": shared}, {"flavour": "standard"}):
         y = MoELayer(w, 2, **kw)(x, logits)
         assert torch.equal(y, MoELayer(w, 2, ops=Steps(), **kw)(x, logits)) and bool(y.isfinite().all()) and float(y.float().abs().max()) > 0
+
+
+def _shifted(t, elements=1):
+    """The same values as a contiguous view that starts ``elements`` after an allocation's start."""
+    buf = torch.empty(t.numel() + elements, dtype=t.dtype, device=t.device)
+    buf[elements:] = t.reshape(-1)
+    return buf[elements:].view(t.shape)
+
+
+@pytest.mark.parametrize("E,T", [(1, 1), (1, 4), (1, 16), (6, 7), (6, 60)])
+def test_few_row_tq1_calls_with_unaligned_scales(kb, E, T):
+    """Few rows through one TQ1 term whose scales start on 2 bytes: the tcgen05 kernel, AUTO's choice, does not take them, the
+    GEMV does, so AUTO takes the GEMV; many rows are refused by either. The same for a workspace off its 256 bytes."""
+    N, K = 300, 512
+    rng = np.random.default_rng(T)
+    (p, s), = make_terms(rng, N, K, 128, "tq1", 1, lead=(E,))
+    offsets = np.linspace(0, T, E + 1).astype(np.int64)
+    x = bf16_tensor(O.synth_acts(rng, (T, K)), DEV)
+    w, sc = kb.tile_weights(torch.from_numpy(p).to(DEV), "tq1", K), torch.from_numpy(s).to(DEV)
+    run = lambda rows, offs, scales, algo: kb.grouped_ternary_gemm_bf16(rows, offs, [w], [scales], K, 128, "tq1", algo=algo)  # noqa: E731
+    got, want = run(x, offsets, _shifted(sc), "auto"), run(x, offsets, sc, "decode")
+    assert torch.equal(got, want)
+    many = torch.zeros(E * 40, K, dtype=torch.bfloat16, device=DEV)
+    for algo, rows, offs in (("auto", many, np.arange(E + 1) * 40), ("prefill", x, offsets)):
+        with pytest.raises(RuntimeError):
+            run(rows, offs, _shifted(sc), algo)
+    lib, out = kb.ext(), torch.empty(T, N, device=DEV)
+    ws = _shifted(torch.empty(int(lib.dst_gemm_workspace_bytes(0, 0, T, K)), dtype=torch.uint8, device=DEV), 16)
+    table = ctypes.c_void_p * 1
+    offs = torch.from_numpy(offsets).to(DEV)
+    assert lib.dst_ternary_grouped_gemm(out.data_ptr(), 0, 0, x.data_ptr(), 0, None, offs.data_ptr(), None, table(w.data.data_ptr()), 1,
+                                        table(sc.data_ptr()), 1, 0, E, T, N, K, 128, 1, 0, ws.data_ptr(), ws.numel(), None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("flavour", ["v4", "standard"])
+def test_moe_layer_with_unaligned_scales(flavour):
+    """The same through a TQ1 layer, in one call and by its steps: a decode-sized step works, a larger one is refused."""
+    from deepseekternarized_b200.moe import B200Ops, MoELayer
+
+    class Steps(B200Ops):
+        pass
+
+    w = _random_experts(40, 512, 512, "tq1", 3)
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    x, logits = torch.randn(900, 512, generator=gen, device=DEV).bfloat16(), torch.randn(900, 40, generator=gen, device=DEV)
+    want = MoELayer(w, 3, flavour=flavour)(x[:100], logits[:100]).double()
+    w.w13_scale, w.w2_scale = [_shifted(s) for s in w.w13_scale], [_shifted(s) for s in w.w2_scale]
+    one, steps = MoELayer(w, 3, flavour=flavour), MoELayer(w, 3, flavour=flavour, ops=Steps())
+    for T in (1, 100):
+        y = one(x[:T], logits[:T])
+        assert torch.equal(y, steps(x[:T], logits[:T]))
+        # the kernels sum in another order, which bf16 roundings after each linear carry on: 2^-9 each, three of them
+        assert float((y.double() - want[:T]).norm() / want[:T].norm()) < 6e-3
+    for layer in (one, steps):
+        with pytest.raises(RuntimeError):
+            layer(x, logits)
 
 
 @pytest.mark.parametrize("n,E", [(1, 1), (31, 5), (1023, 384), (1024, 4096), (1025, 384), (5000, 4096), (3000, 1)])
