@@ -163,8 +163,10 @@ bool weights_ok(const dst_expert_weights* w) {
   if (w->n_terms < 1 || w->n_terms > DST_MAX_TERMS || (w->fmt != DST_FMT_TQ1 && w->fmt != DST_FMT_TQ2) || w->experts < 1 || w->hidden < 1 ||
       w->inter < 1)
     return false;
-  for (int i = 0; i < w->n_terms; ++i)
+  for (int i = 0; i < w->n_terms; ++i) {
     if (!w->w13[i] || !w->s13[i] || !w->w2[i] || !w->s2[i]) return false;
+    if (!w->w13_decode[i] != !w->w13_decode[0] || !w->w2_decode[i] != !w->w2_decode[0]) return false;  // all terms or none
+  }
   return true;
 }
 

@@ -341,9 +341,10 @@ class MoELayer:
         if w.group != 128 or not 1 <= n <= _lib.MAX_TERMS or not len(w.w13_scale) == len(w.w2_packed) == len(w.w2_scale) == n:
             return None
         c = _lib.ExpertWeightsC(experts=E, hidden=H, inter=I, n_terms=n, fmt=kb._fmt_code(w.fmt))
-        copies = w.fmt == "tq1" and all(getattr(p, "decode", None) is not None for ps in (w.w13_packed, w.w2_packed) for p in ps)
         for packed, scales, N, K, to, to_scale, to_decode in ((w.w13_packed, w.w13_scale, 2 * I, H, c.w13, c.s13, c.w13_decode),
                                                               (w.w2_packed, w.w2_scale, H, I, c.w2, c.s2, c.w2_decode)):
+            # a matrix has copies or not by its own K (tile_weights), the other one's do not count
+            copies = w.fmt == "tq1" and all(getattr(p, "decode", None) is not None for p in packed)
             for i in range(n):
                 p, s = packed[i], scales[i]
                 if not (isinstance(p, kb.TiledWeights) and p.E == E and p.N == N and p.K == K and p.fmt == w.fmt and p.data.device == device

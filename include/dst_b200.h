@@ -254,7 +254,7 @@ int dst_combine(const void* down_bf16, const int64_t* order, const int32_t* ids,
  * of 128; anything else is DST_ERR_UNSUPPORTED (dst_moe_layer_workspace_bytes then returns 0).
  *   x [T, hidden] bf16, weights [T, top_k] f32, ids [T, top_k] int32 (an id outside [0, experts) drops that slot)
  *   w13, s13     per term: [experts, 2 inter, ...] tiled weights and scales; w2, s2 [experts, hidden, ...]
- *   w13_decode, w2_decode   optional: the trits of TQ1 weights once more as tiled TQ2 (all terms or none)
+ *   w13_decode, w2_decode   optional, each by itself: the trits of TQ1 weights once more as tiled TQ2 (all terms or none)
  *   workspace    256-byte aligned, dst_moe_layer_workspace_bytes bytes */
 typedef struct dst_expert_weights {
   const void* w13[DST_MAX_TERMS];

@@ -121,3 +121,29 @@ def test_other_entries_reject_bad_arguments(lib):
     assert lib.dst_decode_row_limit(1, 384, 4096) == 16 and lib.dst_decode_row_limit(2, 1, 4096) == 16
     assert lib.dst_gemm_workspace_bytes(_lib.ALGO_GENERIC, 0, 100, 4096) == 0
     assert lib.dst_gemm_workspace_bytes(_lib.ALGO_PREFILL, 0, 100, 4096) >= 100 * 4096 * 2 + 400
+
+
+def test_moe_layer_decode_copies(lib):
+    """Each of a layer's two matrices has its 2-bit decode copies or not by itself, with all its terms or none."""
+    import torch
+
+    from deepseekternarized_b200.kernels import ternary_b200 as kb
+    from deepseekternarized_b200.moe import ExpertWeights, MoELayer
+
+    def weights(E, N, K, copy):
+        new = lambda fmt: kb.TiledWeights(torch.zeros(64, dtype=torch.uint8), E, N, K, fmt)  # noqa: E731
+        packed = [new("tq1"), new("tq1")]
+        for p in packed:
+            p.decode = new("tq2") if copy else None
+        return packed, [torch.zeros(E, N, K // 128, dtype=torch.float16) for _ in packed]
+
+    hidden, inter, E = 2048, 1024, 4
+    for first, second in ((True, False), (False, True), (True, True), (False, False)):
+        w13, s13 = weights(E, 2 * inter, hidden, first)
+        w2, s2 = weights(E, hidden, inter, second)
+        c = MoELayer._c_weights(ExpertWeights(w13, s13, w2, s2, hidden, inter, 128, "tq1"), torch.device("cpu"))
+        assert [c.w13_decode[i] for i in range(2)] == [p.decode.data.data_ptr() if first else None for p in w13]
+        assert [c.w2_decode[i] for i in range(2)] == [p.decode.data.data_ptr() if second else None for p in w2]
+        assert lib.dst_moe_layer_workspace_bytes(2, 2, 0, ctypes.byref(c), None) > 0
+    c.w13_decode[0] = 0x1000  # one of two terms
+    assert lib.dst_moe_layer_workspace_bytes(2, 2, 0, ctypes.byref(c), None) == 0

@@ -656,6 +656,23 @@ def test_moe_layer_in_one_call_wide_experts(fmt, copy, inter):
         assert torch.equal(y, MoELayer(w, 2, ops=Steps(), **kw)(x, logits)) and bool(y.isfinite().all()) and float(y.float().abs().max()) > 0
 
 
+@pytest.mark.parametrize("hidden,inter", [(2048, 768), (768, 2048)])
+def test_moe_layer_in_one_call_with_one_matrix_decode_copy(hidden, inter):
+    """TQ1 with 2-bit copies where only one of the two matrices can have one (K a multiple of 512): the call takes the copy as
+    the single steps do, bit for bit."""
+    from deepseekternarized_b200.moe import B200Ops, MoELayer
+
+    class Steps(B200Ops):
+        pass
+
+    w, shared = (_random_experts(n, hidden, inter, "tq1", n, copy=True) for n in (16, 1))
+    assert (w.w13_packed[0].decode is None) != (w.w2_packed[0].decode is None)
+    gen = torch.Generator(device=DEV).manual_seed(inter)
+    for T in (1, 5, 60, 300):
+        x, logits = torch.randn(T, hidden, generator=gen, device=DEV).bfloat16(), torch.randn(T, 16, generator=gen, device=DEV)
+        assert torch.equal(MoELayer(w, 4, shared=shared)(x, logits), MoELayer(w, 4, shared=shared, ops=Steps())(x, logits))
+
+
 def _shifted(t, elements=1):
     """The same values as a contiguous view that starts ``elements`` after an allocation's start."""
     buf = torch.empty(t.numel() + elements, dtype=t.dtype, device=t.device)
