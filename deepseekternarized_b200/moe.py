@@ -357,8 +357,11 @@ class MoELayer:
 
     def _layer_call(self, x: torch.Tensor, weights: torch.Tensor, ids: torch.Tensor):
         """The layer by one call into the library (``dst_moe_layer``), or None where the steps are called one by one: another
-        ops object or a forced kernel, activations that are not bf16 rows of this layer, weights or shapes it does not cover."""
+        ops object or a forced kernel, a step of the layer or of its ops object that someone replaced, activations that are not
+        bf16 rows of this layer, weights or shapes it does not cover."""
         if type(self.ops) is not B200Ops or self.ops.algo != "auto" or not self.ops.fused_norm:
+            return None
+        if _replaced(self, _LAYER_STEPS) or _replaced(self.ops, _OPS_STEPS):
             return None
         if not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or x.size(1) != self.w.hidden or not (weights.device == ids.device == x.device) \
                 or ids.dtype not in (torch.int32, torch.int64):
@@ -412,6 +415,16 @@ class MoELayer:
         return self.forward_routed(x, weights, ids)
 
     __call__ = forward
+
+
+# The steps that the one call into the library stands for: a subclass, an instance or a patch that has its own gets it called.
+_LAYER_STEPS = {n: getattr(MoELayer, n) for n in ("gather_for_experts", "experts_forward", "shared_forward", "_forward_standard")}
+_OPS_STEPS = {n: getattr(B200Ops, n) for n in ("sort", "gather", "gemm", "swiglu", "swiglu_std", "combine", "combine_weighted", "_norm_ok")}
+
+
+def _replaced(obj, steps: dict) -> bool:
+    cls, own = type(obj), vars(obj)
+    return any(n in own or getattr(cls, n) is not f for n, f in steps.items())
 
 
 def expert_owner_split(n_experts: int, world: int) -> int:

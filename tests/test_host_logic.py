@@ -361,6 +361,16 @@ def stub_library(monkeypatch):
             calls.append((threading.current_thread().name, list(a[8])))
             return 0
 
+        def dst_moe_layer_workspace_bytes(self, *a):
+            return 256
+
+        def dst_moe_layer(self, *a):
+            calls.append((threading.current_thread().name, "moe_layer"))
+            return 0
+
+        def __getattr__(self, name):  # every other entry does nothing
+            return lambda *a: 0
+
     def tile(packed, fmt, K, decode_copy=False):
         hooks.get("tile", lambda: None)()
         t = kb.TiledWeights(torch.zeros(packed.numel() + 64, dtype=torch.uint8), 1, packed.size(1), K, fmt)
@@ -480,3 +490,50 @@ def test_linear_copies_after_a_call(stub_library, copies):
     old.__setstate__({**lin.__dict__, "_dev": (torch.device("cpu"), lin._dev.packed, lin._dev.scales)})
     old(x)
     assert calls[3][1] == _kept(old)
+
+
+_V4_STEPS = ["sort", "gather", "gemm", "swiglu", "combine", "_norm_ok"]
+_STANDARD_STEPS = ["sort", "gather", "gemm", "swiglu_std", "combine_weighted", "_norm_ok"]
+
+
+@pytest.mark.parametrize("flavour,where,name", [("v4", None, None), ("standard", None, None)]
+                         + [("v4", where, n) for where in ("ops", "B200Ops") for n in _V4_STEPS]
+                         + [("standard", where, n) for where in ("ops", "B200Ops") for n in _STANDARD_STEPS]
+                         + [("v4", where, n) for where in ("layer", "subclass") for n in ("gather_for_experts", "experts_forward", "shared_forward")]
+                         + [("standard", where, n) for where in ("layer", "subclass") for n in ("gather_for_experts", "_forward_standard")])
+def test_layer_calls_replaced_steps(stub_library, monkeypatch, flavour, where, name):
+    """A layer makes one call into the library unless a step that the call stands for was replaced, on the ops object, on its
+    class, on the layer or in a subclass of it: then the replacement is called, as by the single steps."""
+    from deepseekternarized_b200 import moe as M
+
+    class Reached(Exception):
+        pass
+
+    def replacement(*a, **kw):
+        raise Reached
+
+    calls, _, _ = stub_library
+    monkeypatch.setattr(kb, "grouped_ternary_gemm_bf16", lambda x, offsets, packed, *a, **kw: torch.zeros(x.size(0), packed[0].N).bfloat16())
+    monkeypatch.setattr(kb, "sort_by_expert", lambda ids, n: (torch.zeros(ids.numel(), dtype=torch.int64), torch.zeros(n + 1, dtype=torch.int64)))
+    E, H, I, k = 4, 128, 128, 2
+
+    def weights(n):
+        tiles = lambda N, K: [kb.TiledWeights(torch.zeros(64, dtype=torch.uint8), n, N, K, "tq2")]  # noqa: E731
+        return M.ExpertWeights(tiles(2 * I, H), [torch.zeros(n, 2 * I, 1).half()], tiles(H, I), [torch.zeros(n, H, 1).half()], H, I, 128, "tq2")
+
+    cls, ops_obj = M.MoELayer, M.B200Ops()
+    if where == "subclass":
+        cls = type("Mine", (M.MoELayer,), {name: replacement})
+    if where == "B200Ops":
+        monkeypatch.setattr(M.B200Ops, name, replacement)
+    layer = cls(weights(E), k, ops=ops_obj, flavour=flavour, shared=weights(1) if flavour == "v4" else None)
+    if where in ("ops", "layer"):
+        setattr(ops_obj if where == "ops" else layer, name, replacement)
+    args = _cuda_like(torch.zeros(3, H).bfloat16()), torch.ones(3, k), torch.zeros(3, k, dtype=torch.int32)
+    if name is None:
+        layer.forward_routed(*args)
+        assert [c[1] for c in calls] == ["moe_layer"]
+    else:
+        with pytest.raises(Reached):
+            layer.forward_routed(*args)
+        assert calls == []
