@@ -156,6 +156,8 @@ _SIGNATURES = {
                                                        ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int,
                                                        ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
     "dst_check_device_status": (ctypes.c_int, [ctypes.c_void_p]),
+    "dst_debug_prefill_plan": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64,
+                                              ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p]),
     "dst_debug_prefill_timeout": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]),
 }
 

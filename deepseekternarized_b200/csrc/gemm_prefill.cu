@@ -1230,8 +1230,10 @@ size_t plan_smem(PrefillParams& p, int min_nb) {
   return 0;
 }
 
+// Chooses the token tile and places the CTA's shared memory: returns the dynamic bytes (0: not covered), p.tn_max and whether
+// it is the SMALL form.
 template <int FMT, int TERMS>
-int launch_fmt(const TmaMaps& maps, PrefillParams p, cudaStream_t st) {
+size_t plan_tiles(PrefillParams& p, bool& small_form) {
   // The token tile is as large as the experts are expected to need (up to 320 rows) as long as a B ring of four 64-K stages
   // fits: that much hides the latency of the copies behind the MMAs of a stage. Then a third packed-slab slot if there is
   // room for it.
@@ -1257,12 +1259,84 @@ int launch_fmt(const TmaMaps& maps, PrefillParams p, cudaStream_t st) {
     }
     if (best_tn != 0) tn_cap = best_tn;
   }
+  small_form = false;
   for (p.tn_max = tn_cap; p.tn_max > PF_SMALL_TN; p.tn_max -= 32)
-    if (const size_t smem = plan_smem<FMT, TERMS, false>(p, 4)) return launch_plan<FMT, TERMS, false>(maps, p, smem, st);
+    if (const size_t smem = plan_smem<FMT, TERMS, false>(p, 4)) return smem;
+  small_form = true;
   for (; p.tn_max >= 64; p.tn_max -= 32)
-    if (const size_t smem = plan_smem<FMT, TERMS, true>(p, 2)) return launch_plan<FMT, TERMS, true>(maps, p, smem, st);
-  return DST_ERR_UNSUPPORTED;
+    if (const size_t smem = plan_smem<FMT, TERMS, true>(p, 2)) return smem;
+  return 0;
 }
+size_t plan_tiles(int fmt, PrefillParams& p, bool& small_form) {
+  if (fmt == DST_FMT_TQ2)
+    return p.n_terms == 1 ? plan_tiles<2, 1>(p, small_form) : p.n_terms == 2 ? plan_tiles<2, 2>(p, small_form) : plan_tiles<2, 4>(p, small_form);
+  return p.n_terms == 1 ? plan_tiles<1, 1>(p, small_form) : p.n_terms == 2 ? plan_tiles<1, 2>(p, small_form) : plan_tiles<1, 4>(p, small_form);
+}
+
+// Tensor maps over the fp16 rows: [T, K], boxes of 64 K-elements x 16 i token rows, 128-byte swizzle, zero fill outside. One
+// for every box height that the kernel can choose: the rows of a tile come from the offsets on the device, of which only
+// the tile's size is certain here (the caller's host copy may differ).
+int map_heights(int tn_max) { return (tn_max < 256 ? tn_max : 256) / 16; }
+int encode_maps(TmaMaps& maps, const __half* rows, int64_t T, int64_t K, int heights) {
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)T};
+  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  const cuuint32_t estr[2] = {1, 1};
+  for (int i = 0; i < heights; ++i) {
+    const cuuint32_t box[2] = {64, (cuuint32_t)(16 * (i + 1))};
+    const CUresult cr = encode_fn()(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(rows), dims, strides, box, estr,
+                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return record_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
+  }
+  return DST_OK;
+}
+
+template <int FMT, int TERMS>
+int launch_form(const TmaMaps& maps, const PrefillParams& p, bool small_form, size_t smem, cudaStream_t st) {
+  return small_form ? launch_plan<FMT, TERMS, true>(maps, p, smem, st) : launch_plan<FMT, TERMS, false>(maps, p, smem, st);
+}
+int launch_run(int fmt, const __half* rows, PrefillParams& p, cudaStream_t st) {
+  bool small_form = false;
+  const size_t smem = plan_tiles(fmt, p, small_form);
+  if (smem == 0) return DST_ERR_UNSUPPORTED;
+  TmaMaps maps;
+  const int rc = encode_maps(maps, rows, p.T, p.K, map_heights(p.tn_max));
+  if (rc != DST_OK) return rc;
+  if (fmt == DST_FMT_TQ2)
+    return p.n_terms == 1   ? launch_form<2, 1>(maps, p, small_form, smem, st)
+           : p.n_terms == 2 ? launch_form<2, 2>(maps, p, small_form, smem, st)
+                            : launch_form<2, 4>(maps, p, small_form, smem, st);
+  return p.n_terms == 1   ? launch_form<1, 1>(maps, p, small_form, smem, st)
+         : p.n_terms == 2 ? launch_form<1, 2>(maps, p, small_form, smem, st)
+                          : launch_form<1, 4>(maps, p, small_form, smem, st);
+}
+
+// The sizes of a launch: everything that plan_tiles looks at but the experts of the run (p.E)
+void size_params(const GemmArgs& a, PrefillParams& p) {
+  p.n_terms = a.terms.n;
+  p.row_target = a.row_target;
+  // 128-bit stores from the epilogue: two-byte outputs, whole 8-column pieces, 16-byte aligned rows
+  p.wide_drain = (a.out_dtype != DST_OUT_F32 && !a.accumulate && a.N % 8 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) ? 1 : 0;
+  if (a.row_target != nullptr)
+    for (int i = 0; i < DST_MAX_PEERS; ++i)
+      if ((reinterpret_cast<uintptr_t>(a.peer_out[i]) & 15) != 0) p.wide_drain = 0;
+  p.T = (int)a.T;
+  p.N = (int)a.N;
+  p.K = (int)a.K;
+  p.G = (int)a.G;
+  p.NT = (int)cdiv64(a.N, 128);
+  p.S = (int)tiled_superblocks(a.fmt, a.K);
+  p.kstages = (int)(a.K / 64);
+  // Rows per expert: known when the caller passed host offsets, else three standard deviations of an even routing above the
+  // mean (an expert with more is split into two tiles, which dequantises its weights twice; a tile sized for twice the mean
+  // costs every expert the form of the kernel for larger tiles: 96 rows on 96 experts of 4096 x 4096, TQ1, 428 against
+  // 596 us)
+  const int64_t mean = cdiv64(a.T, a.E);
+  p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : mean + (int64_t)ceil(3.0 * sqrt((double)mean)));
+  if (p.rows_hint < 1) p.rows_hint = 1;
+}
+int run_experts_of(int64_t E, int64_t e0) { return (int)(E - e0 < PF_MAX_E ? E - e0 : PF_MAX_E); }
+
 
 }  // namespace
 
@@ -1316,74 +1390,36 @@ int launch_prefill(const GemmArgs& a, cudaStream_t stream) {
                                                                    static_cast<__half*>(a.workspace), const_cast<float*>(rs));
   DST_CUDA_TRY(cudaGetLastError());
 
-  // 2. tensor maps over the fp16 rows: [T, K], boxes of 64 K-elements x 16 i token rows, 128-byte swizzle, zero fill outside
-  TmaMaps maps;
-  const cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.T};
-  const cuuint64_t strides[1] = {(cuuint64_t)a.K * 2};
-  const cuuint32_t estr[2] = {1, 1};
-  const int heights = (int)((a.max_rows >= 0 && a.max_rows < 256 ? a.max_rows : 256) + 15) / 16;  // no tile has more rows than an expert
-  for (int i = 0; i < heights; ++i) {
-    const cuuint32_t box[2] = {64, (cuuint32_t)(16 * (i + 1))};
-    const CUresult cr = encode_fn()(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(xh), dims, strides, box, estr,
-                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return record_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
-  }
-
+  // 2. one launch per run of experts
   PrefillParams p;
   for (int i = 0; i < DST_MAX_TERMS; ++i) {
     p.tiled[i] = i < a.terms.n ? a.terms.packed[i] : nullptr;
     p.scale[i] = i < a.terms.n ? static_cast<const __half*>(a.terms.scale[i]) : nullptr;
   }
-  p.n_terms = a.terms.n;
+  size_params(a, p);
   p.row_scale = rs;
   p.offsets = a.offsets;
   p.out = a.out;
   p.out_dtype = a.out_dtype;
   p.accumulate = a.accumulate;
-  p.row_target = a.row_target;
   for (int i = 0; i < DST_MAX_PEERS; ++i) p.peer_out[i] = a.peer_out[i];
   p.n_peer_out = a.n_peer_out;
   p.peer_rows = a.peer_rows;
-  // 128-bit stores from the epilogue: two-byte outputs, whole 8-column pieces, 16-byte aligned rows
-  p.wide_drain = (a.out_dtype != DST_OUT_F32 && !a.accumulate && a.N % 8 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0) ? 1 : 0;
-  if (a.row_target != nullptr)
-    for (int i = 0; i < DST_MAX_PEERS; ++i)
-      if ((reinterpret_cast<uintptr_t>(a.peer_out[i]) & 15) != 0) p.wide_drain = 0;
   if (a.row_target != nullptr && (a.out_dtype == DST_OUT_F32 || a.accumulate)) return DST_ERR_UNSUPPORTED;
-  p.E = (int)a.E;
-  p.T = (int)a.T;
-  p.N = (int)a.N;
-  p.K = (int)a.K;
-  p.G = (int)a.G;
-  p.NT = (int)cdiv64(a.N, 128);
-  p.S = (int)tiled_superblocks(a.fmt, a.K);
-  p.kstages = (int)(a.K / 64);
-  // Rows per expert: known when the caller passed host offsets, else three standard deviations of an even routing above the
-  // mean (an expert with more is split into two tiles, which dequantises its weights twice; a tile sized for twice the mean
-  // costs every expert the form of the kernel for larger tiles: 96 rows on 96 experts of 4096 x 4096, TQ1, 428 against
-  // 596 us)
-  const int64_t mean = cdiv64(a.T, a.E);
-  p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : mean + (int64_t)ceil(3.0 * sqrt((double)mean)));
-  if (p.rows_hint < 1) p.rows_hint = 1;
-#define DST_PF_LAUNCH(FMT_)                                                            \
-  (a.terms.n == 1 ? launch_fmt<FMT_, 1>(maps, p, stream)                               \
-                  : a.terms.n == 2 ? launch_fmt<FMT_, 2>(maps, p, stream) : launch_fmt<FMT_, 4>(maps, p, stream))
   // The kernel keeps per-expert tables in shared memory: more experts than fit there are served by one launch
   // per run of PF_MAX_E experts (offsets are absolute token rows, so only the per-expert pointers move).
   const int64_t tiled_per_expert = (int64_t)p.NT * p.S * PF_SLAB, scales_per_expert = a.N * a.G;
   for (int64_t e0 = 0; e0 < a.E; e0 += PF_MAX_E) {
-    p.E = (int)(a.E - e0 < PF_MAX_E ? a.E - e0 : PF_MAX_E);
+    p.E = run_experts_of(a.E, e0);
     p.offsets = a.offsets ? a.offsets + e0 : nullptr;
     for (int i = 0; i < a.terms.n; ++i) {
       p.tiled[i] = a.terms.packed[i] + e0 * tiled_per_expert;
       p.scale[i] = static_cast<const __half*>(a.terms.scale[i]) + e0 * scales_per_expert;
     }
-    const int rc = a.fmt == DST_FMT_TQ2 ? DST_PF_LAUNCH(2) : DST_PF_LAUNCH(1);
+    const int rc = launch_run(a.fmt, xh, p, stream);
     if (rc != DST_OK) return rc;
   }
   return DST_OK;
-#undef DST_PF_LAUNCH
 }
 
 }  // namespace dst
@@ -1413,6 +1449,35 @@ extern "C" int dst_debug_prefill_timeout(long long wait_cycles, int drop_drain_a
   DST_CUDA_TRY(cudaMemcpyToSymbol(dst::g_wait_cycles, &cycles, sizeof(cycles)));
   DST_CUDA_TRY(cudaMemcpyToSymbol(dst::g_drop_drain_arrivals, &drop, sizeof(drop)));
   dst::g_debug_max_ctas = max_ctas > 0 ? max_ctas : 0;
+  return DST_OK;
+}
+
+extern "C" int dst_debug_prefill_plan(int fmt, int n_terms, int64_t E, int64_t T, int64_t N, int64_t K, int64_t max_rows, int out_dtype, int64_t first_expert,
+                                      int* plan) {
+  using namespace dst;
+  if (!plan || (fmt != DST_FMT_TQ1 && fmt != DST_FMT_TQ2) || n_terms < 1 || n_terms > DST_MAX_TERMS || E < 1 || T < 1 || N < 1 || K < 128 ||
+      K % 128 != 0 || first_expert < 0 || first_expert >= E || T >= (int64_t(1) << 30) || N > (int64_t(1) << 22) || K > (int64_t(1) << 24))
+    return DST_ERR_BAD_ARG;
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.terms.n = n_terms;
+  a.E = E;
+  a.T = T;
+  a.N = N;
+  a.K = K;
+  a.G = K / 128;
+  a.fmt = fmt;
+  a.max_rows = max_rows;
+  a.out_dtype = out_dtype;
+  PrefillParams p;
+  memset(&p, 0, sizeof(p));
+  size_params(a, p);
+  p.E = run_experts_of(E, first_expert / PF_MAX_E * PF_MAX_E);
+  bool small_form = false;
+  const size_t smem = plan_tiles(fmt, p, small_form);
+  if (smem == 0) return DST_ERR_UNSUPPORTED;
+  const int values[DST_PREFILL_PLAN_INTS] = {p.tn_max, p.nb, p.na, p.nslab, small_form ? 1 : 0, (int)smem, map_heights(p.tn_max), p.E};
+  memcpy(plan, values, sizeof(values));
   return DST_OK;
 }
 

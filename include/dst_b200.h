@@ -418,6 +418,16 @@ int dst_check_device_status(dst_stream_t stream);
  */
 int dst_debug_prefill_timeout(long long wait_cycles, int drop_drain_arrivals, int max_ctas);
 
+/*
+ * Test hook: the tcgen05 kernel's plan for a grouped GEMM (host arithmetic, needs no GPU), for the launch that holds expert
+ * `first_expert`; max_rows = the most rows of an expert by the host offsets, -1 where they are on the device only.
+ * plan[0 ..]: token rows per tile at most, activation stages, TMEM slots, packed-slab slots, 1 for the form of small tiles,
+ * dynamic shared memory, tensor maps encoded (of 16, 32, ... rows), experts of the launch.
+ */
+#define DST_PREFILL_PLAN_INTS 8
+int dst_debug_prefill_plan(int fmt, int n_terms, int64_t E, int64_t T, int64_t N, int64_t K, int64_t max_rows, int out_dtype, int64_t first_expert,
+                           int* plan);
+
 #ifdef __cplusplus
 }
 #endif

@@ -147,3 +147,26 @@ def test_moe_layer_decode_copies(lib):
         assert lib.dst_moe_layer_workspace_bytes(2, 2, 0, ctypes.byref(c), None) > 0
     c.w13_decode[0] = 0x1000  # one of two terms
     assert lib.dst_moe_layer_workspace_bytes(2, 2, 0, ctypes.byref(c), None) == 0
+
+
+def _prefill_plan(lib, fmt, n_terms, E, T, N, K, max_rows=-1, out_dtype=1, first_expert=0):
+    plan = (ctypes.c_int * 8)()
+    assert lib.dst_debug_prefill_plan(fmt, n_terms, E, T, N, K, max_rows, out_dtype, first_expert, plan) == _lib.OK
+    return dict(zip(("tn_max", "nb", "na", "nslab", "small", "smem", "maps", "experts"), plan))
+
+
+@pytest.mark.parametrize("fmt", [1, 2])
+@pytest.mark.parametrize("n_terms", [1, 2, 3, 4])
+def test_prefill_plan_encodes_every_tensor_map_a_tile_can_choose(lib, fmt, n_terms):
+    """The rows of a tile come from the device's offsets: whatever the host copy said (max_rows), every tile of up to tn_max
+    rows finds an encoded map of its height (rows rounded up to 16, half of them above 256), inside the plan's limits."""
+    for E, T, N in ((1, 1, 4096), (1, 333, 4096), (1, 4096, 300), (6, 7, 512), (96, 9600, 4096), (384, 98304, 4096), (2000, 5000, 256)):
+        for max_rows in {-1 if E > 1 else T, 1 if E > 1 else T, 17 if E > 1 else T, -(-T // E), T}:
+            for out_dtype in (0, 1):
+                p = _prefill_plan(lib, fmt, n_terms, E, T, N, 2048, max_rows, out_dtype)
+                assert 64 <= p["tn_max"] <= 320 and p["tn_max"] % 32 == 0 and p["small"] == (p["tn_max"] <= 128) and p["nb"] >= 2
+                assert p["tn_max"] + p["na"] * 32 * (2 if p["small"] else 1) <= 512 and p["smem"] <= 232448 - 1024
+                for rows in range(1, p["tn_max"] + 1):
+                    n_eff = -(-rows // 16) * 16 if rows <= 256 else -(-rows // 32) * 32
+                    height = n_eff if n_eff <= 256 else n_eff // 2
+                    assert height // 16 <= p["maps"] <= 16
