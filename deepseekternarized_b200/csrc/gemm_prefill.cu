@@ -126,6 +126,7 @@ struct PrefillParams {
   int E, T, N, K, G, NT, S, kstages;
   // chosen by the host from the shared-memory budget
   int tn_max;       // token rows per tile at most (a multiple of 32, <= PF_TN_MAX): accumulator columns 0 .. tn_max - 1, the A ring after them
+  int one_matrix;   // host: the call has one matrix and no offsets matter, all T rows are its own (a run of one expert of many is not that)
   int rows_hint;    // most rows an expert is expected to have (host knowledge or the mean and three deviations), sizes tn_max
   int nb;           // B stages in shared memory
   int na;           // A slots in TMEM = length of the barrier rings (nb <= na): stage g uses A slot g % na and B stage g % nb
@@ -1239,7 +1240,7 @@ size_t plan_tiles(PrefillParams& p, bool& small_form) {
   // room for it.
   int tn_cap = (p.rows_hint + 31) / 32 * 32;
   tn_cap = tn_cap < 64 ? 64 : (tn_cap > PF_TN_MAX ? PF_TN_MAX : tn_cap);
-  if (p.E == 1) {
+  if (p.one_matrix) {
     // One matrix: the row count is known, and few, large tiles may leave SMs idle. The token tile that gives the least (waves of
     // tiles) x (time of a 64-K stage, ns: fits of what 64 to 256 rows and one and two terms measured). 333 rows through
     // 4096 x 4096: 4 x 32 tiles of 84 rows instead of 2 x 32 of 167, kernel 30 -> 26 us; 2048 rows through 4096 x 11008, two terms: 203 -> 199 us per call.
@@ -1334,6 +1335,7 @@ void size_params(const GemmArgs& a, PrefillParams& p) {
   const int64_t mean = cdiv64(a.T, a.E);
   p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : mean + (int64_t)ceil(3.0 * sqrt((double)mean)));
   if (p.rows_hint < 1) p.rows_hint = 1;
+  p.one_matrix = a.E == 1 ? 1 : 0;
 }
 int run_experts_of(int64_t E, int64_t e0) { return (int)(E - e0 < PF_MAX_E ? E - e0 : PF_MAX_E); }
 

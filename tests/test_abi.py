@@ -170,3 +170,13 @@ def test_prefill_plan_encodes_every_tensor_map_a_tile_can_choose(lib, fmt, n_ter
                     n_eff = -(-rows // 16) * 16 if rows <= 256 else -(-rows // 32) * 32
                     height = n_eff if n_eff <= 256 else n_eff // 2
                     assert height // 16 <= p["maps"] <= 16
+
+
+@pytest.mark.parametrize("T", [1024, 10240, 50000, 102400, 300000])
+def test_prefill_plan_of_a_last_run_of_one_expert(lib, T):
+    """1024 experts are two launches, of 1023 and of one: the second one's rows are one expert's, not all of the call's, so its
+    tile is chosen like the first one's. One matrix has all rows."""
+    for n_terms, max_rows, N in ((1, -1, 128), (1, -1, 300), (1, -1, 4096), (2, -1, 128), (2, -1, 4096), (1, T // 1024 + 40, 128)):
+        first, last = (_prefill_plan(lib, 1, n_terms, 1024, T, N, 4096, max_rows, first_expert=e) for e in (0, 1023))
+        assert (first["experts"], last["experts"]) == (1023, 1)
+        assert {k: v for k, v in first.items() if k != "experts"} == {k: v for k, v in last.items() if k != "experts"}
