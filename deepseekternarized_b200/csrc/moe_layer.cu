@@ -101,12 +101,20 @@ struct Buffers {  // of one set of experts
   __half* gu;
   void* down;
 };
-Buffers take_buffers(Carve& c, const dst_expert_weights& w, const Gemm& g1, const Gemm& g2, int64_t n) {
+// `down` lies over `xs`: the second GEMM writes it after the first one has read those (one stream). What is taken behind the
+// returned mark is free again once the second GEMM is done. A layer's single steps hold xs, gu, h and down at once; the call
+// needs no more memory than they do.
+Buffers take_buffers(Carve& c, const dst_expert_weights& w, const Gemm& g1, const Gemm& g2, int64_t n, size_t* mark) {
   Buffers b;
+  const size_t start = c.used;
+  b.down = c.take<uint16_t>((size_t)n * w.hidden);
+  const size_t down_end = c.used;
+  c.used = start;
   b.xs = take_rows(c, g1.path, n, w.hidden);
+  if (c.used < down_end) c.used = down_end;
+  *mark = c.used;
   b.gu = c.take<__half>((size_t)n * 2 * w.inter);
   b.h = take_rows(c, g2.path, n, w.inter);
-  b.down = c.take<uint16_t>((size_t)n * w.hidden);
   return b;
 }
 
@@ -185,14 +193,18 @@ int layer(const void* x, const float* weights, const int32_t* ids, int64_t T, in
   uint8_t* sort_ws = c.take<uint8_t>(dst_sort_workspace_bytes(n, w->experts));
   Gemm g1 = make_gemm(*w, false, n, offsets), g2 = make_gemm(*w, true, n, offsets);
   if (g1.path == PATH_NONE || g2.path == PATH_NONE) return DST_ERR_UNSUPPORTED;
-  const Buffers b = take_buffers(c, *w, g1, g2, n);
+  size_t mark = 0;
+  const Buffers b = take_buffers(c, *w, g1, g2, n, &mark);
   Gemm s1, s2;
   Buffers sb;
   if (shared) {
     s1 = make_gemm(*shared, false, T, nullptr);
     s2 = make_gemm(*shared, true, T, nullptr);
     if (s1.path == PATH_NONE || s2.path == PATH_NONE) return DST_ERR_UNSUPPORTED;
-    sb = take_buffers(c, *shared, s1, s2, T);
+    const size_t end = c.used;
+    c.used = mark;  // the shared expert runs after the routed ones, in the memory of their gate, up and SwiGLU rows
+    sb = take_buffers(c, *shared, s1, s2, T, &mark);
+    if (c.used < end) c.used = end;
   }
   if (bytes) {  // only asked for the size
     *bytes = c.used;

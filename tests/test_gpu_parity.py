@@ -656,6 +656,32 @@ def test_moe_layer_in_one_call_wide_experts(fmt, copy, inter):
         assert torch.equal(y, MoELayer(w, 2, ops=Steps(), **kw)(x, logits)) and bool(y.isfinite().all()) and float(y.float().abs().max()) > 0
 
 
+@pytest.mark.parametrize("T", [8, 300, 6000])
+@pytest.mark.parametrize("flavour", ["v4", "standard"])
+@pytest.mark.parametrize("fmt", ["tq1", "tq2"])
+def test_moe_layer_in_one_call_needs_no_more_memory_than_its_steps(fmt, flavour, T):
+    """Peak device memory of the one call against that of the single steps (a megabyte for the allocator's rounding)."""
+    from deepseekternarized_b200.moe import B200Ops, MoELayer
+
+    class Steps(B200Ops):
+        pass
+
+    w = _random_experts(16, 1024, 512, fmt, 1)
+    kw = {"flavour": flavour} if flavour == "standard" else {"shared": _random_experts(1, 1024, 512, fmt, 2)}
+    x, logits = torch.randn(T, 1024, device=DEV).bfloat16(), torch.randn(T, 16, device=DEV)
+    peak = []
+    for layer in (MoELayer(w, 4, **kw), MoELayer(w, 4, ops=Steps(), **kw)):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        y = layer(x, logits)
+        torch.cuda.synchronize()
+        peak.append(torch.cuda.max_memory_allocated() - before)
+        del y
+    assert peak[0] <= peak[1] + (1 << 20)
+
+
 @pytest.mark.parametrize("hidden,inter", [(2048, 768), (768, 2048)])
 def test_moe_layer_in_one_call_with_one_matrix_decode_copy(hidden, inter):
     """TQ1 with 2-bit copies where only one of the two matrices can have one (K a multiple of 512): the call takes the copy as
