@@ -48,6 +48,7 @@
 // roles leave their loops, the CTA frees TMEM and the kernel records DST_ERR_TIMEOUT in the status word.
 #include <cuda.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
 
@@ -1173,9 +1174,28 @@ EncodeFn encode_fn() {
   return fn;
 }
 
+// The kernel's dynamic shared memory starts where plan_smem reckons with (the kernel looks again, but can only leave without
+// output): behind the system's part and at most 1 KB of the kernel's own static part.
+template <typename Kernel>
+int check_smem_start(Kernel kernel, std::atomic<int>& known) {
+  if (known.load(std::memory_order_relaxed) == 0) {
+    int dev = 0, reserved = 0;
+    cudaFuncAttributes attr;
+    DST_CUDA_TRY(cudaGetDevice(&dev));
+    DST_CUDA_TRY(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+    DST_CUDA_TRY(cudaFuncGetAttributes(&attr, kernel));
+    const bool fits = (uint32_t)reserved >= PF_SMEM_FIRST && (size_t)reserved + ((attr.sharedSizeBytes + 127) & ~(size_t)127) <= PF_SMEM_START;
+    known.store(fits ? 1 : 2, std::memory_order_relaxed);
+  }
+  return known.load(std::memory_order_relaxed) == 1 ? DST_OK : DST_ERR_UNSUPPORTED;
+}
+
 template <int FMT, int TERMS, bool SMALL>
 int launch_plan(const TmaMaps& maps, const PrefillParams& p, size_t smem, cudaStream_t st) {
   auto kernel = prefill_kernel<FMT, TERMS, SMALL>;
+  static std::atomic<int> smem_start{0};
+  const int rc = check_smem_start(kernel, smem_start);
+  if (rc != DST_OK) return rc;
   DST_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 148;
   DST_CUDA_TRY(cudaGetDevice(&dev));
@@ -1497,7 +1517,7 @@ extern "C" int dst_check_device_status(dst_stream_t stream) {
   int st_ep = 0;  // and so does the expert-parallel barrier
   const int rc2 = dst::ep_take_status(&st_ep);
   if (rc2 != DST_OK) return rc2;
-  return (st != 0 || st_decode != 0 || st_ep != 0) ? DST_ERR_TIMEOUT : DST_OK;
+  return st != 0 ? st : (st_decode != 0 || st_ep != 0) ? DST_ERR_TIMEOUT : DST_OK;  // the words hold the status itself
 }
 
 // ------------------------------------------------------------------------------------------ no-allocation entry

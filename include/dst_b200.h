@@ -405,7 +405,8 @@ int dst_ternary_grouped_gemm_noalloc(void* out, int out_dtype, int accumulate, c
                                      int64_t E, int64_t T, int64_t N, int64_t K, int fmt, dst_stream_t stream);
 
 /* Reads (and clears) the device-side status words that bounded waits in the tcgen05, decode and barrier kernels write when
- * they give up. Synchronises `stream`. Returns DST_OK or DST_ERR_TIMEOUT. */
+ * they give up. Synchronises `stream`. Returns DST_OK, DST_ERR_TIMEOUT, or DST_ERR_UNSUPPORTED where the tcgen05 kernel
+ * left without output (its shared memory did not start where the host had planned it). */
 int dst_check_device_status(dst_stream_t stream);
 
 /*
