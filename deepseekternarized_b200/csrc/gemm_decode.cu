@@ -898,12 +898,13 @@ int64_t decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N) 
 }
 
 // The choice itself. The GEMV keeps, up to its own limit, a call whose tensors the tcgen05 kernel does not take as they lie in
-// memory (scales that are a view at an odd offset, say), and one with float32 results: the tensor core adds all of K in one
-// accumulator, the GEMV 128 elements and then by fused multiply-adds, which is more exact (TQ1, normal activations, relative
-// error against 64 bits at K = 4096 1.1e-6 against 4.1e-6; a 16-bit result rounds to 1.7e-3 or 2e-4 either way).
+// memory (scales that are a view at an odd offset, say), and one whose results show the difference in exactness: the tensor
+// core adds all of K in one accumulator, the GEMV 128 elements and then by fused multiply-adds. Relative error against 64 bits
+// (TQ1, normal activations, K = 4096), GEMV / tcgen05: float32 results 1.1e-6 / 4.1e-6, float16 2.1026e-4 / 2.1029e-4, bf16
+// 1.6661e-3 both.
 bool auto_takes_decode(const GemmArgs& a) {
   const int64_t rows = a.max_rows >= 0 ? a.max_rows : cdiv64(a.T, a.E);
-  const bool by_speed = a.out_dtype != DST_OUT_F32 && prefill_aligned(a);
+  const bool by_speed = a.out_dtype == DST_OUT_BF16 && prefill_aligned(a);
   const int64_t limit = by_speed ? decode_auto_rows(a.fmt, a.terms.n, a.E, a.T, a.N) : decode_row_limit(a.fmt, a.E, a.N);
   return rows <= limit && decode_supports(a);
 }

@@ -167,7 +167,7 @@ int64_t dst_decode_row_limit(int fmt, int64_t E, int64_t N);
 
 /* Token rows per expert up to which DST_ALGO_AUTO takes the decode GEMV for T rows in all over E experts of N rows and
  * n_terms stacked terms: the limit above, except for single-term TQ1 tiles (8 when T rows leave every CTA at most one
- * work unit and E > 1, else 0). A call with float32 results, or whose tensors are not aligned for the tcgen05 kernel (scales
+ * work unit and E > 1, else 0). A call without bf16 results, or whose tensors are not aligned for the tcgen05 kernel (scales
  * and weights 16 bytes, workspace 256), keeps dst_decode_row_limit. No reference counterpart. */
 int64_t dst_decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N);
 

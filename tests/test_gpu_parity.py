@@ -733,23 +733,26 @@ def test_few_row_tq1_calls_with_unaligned_scales(kb, E, T):
     assert torch.equal(out, want)
 
 
+@pytest.mark.parametrize("out_dtype,tol", [(torch.float32, 2e-6), (torch.float16, 3e-4)])
 @pytest.mark.parametrize("E,T", [(1, 1), (1, 4), (1, 16), (6, 7), (6, 60)])
-def test_few_row_tq1_float32_results_are_the_gemvs(kb, E, T):
-    """Float32 results of few rows through one TQ1 term come from the kernel with the more exact sums, whatever is faster."""
+def test_few_row_tq1_results_finer_than_bf16_are_the_gemvs(kb, E, T, out_dtype, tol):
+    """Float32 and float16 results of few rows through one TQ1 term come from the kernel with the more exact sums, whatever is
+    faster."""
     N, K = 520, 4096
     rng = np.random.default_rng(T)
     (p, s), = make_terms(rng, N, K, 128, "tq1", 1, lead=(E,))
     offsets = np.linspace(0, T, E + 1).astype(np.int64)
     x = O.synth_acts(rng, (T, K))
     w, sc, xt = kb.tile_weights(torch.from_numpy(p).to(DEV), "tq1", K), torch.from_numpy(s).to(DEV), bf16_tensor(x, DEV)
-    got, want = (kb.grouped_ternary_gemm_bf16(xt, offsets, [w], [sc], K, 128, "tq1", algo=a) for a in ("auto", "decode"))
+    got, want = (kb.grouped_ternary_gemm_bf16(xt, offsets, [w], [sc], K, 128, "tq1", algo=a, out_dtype=out_dtype) for a in ("auto", "decode"))
     assert torch.equal(got, want)
     for e in range(E):
         a, b = offsets[e], offsets[e + 1]
         if b > a:
             y64 = O.gemm_f64(x[a:b], [(p[e], s[e])], K, 128, "tq1")
-            # products with trits are exact; 128-element sums of 2^-24 each, then 32 groups: some 1e-6 of the norm
-            assert O.rel_fro(got[a:b].cpu().numpy(), y64) < 2e-6
+            # products with trits are exact; 128-element sums of 2^-24 each, then 32 groups: some 1e-6 of the norm; a float16
+            # result rounds by 2^-12 at most (2.4e-4)
+            assert O.rel_fro(got[a:b].float().cpu().numpy(), y64) < tol
 
 
 @pytest.mark.parametrize("flavour", ["v4", "standard"])
