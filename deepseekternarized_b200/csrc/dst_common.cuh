@@ -67,6 +67,7 @@ __device__ __forceinline__ float silu_fast(float g) {
   return __fdividef(g, 1.f + __expf(-g));
 }
 
+int sm_count();  // of the current device (148, a B200's, where there is none)
 int64_t tiled_superblocks(int fmt, int64_t K);
 size_t prefill_workspace_bytes(int act_dtype, int64_t T, int64_t K);
 size_t decode_workspace_bytes(int64_t T, int64_t K);  // optional: lets the decode GEMV quantise each token once, ahead of itself
@@ -87,13 +88,14 @@ bool prefill_aligned(const GemmArgs& a);  // the alignments that launch_prefill 
 bool decode_swiglu_quant_supports(int64_t inter);
 int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const int64_t* order, int64_t T, int64_t inter, float limit,
                         bool standard, void* workspace, cudaStream_t stream);
+// read and clear the status words of the decode kernel and of the expert-parallel barrier kernel (0 or DST_ERR_TIMEOUT)
 int decode_take_status(int* status);
+int ep_take_status(int* status);
 // moe_kernels.cu: the routing sort with the inverse order (inv may be null), and the combine from it
 int sort_rows(const void* ids, int ids_are_i32, int64_t n, int64_t E, int64_t* order, int64_t* offsets, int32_t* bad_count, void* workspace,
               int64_t* inv, cudaStream_t st);
 int combine_rows(const void* down_bf16, const int64_t* inv, const int32_t* ids, const float* weights, int64_t T, int top_k, int64_t hidden,
                  const void* add_bf16, void* y_bf16, cudaStream_t st);
-int ep_take_status(int* status);      // the same for the expert-parallel barrier kernel  // reads and clears the decode kernel's status word (0 or DST_ERR_TIMEOUT)
 
 // ---------------------------------------------------------------------------------------------
 // Trit decoding. TQ1 digit i of byte v: ((v / 3^i) % 3) - 1 for v < 243, else 0

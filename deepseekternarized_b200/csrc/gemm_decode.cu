@@ -808,15 +808,12 @@ int launch_one(DecodeParams p, int sms, cudaStream_t stream) {
   return DST_OK;
 }
 
-#ifndef DC_WIDE_FROM
-#define DC_WIDE_FROM 5
-#endif
 template <typename XT>
 int launch_rows(const DecodeParams& p, int64_t rows_hint, bool rows_known, int sms, cudaStream_t stream) {
   // one row per expert at most, for certain: passes of one row, the least shared memory
   if (p.T == 1 || (rows_known && rows_hint <= 1)) return launch_one<4, 1, 4, 1, XT>(p, sms, stream);
   // up to four: passes of up to four rows, each pass shaped by the rows it has
-  if (rows_hint < DC_WIDE_FROM && rows_hint <= 4) return launch_one<0, 1, 4, 1, XT>(p, sms, stream);
+  if (rows_hint <= 4) return launch_one<0, 1, 4, 1, XT>(p, sms, stream);
   // five or more rows: one CTA per SM whose eight consumer warps own 32 weight rows each and share the staged token
   // rows (8, then 16 per pass), when there is a 256-row unit for every SM; else the small CTAs
   const long long wide_units = (long long)p.E * blocks_per_expert<256>(p.NT);
@@ -825,7 +822,6 @@ int launch_rows(const DecodeParams& p, int64_t rows_hint, bool rows_known, int s
     if (rc == DST_ERR_UNSUPPORTED) rc = launch_one<1, 2, 8, 2, XT>(p, sms, stream);
     if (rc != DST_ERR_UNSUPPORTED) return rc;
   }
-  if (rows_hint <= 4) return launch_one<0, 1, 4, 1, XT>(p, sms, stream);
   const int rc = launch_one<1, 2, 4, 1, XT>(p, sms, stream);
   return rc == DST_ERR_UNSUPPORTED ? launch_one<0, 1, 4, 1, XT>(p, sms, stream) : rc;  // 16 staged rows of a long K may not fit
 }
@@ -877,21 +873,24 @@ int decode_swiglu_quant(const void* gu_bf16, const float* route_weights, const i
   return DST_OK;
 }
 
-// Up to how many token rows per expert the decode GEMV can beat the tcgen05 kernel (measured on 4096 x 4096 experts): 32
-// where the many-row CTAs apply (TQ2 tiles, a 256-row unit for every SM; two passes of 16 rows), else 16.
-static int sm_count() {
+int sm_count() {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return sms;
 }
+
+// Up to how many token rows per expert the decode GEMV can beat the tcgen05 kernel (measured on 4096 x 4096 experts): 32
+// where the many-row CTAs apply (TQ2 tiles, a 256-row unit for every SM; two passes of 16 rows), else 16.
 int64_t decode_row_limit(int fmt, int64_t E, int64_t N) {
   return fmt == DST_FMT_TQ2 && E * ((N + 255) / 256) >= sm_count() ? 32 : 16;
 }
 
-// ... and up to how many AUTO takes it for T rows. One TQ1 term: the GEMV runs at 1.0 TB/s of packed bytes with one row per
-// expert and 0.6 with eight, the tcgen05 kernel at 1.03 whatever the rows (48 experts of 4096 x 4096: 172 / 270 us against 167 / 169), so the
-// GEMV is left the steps whose units all run at once (6 experts, one row each: 45 against 58 us) and not a single matrix
-// (11008 x 4096, four rows: 61 against 32 us). More terms: the tcgen05 kernel adds them in fp16, the GEMV one by one in fp32.
+// ... and up to how many AUTO takes it for T rows, as far as speed goes. One TQ1 term: the GEMV runs at 1.0 TB/s of packed bytes with one
+// row per expert and 0.6 with eight, the tcgen05 kernel at 1.03 whatever the rows (48 experts of 4096 x 4096: 172 / 270 us against 167 /
+// 169), so the GEMV is left the steps whose units all run at once (six rows on 384 experts of 4096 x 4096: 45 against 54 us; with
+// few experts in all the tcgen05 kernel would be the faster one there too: 6 rows on 6 experts 57 against 30 us, on 64 of 2048 x
+// 2048 31 against 24) and not a single matrix (11008 x 4096, four rows: 61 against 32 us). More terms: the tcgen05 kernel
+// adds them in fp16, the GEMV one by one in fp32.
 int64_t decode_auto_rows(int fmt, int n_terms, int64_t E, int64_t T, int64_t N) {
   if (fmt != DST_FMT_TQ1 || n_terms > 1) return decode_row_limit(fmt, E, N);
   return E > 1 && T * ((N + 255) / 256) <= sm_count() ? 8 : 0;

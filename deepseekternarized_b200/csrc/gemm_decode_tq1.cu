@@ -7,7 +7,7 @@
 // hardware), the token rows are staged once per expert in shared memory pre-scaled by 4^-f, and the per-(token,
 // group) sums of x remove the u = t + 1 offset. What TQ1 adds:
 //
-//   bytes -> fields   a shared-memory table (the entries the tcgen05 kernel uses, gemm_prefill.cu) maps a byte
+//   bytes -> fields   a shared-memory table maps a byte
 //                     to its five digits as 2-bit fields, placed for both positions a byte can take in a pair of
 //                     bytes; one AND-OR merges two entries into a word of five (even, odd) trit pairs, and five
 //                     ANDs give five A registers. Per byte: one table read and ~4.5 integer instructions, which
@@ -29,7 +29,7 @@
 // the lanes consume them, zeros included) serve 256 weight rows. Up to 8 token rows per pass; an expert with
 // more rows is processed in several passes (the weights are re-read, from L2). The CTAs' runs of units are cut over the
 // experts that have rows (decode_units.cuh): 8 tokens on 384 experts, both GEMVs 1213 us cut over all experts, ~260 now.
-// AUTO leaves it the steps that decode_auto_rows (gemm_decode.cu) names: the tcgen05 kernel is as fast for many units.
+// AUTO leaves it the steps that auto_takes_decode (gemm_decode.cu) names: the tcgen05 kernel is as fast for many units.
 //
 // Coverage: TQ1 tiled weights, group 128, K % 128 == 0, fp16 scales, bf16 or fp16 activations.
 #include "decode_units.cuh"

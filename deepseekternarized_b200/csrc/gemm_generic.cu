@@ -360,7 +360,8 @@ int launch_canonical(CanonArgs a, int64_t passes, cudaStream_t st) {
   // enough CTAs for two per SM where splitting K between warps can give them
   a.wk = 1;
   const int64_t tiles = cdiv64(a.g.N, 16) * std::min(a.g.E, a.g.T) * passes;
-  while (a.wk < CI_WARPS && cdiv64(tiles * a.wk, CI_WARPS) < 2 * 148 && a.wk * STEP < whole) a.wk *= 2;
+  const int64_t ctas = 2 * sm_count();
+  while (a.wk < CI_WARPS && cdiv64(tiles * a.wk, CI_WARPS) < ctas && a.wk * STEP < whole) a.wk *= 2;
   const size_t stage = (size_t)TOK * (a.chunk + 16) + (size_t)TOK * (a.chunk / STEP) * 4;
   const size_t smem = std::max(stage, (size_t)CI_WARPS * NB * 4 * 32 * 4);
   auto kernel = canonical_i8_kernel<FMT, STEP, NB>;

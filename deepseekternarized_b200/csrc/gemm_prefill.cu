@@ -1264,6 +1264,7 @@ size_t plan_tiles(PrefillParams& p, bool& small_form) {
     // One matrix: the row count is known, and few, large tiles may leave SMs idle. The token tile that gives the least (waves of
     // tiles) x (time of a 64-K stage, ns: fits of what 64 to 256 rows and one and two terms measured). 333 rows through
     // 4096 x 4096: 4 x 32 tiles of 84 rows instead of 2 x 32 of 167, kernel 30 -> 26 us; 2048 rows through 4096 x 11008, two terms: 203 -> 199 us per call.
+    const int sms = sm_count();
     float best = 0.f;
     int best_tn = 0;
     for (int tn = 64; tn <= tn_cap; tn += 32) {
@@ -1272,7 +1273,7 @@ size_t plan_tiles(PrefillParams& p, bool& small_form) {
       if ((small ? plan_smem<FMT, TERMS, true>(p, 2) : plan_smem<FMT, TERMS, false>(p, 4)) == 0) continue;
       const long long tiles = cdiv64(p.T, tn), rows = cdiv64(p.T, tiles);
       const float stage = (small ? 245.f + 0.9f * (float)(rows > 64 ? rows - 64 : 0) : 230.f + 0.9f * (float)rows) + 135.f * (float)(p.n_terms - 1);
-      const float cost = (float)cdiv64(tiles * p.NT, 148) * stage;
+      const float cost = (float)cdiv64(tiles * p.NT, sms) * stage;
       if (best_tn == 0 || cost < best) {
         best = cost;
         best_tn = tn;
@@ -1349,9 +1350,12 @@ void size_params(const GemmArgs& a, PrefillParams& p) {
   p.S = (int)tiled_superblocks(a.fmt, a.K);
   p.kstages = (int)(a.K / 64);
   // Rows per expert: known when the caller passed host offsets, else three standard deviations of an even routing above the
-  // mean (an expert with more is split into two tiles, which dequantises its weights twice; a tile sized for twice the mean
-  // costs every expert the form of the kernel for larger tiles: 96 rows on 96 experts of 4096 x 4096, TQ1, 428 against
-  // 596 us)
+  // mean. An expert with more is split into two tiles, which dequantises its weights twice; a tile sized for twice the mean
+  // costs every expert the form of the kernel for larger tiles (96 rows on 96 experts of 4096 x 4096, TQ1, 428 against
+  // 596 us). Under a skewed router (Zipf exponents 0, 0.3, 0.6, 1; 384 TQ1, 64 TQ2 and 128 two-term TQ2 experts) this size
+  // against twice the mean took 0.88-0.95 of the time at 24 to 48 rows of the small TQ2 experts and the same elsewhere;
+  // 0.94-1.00 even and up to 1.08 skewed at 64; 0.78-0.90 at 80 and 96 (two terms 0.91-1.03); 0.92-1.01 even and up to
+  // 1.14 (TQ1, 128 rows, exponent 1) from 128 on.
   const int64_t mean = cdiv64(a.T, a.E);
   p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : mean + (int64_t)ceil(3.0 * sqrt((double)mean)));
   if (p.rows_hint < 1) p.rows_hint = 1;
