@@ -15,6 +15,15 @@ namespace {
 template <int RI>
 __host__ __device__ __forceinline__ int blocks_per_expert(int NT) { return (NT * 128 + RI - 1) / RI; }
 
+// Passes at most of T rows on E experts: the sum of ceil(rows / MT) over the experts that have some.
+template <int MT>
+inline long long max_passes(long long E, long long T) { return (T + (MT - 1) * (E < T ? E : T)) / MT; }
+
+// a / b for 0 <= a, 0 < b < 2^31, in 32 bits where a allows it (a 64-bit division is some hundred instructions)
+__device__ __forceinline__ long long div_small(long long a, int b) {
+  return a <= 0xffffffffLL ? (long long)((uint32_t)a / (uint32_t)b) : a / b;
+}
+
 struct Unit {
   int e, n0;           // expert and first weight row
   int64_t ra, rb, m0;  // the expert's token rows [ra, rb) and the pass's first one
@@ -31,7 +40,7 @@ struct UnitWalk {
     blocks = blocks_per_expert<RI>(p.NT);
     u.e = e;
     row_range(p.offsets, e, p.T, u.ra, u.rb);
-    const long long pass = local / blocks;
+    const long long pass = div_small(local, blocks);
     block = (int)(local - pass * blocks);
     u.m0 = u.ra + pass * MT;
     u.n0 = block * RI;
@@ -81,6 +90,25 @@ __device__ __forceinline__ void find_run(const P& p, long long* scratch, UnitRun
     row_range(p.offsets, e, p.T, a, b);
     return (b - a + MT - 1) / MT * blocks;
   };
+  // this CTA's share of `total` units: equal runs. Fewer units than CTAs: one each for the first CTAs, which start on different
+  // SMs (spread over all CTAs instead, every second one of a grid twice the units left half of the SMs idle)
+  auto share = [&](long long total, long long& u0, long long& u1) {
+    const int b = (int)blockIdx.x;
+    const long long base = div_small(total, (int)gridDim.x), more = total - base * (long long)gridDim.x;
+    u0 = base * b + (b < more ? b : more);
+    u1 = u0 + base + (b < more ? 1 : 0);
+  };
+  if (p.E == 1) {  // one matrix: nothing to look for
+    if (threadIdx.x == 0) {
+      long long u0, u1;
+      share(units_of(0), u0, u1);
+      run->e = 0;
+      run->local = u0;
+      run->count = u1 - u0;
+    }
+    __syncthreads();
+    return;
+  }
   long long sum = 0;
   for (int e = e0; e < e1; ++e) sum += units_of(e);
   long long incl = sum;
@@ -96,7 +124,8 @@ __device__ __forceinline__ void find_run(const P& p, long long* scratch, UnitRun
     if (w < warp) before += scratch[w];
     total += scratch[w];
   }
-  const long long u0 = total * blockIdx.x / gridDim.x, u1 = total * (blockIdx.x + 1) / gridDim.x;
+  long long u0, u1;
+  share(total, u0, u1);
   if (u0 < u1 && u0 >= before && u0 < before + sum) {
     long long left = u0 - before;
     for (int e = e0; e < e1; ++e) {

@@ -463,9 +463,7 @@ int launch_decode_tq1(const GemmArgs& a, cudaStream_t stream) {
   int dev = 0, sms = 148;
   DST_CUDA_TRY(cudaGetDevice(&dev));
   DST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // units at most: every token row a pass of its own, or every expert with rows in them and full passes
-  const long long passes = p.T < p.E ? (long long)p.T : (long long)p.E + p.T / D1_MT;
-  const long long items = passes * ((p.NT + 1) >> 1);
+  const long long items = max_passes<D1_MT>(p.E, p.T) * ((p.NT + 1) >> 1);
   const size_t smem = d1_smem(p.S, p.G);
   int per_sm = (int)((220 * 1024) / (smem + 1024));
   per_sm = per_sm < 1 ? 1 : (per_sm > 2 ? 2 : per_sm);

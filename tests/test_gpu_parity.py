@@ -309,6 +309,35 @@ def test_grouped_decode_few_of_many_experts(kb, fmt, rows):
         check_gemm(y[a:b], x[a:b], [(p[e], s[e]) for p, s in terms], K, 128, fmt)
 
 
+@pytest.mark.parametrize("N,K", [(200, 512), (4096, 1024), (64, 2048)])
+@pytest.mark.parametrize("k_terms", [1, 2])
+@pytest.mark.parametrize("act", [torch.bfloat16, torch.int8])
+def test_decode_forms_for_rows_known_on_the_host(kb, N, K, k_terms, act):
+    """One to five rows at most, the counts known on the host (one matrix; experts with fewer rows and without among them): the
+    form for that many rows against the oracle, fewer and more work units than CTAs."""
+    rng = np.random.default_rng(N + K)
+    for most in (1, 2, 3, 4, 5):
+        for counts in ([most], [most, 0, 1, most, 0, 0, min(2, most), most] * 3):
+            E, T = len(counts), sum(counts)
+            terms = make_terms(rng, N, K, 128, "tq2", k_terms, lead=(E,))
+            offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+            if act == torch.int8:
+                x = rng.integers(-127, 128, (T, K)).astype(np.float32)
+                xt = torch.from_numpy(x).to(DEV, torch.int8)
+            else:
+                x = O.synth_acts(rng, (T, K))
+                xt = bf16_tensor(x, DEV)
+            tiled = [kb.tile_weights(torch.from_numpy(p).to(DEV), "tq2", K) for p, _ in terms]
+            y = torch.empty(T, N, device=DEV)
+            kb._grouped(kb.ext(), xt, None, None if E == 1 else offsets, tiled, [torch.from_numpy(s).to(DEV) for _, s in terms], K, 128, "tq2", y,
+                        False, "decode")
+            assert kb.ext().dst_check_device_status(None) == 0
+            for e in range(E):
+                a, b = int(offsets[e]), int(offsets[e + 1])
+                if b > a:
+                    check_gemm(y[a:b].cpu().numpy(), x[a:b], [(p[e], s[e]) for p, s in terms], K, 128, "tq2")
+
+
 @pytest.mark.parametrize("fmt", ["tq2", "tq1"])
 @pytest.mark.parametrize("K,group", [(4160, 128), (2048, 256), (192, 64), (131, 64), (7, 64), (4096 + 36, 128), (1024, 192)])
 def test_int8_grouped_canonical_weights(kb, fmt, K, group):
@@ -635,8 +664,8 @@ def _random_experts(n, hidden, inter, fmt, seed, k_terms=1, copy=False):
     return ExpertWeights(packed["w13"], scale["w13"], packed["w2"], scale["w2"], hidden, inter, 128, fmt).prepare(decode_copy=copy)
 
 
-@pytest.mark.parametrize("fmt,copy", [("tq2", False), ("tq1", True), ("tq1", False)])
-@pytest.mark.parametrize("inter", [16384, 16896, 18432, 24576, 25088, 25600])
+@pytest.mark.parametrize("fmt,copy,inter", [("tq2", False, i) for i in (16384, 16896, 18432, 24576, 25088, 25600)]
+                         + [("tq1", True, i) for i in (16384, 18432, 25088)] + [("tq1", False, i) for i in (18432, 25600)])
 def test_moe_layer_in_one_call_wide_experts(fmt, copy, inter):
     """Intermediate sizes up to and beyond the longest row that the decode GEMV takes (25 088), a decode-sized step, routed and
     as the shared expert: the call gives what the single steps give, bit for bit."""
@@ -645,8 +674,6 @@ def test_moe_layer_in_one_call_wide_experts(fmt, copy, inter):
     class Steps(B200Ops):
         pass
 
-    if copy and inter > 25088:
-        pytest.skip("the single steps read a decode copy with the GEMV only")
     hidden, T = 512, 3
     w, shared = _random_experts(4, hidden, inter, fmt, 1, copy=copy), _random_experts(1, hidden, inter, fmt, 2, copy=copy)
     gen = torch.Generator(device=DEV).manual_seed(inter)

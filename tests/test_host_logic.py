@@ -537,3 +537,27 @@ def test_layer_calls_replaced_steps(stub_library, monkeypatch, flavour, where, n
         with pytest.raises(Reached):
             layer.forward_routed(*args)
         assert calls == []
+
+
+def test_decode_units_are_shared_out_once():
+    """The decode GEMVs' runs of work units (csrc/decode_units.cuh, restated): every unit in one CTA's run, runs that differ by one
+    unit at most, one unit each for the first CTAs where there are fewer units than CTAs; and the host's bound on the passes."""
+    import random
+
+    rnd = random.Random(3)
+    for _ in range(300):
+        ctas, total = rnd.choice([1, 2, 148, 344, 592]), rnd.choice([0, 1, 64, 172, 343, 344, 592, 5000, rnd.randint(0, 100000)])
+        runs, base, more = [], total // ctas, total % ctas
+        for b in range(ctas):
+            u0 = base * b + min(b, more)
+            runs.append((u0, u0 + base + (b < more)))
+        assert runs[0][0] == 0 and runs[-1][1] == total and all(a[1] == b[0] for a, b in zip(runs, runs[1:]))
+        assert max(v - u for u, v in runs) - min(v - u for u, v in runs) <= 1
+        if total < ctas:
+            assert runs[:total] == [(i, i + 1) for i in range(total)]
+    for _ in range(300):
+        mt, E = rnd.choice([1, 2, 4, 8, 16]), rnd.choice([1, 2, 90, 384])
+        rows = [rnd.choice([0, 0, 1, 2, 3, rnd.randint(0, 40)]) for _ in range(E)]
+        T = sum(rows)
+        bound, passes = (T + (mt - 1) * min(E, T)) // mt, sum(-(-r // mt) for r in rows)
+        assert passes <= bound and (E > 1 or passes == bound)
