@@ -127,7 +127,6 @@ struct PrefillParams {
   int E, T, N, K, G, NT, S, kstages;
   // chosen by the host from the shared-memory budget
   int tn_max;       // token rows per tile at most (a multiple of 32, <= PF_TN_MAX): accumulator columns 0 .. tn_max - 1, the A ring after them
-  int one_matrix;   // host: the call has one matrix and no offsets matter, all T rows are its own (a run of one expert of many is not that)
   int rows_hint;    // most rows an expert is expected to have (host knowledge or the mean and three deviations), sizes tn_max
   int nb;           // B stages in shared memory
   int na;           // A slots in TMEM = length of the barrier rings (nb <= na): stage g uses A slot g % na and B stage g % nb
@@ -1252,15 +1251,15 @@ size_t plan_smem(PrefillParams& p, int min_nb) {
 }
 
 // Chooses the token tile and places the CTA's shared memory: returns the dynamic bytes (0: not covered), p.tn_max and whether
-// it is the SMALL form.
+// it is the SMALL form. one_matrix: all T rows of the call are one matrix's (a last run of one expert of many is not that).
 template <int FMT, int TERMS>
-size_t plan_tiles(PrefillParams& p, bool& small_form) {
+size_t plan_tiles(PrefillParams& p, bool one_matrix, bool& small_form) {
   // The token tile is as large as the experts are expected to need (up to 320 rows) as long as a B ring of four 64-K stages
   // fits: that much hides the latency of the copies behind the MMAs of a stage. Then a third packed-slab slot if there is
   // room for it.
   int tn_cap = (p.rows_hint + 31) / 32 * 32;
   tn_cap = tn_cap < 64 ? 64 : (tn_cap > PF_TN_MAX ? PF_TN_MAX : tn_cap);
-  if (p.one_matrix) {
+  if (one_matrix) {
     // One matrix: the row count is known, and few, large tiles may leave SMs idle. The token tile that gives the least (waves of
     // tiles) x (time of a 64-K stage, ns: fits of what 64 to 256 rows and one and two terms measured). 333 rows through
     // 4096 x 4096: 4 x 32 tiles of 84 rows instead of 2 x 32 of 167, kernel 30 -> 26 us; 2048 rows through 4096 x 11008, two terms: 203 -> 199 us per call.
@@ -1289,10 +1288,14 @@ size_t plan_tiles(PrefillParams& p, bool& small_form) {
     if (const size_t smem = plan_smem<FMT, TERMS, true>(p, 2)) return smem;
   return 0;
 }
-size_t plan_tiles(int fmt, PrefillParams& p, bool& small_form) {
+size_t plan_tiles(int fmt, PrefillParams& p, bool one_matrix, bool& small_form) {
   if (fmt == DST_FMT_TQ2)
-    return p.n_terms == 1 ? plan_tiles<2, 1>(p, small_form) : p.n_terms == 2 ? plan_tiles<2, 2>(p, small_form) : plan_tiles<2, 4>(p, small_form);
-  return p.n_terms == 1 ? plan_tiles<1, 1>(p, small_form) : p.n_terms == 2 ? plan_tiles<1, 2>(p, small_form) : plan_tiles<1, 4>(p, small_form);
+    return p.n_terms == 1   ? plan_tiles<2, 1>(p, one_matrix, small_form)
+           : p.n_terms == 2 ? plan_tiles<2, 2>(p, one_matrix, small_form)
+                            : plan_tiles<2, 4>(p, one_matrix, small_form);
+  return p.n_terms == 1   ? plan_tiles<1, 1>(p, one_matrix, small_form)
+         : p.n_terms == 2 ? plan_tiles<1, 2>(p, one_matrix, small_form)
+                          : plan_tiles<1, 4>(p, one_matrix, small_form);
 }
 
 // Tensor maps over the fp16 rows: [T, K], boxes of 64 K-elements x 16 i token rows, 128-byte swizzle, zero fill outside. One
@@ -1317,9 +1320,9 @@ template <int FMT, int TERMS>
 int launch_form(const TmaMaps& maps, const PrefillParams& p, bool small_form, size_t smem, cudaStream_t st) {
   return small_form ? launch_plan<FMT, TERMS, true>(maps, p, smem, st) : launch_plan<FMT, TERMS, false>(maps, p, smem, st);
 }
-int launch_run(int fmt, const __half* rows, PrefillParams& p, cudaStream_t st) {
+int launch_run(int fmt, const __half* rows, PrefillParams& p, bool one_matrix, cudaStream_t st) {
   bool small_form = false;
-  const size_t smem = plan_tiles(fmt, p, small_form);
+  const size_t smem = plan_tiles(fmt, p, one_matrix, small_form);
   if (smem == 0) return DST_ERR_UNSUPPORTED;
   TmaMaps maps;
   const int rc = encode_maps(maps, rows, p.T, p.K, map_heights(p.tn_max));
@@ -1359,7 +1362,6 @@ void size_params(const GemmArgs& a, PrefillParams& p) {
   const int64_t mean = cdiv64(a.T, a.E);
   p.rows_hint = (int)(a.max_rows >= 0 ? a.max_rows : mean + (int64_t)ceil(3.0 * sqrt((double)mean)));
   if (p.rows_hint < 1) p.rows_hint = 1;
-  p.one_matrix = a.E == 1 ? 1 : 0;
 }
 int run_experts_of(int64_t E, int64_t e0) { return (int)(E - e0 < PF_MAX_E ? E - e0 : PF_MAX_E); }
 
@@ -1442,7 +1444,7 @@ int launch_prefill(const GemmArgs& a, cudaStream_t stream) {
       p.tiled[i] = a.terms.packed[i] + e0 * tiled_per_expert;
       p.scale[i] = static_cast<const __half*>(a.terms.scale[i]) + e0 * scales_per_expert;
     }
-    const int rc = launch_run(a.fmt, xh, p, stream);
+    const int rc = launch_run(a.fmt, xh, p, a.E == 1, stream);
     if (rc != DST_OK) return rc;
   }
   return DST_OK;
@@ -1500,7 +1502,7 @@ extern "C" int dst_debug_prefill_plan(int fmt, int n_terms, int64_t E, int64_t T
   size_params(a, p);
   p.E = run_experts_of(E, first_expert / PF_MAX_E * PF_MAX_E);
   bool small_form = false;
-  const size_t smem = plan_tiles(fmt, p, small_form);
+  const size_t smem = plan_tiles(fmt, p, E == 1, small_form);
   if (smem == 0) return DST_ERR_UNSUPPORTED;
   const int values[DST_PREFILL_PLAN_INTS] = {p.tn_max, p.nb, p.na, p.nslab, small_form ? 1 : 0, (int)smem, map_heights(p.tn_max), p.E};
   memcpy(plan, values, sizeof(values));
