@@ -32,6 +32,7 @@ CPU ranks (gloo) by passing their own ops object built on the test oracle.
 from __future__ import annotations
 
 import ctypes
+import operator
 from dataclasses import dataclass
 
 import torch
@@ -361,7 +362,7 @@ class MoELayer:
         bf16 rows of this layer, weights or shapes it does not cover."""
         if type(self.ops) is not B200Ops or self.ops.algo != "auto" or not self.ops.fused_norm:
             return None
-        if _replaced(self, _LAYER_STEPS) or _replaced(self.ops, _OPS_STEPS):
+        if _LAYER_STEPS.replaced(self) or _OPS_STEPS.replaced(self.ops):
             return None
         if not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or x.size(1) != self.w.hidden or not (weights.device == ids.device == x.device) \
                 or ids.dtype not in (torch.int32, torch.int64):
@@ -417,14 +418,20 @@ class MoELayer:
     __call__ = forward
 
 
-# The steps that the one call into the library stands for: a subclass, an instance or a patch that has its own gets it called.
-_LAYER_STEPS = {n: getattr(MoELayer, n) for n in ("gather_for_experts", "experts_forward", "shared_forward", "_forward_standard")}
-_OPS_STEPS = {n: getattr(B200Ops, n) for n in ("sort", "gather", "gemm", "swiglu", "swiglu_std", "combine", "combine_weighted", "_norm_ok")}
+class _Steps:
+    """Methods of a class that the one call into the library stands for: a subclass, an instance or a patch that has its own gets
+    it called. Looked up by one attribute getter: this is host time of every call (0.6 us, 1.7 by a loop over the names)."""
+
+    def __init__(self, cls, *names: str):
+        self.names, self.get = frozenset(names), operator.attrgetter(*names)
+        self.methods = self.get(cls)
+
+    def replaced(self, obj) -> bool:
+        return self.get(type(obj)) != self.methods or not self.names.isdisjoint(vars(obj))
 
 
-def _replaced(obj, steps: dict) -> bool:
-    cls, own = type(obj), vars(obj)
-    return any(n in own or getattr(cls, n) is not f for n, f in steps.items())
+_LAYER_STEPS = _Steps(MoELayer, "gather_for_experts", "experts_forward", "shared_forward", "_forward_standard")
+_OPS_STEPS = _Steps(B200Ops, "sort", "gather", "gemm", "swiglu", "swiglu_std", "combine", "combine_weighted", "_norm_ok")
 
 
 def expert_owner_split(n_experts: int, world: int) -> int:
