@@ -1259,30 +1259,37 @@ size_t plan_tiles(PrefillParams& p, bool one_matrix, bool& small_form) {
   // room for it.
   int tn_cap = (p.rows_hint + 31) / 32 * 32;
   tn_cap = tn_cap < 64 ? 64 : (tn_cap > PF_TN_MAX ? PF_TN_MAX : tn_cap);
+  int short_ring_tn = 0;  // the token tile that is taken with a ring of three stages
   if (one_matrix) {
     // One matrix: the row count is known, and few, large tiles may leave SMs idle. The token tile that gives the least (waves of
     // tiles) x (time of a 64-K stage, ns: fits of what 64 to 256 rows and one and two terms measured). 333 rows through
     // 4096 x 4096: 4 x 32 tiles of 84 rows instead of 2 x 32 of 167, kernel 30 -> 26 us; 2048 rows through 4096 x 11008, two terms: 203 -> 199 us per call.
+    // The largest tile is weighed with three stages where four do not fit (TQ1, whose table takes 32 KB; a stage then takes up
+    // to 1.3 times as long): 1200 rows through 4096 x 4096, TQ1, are one wave of 128 tiles of 300 rows instead of 160 of 240
+    // rows in two, 55 -> 44 us (49 with the 16 KB table of the kernel before).
     const int sms = sm_count();
     float best = 0.f;
     int best_tn = 0;
     for (int tn = 64; tn <= tn_cap; tn += 32) {
       p.tn_max = tn;
       const bool small = tn <= PF_SMALL_TN;
-      if ((small ? plan_smem<FMT, TERMS, true>(p, 2) : plan_smem<FMT, TERMS, false>(p, 4)) == 0) continue;
+      const bool fits = (small ? plan_smem<FMT, TERMS, true>(p, 2) : plan_smem<FMT, TERMS, false>(p, 4)) != 0;
+      const bool short_ring = !fits && tn == PF_TN_MAX && plan_smem<FMT, TERMS, false>(p, 3) != 0;
+      if (!fits && !short_ring) continue;
       const long long tiles = cdiv64(p.T, tn), rows = cdiv64(p.T, tiles);
       const float stage = (small ? 245.f + 0.9f * (float)(rows > 64 ? rows - 64 : 0) : 230.f + 0.9f * (float)rows) + 135.f * (float)(p.n_terms - 1);
-      const float cost = (float)cdiv64(tiles * p.NT, sms) * stage;
+      const float cost = (float)cdiv64(tiles * p.NT, sms) * stage * (short_ring ? 1.3f : 1.f);
       if (best_tn == 0 || cost < best) {
         best = cost;
         best_tn = tn;
+        short_ring_tn = short_ring ? tn : 0;
       }
     }
     if (best_tn != 0) tn_cap = best_tn;
   }
   small_form = false;
   for (p.tn_max = tn_cap; p.tn_max > PF_SMALL_TN; p.tn_max -= 32)
-    if (const size_t smem = plan_smem<FMT, TERMS, false>(p, 4)) return smem;
+    if (const size_t smem = plan_smem<FMT, TERMS, false>(p, p.tn_max == short_ring_tn ? 3 : 4)) return smem;
   small_form = true;
   for (; p.tn_max >= 64; p.tn_max -= 32)
     if (const size_t smem = plan_smem<FMT, TERMS, true>(p, 2)) return smem;

@@ -471,6 +471,25 @@ def test_prefill_both_forms_at_their_edges(kb, fmt, k_terms, K):
                 check_gemm(y[a:b], x[a:b], [(p[e], s[e]) for p, s in terms], K, 128, fmt)
 
 
+@pytest.mark.parametrize("fmt,k_terms", [("tq1", 1), ("tq1", 2), ("tq2", 1)])
+@pytest.mark.parametrize("T,N,K", [(1200, 4096, 640), (1280, 4090, 128), (310, 11008, 384), (4000, 4096, 256)])
+def test_prefill_one_matrix_token_tiles(kb, fmt, k_terms, T, N, K):
+    """One matrix whose rows the plan gives the largest tile, also with a ring of three stages (TQ1: the table leaves no room for
+    four), against float64 on the device."""
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    trits = [torch.randint(-1, 2, (N, K), generator=gen, device=DEV, dtype=torch.int8) for _ in range(k_terms)]
+    scales = [(torch.rand(N, K // 128, generator=gen, device=DEV) + 0.1).half() for _ in range(k_terms)]
+    x = torch.randn(T, K, generator=gen, device=DEV).bfloat16()
+    from deepseekternarized_b200.ternary.pack import pack
+
+    tiled = [kb.tile_weights(pack(t, fmt)[None], fmt, K) for t in trits]
+    y = kb.grouped_ternary_gemm_bf16(x, None, tiled, [s[None] for s in scales], K, 128, fmt, algo="prefill")
+    assert kb.ext().dst_check_device_status(None) == 0
+    want = x.double() @ sum(t.double() * s.double().repeat_interleave(128, -1) for t, s in zip(trits, scales)).T
+    # one term: exact products, sums in float32; two terms are added in fp16 first (2^-12 of a weight)
+    assert float((y.double() - want).norm() / want.norm()) < (1e-5 if k_terms == 1 else 3e-4)
+
+
 @pytest.mark.parametrize("N", [200, 196, 384])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16])
 def test_prefill_sixteen_bit_outputs_equal_rounded_fp32_outputs(kb, N, out_dtype):
